@@ -27,15 +27,25 @@ namespace {
 
 constexpr int kGenBlock = 256;
 
+// The bits of 8 levels, most significant first, one 16-bit lane of r each:
+// bit = lane >= threshold, t1 where the level's source bit (bit 7 - l of
+// sbits) is set, else t0.
+__device__ __forceinline__ uint32_t rmat_bits(const Rand4 &r, uint32_t sbits, uint32_t t0, uint32_t t1)
+{
+    uint32_t v = 0;
+#pragma unroll
+    for (int l = 0; l < 8; l++) v = (v << 1) | (lane16(r, l) >= ((sbits >> (7 - l)) & 1u ? t1 : t0) ? 1u : 0u);
+    return v;
+}
+
 __device__ __forceinline__ uint32_t rmat_src(uint64_t seed, uint64_t i, int scale, uint32_t t_src)
 {
     uint32_t v = 0;
-    Rand4 r{};
-    for (int l = 0; l < scale; l++) {
-        if ((l & 7) == 0)
-            r = philox4x32_10((uint32_t)i, (uint32_t)(i >> 32), kTagRmatSrc, (uint32_t)(l >> 3), (uint32_t)seed,
-                              (uint32_t)(seed >> 32));
-        v = (v << 1) | (lane16(r, l & 7) >= t_src ? 1u : 0u);
+    for (int l = 0; l < scale; l += 8) {
+        const Rand4 r = philox4x32_10((uint32_t)i, (uint32_t)(i >> 32), kTagRmatSrc, (uint32_t)(l >> 3),
+                                      (uint32_t)seed, (uint32_t)(seed >> 32));
+        const int n = scale - l < 8 ? scale - l : 8;
+        v = (v << n) | rmat_bits(r, 0u, t_src, t_src) >> (8 - n);
     }
     return v;
 }
@@ -44,52 +54,95 @@ __device__ __forceinline__ uint32_t rmat_dst(uint64_t seed, uint32_t u, uint32_t
                                              uint32_t t_d1)
 {
     uint32_t v = 0;
-    Rand4 r{};
-    for (int l = 0; l < scale; l++) {
-        if ((l & 7) == 0)
-            r = philox4x32_10(u, k, kTagRmatDst, (uint32_t)(l >> 3), (uint32_t)seed, (uint32_t)(seed >> 32));
-        const uint32_t sbit = (u >> (scale - 1 - l)) & 1u;
-        v = (v << 1) | (lane16(r, l & 7) >= (sbit ? t_d1 : t_d0) ? 1u : 0u);
+    for (int l = 0; l < scale; l += 8) {
+        const Rand4 r =
+            philox4x32_10(u, k, kTagRmatDst, (uint32_t)(l >> 3), (uint32_t)seed, (uint32_t)(seed >> 32));
+        const int n = scale - l < 8 ? scale - l : 8;
+        // the n source bits below the l already used, at the top of 8 bits
+        const uint32_t sbits = ((u >> (scale - l - n)) << (8 - n)) & 0xFFu;
+        v = (v << n) | rmat_bits(r, sbits, t_d0, t_d1) >> (8 - n);
     }
     return v;
 }
 
+// Out-degrees.  RMAT sources crowd the low ids (the top 8 levels are all zero
+// for (a+b)^8 = 11 % of the edges, the lowest 32 ids alone draw 1.6 % at
+// scale 20), and atomics on one line serialise in L2: the counters of the
+// lowest kHotIds ids are kept per CTA in shared memory and added once at the
+// end.  2^24 edges at scale 20: 440 -> 288 us, the time of the draws.
+constexpr uint32_t kHotIds = 4096;
+
 __global__ void __launch_bounds__(kGenBlock) degrees_kernel(uint64_t E, uint64_t seed, int scale, uint32_t t_src,
                                                             uint32_t *deg)
 {
+    __shared__ uint32_t hot[kHotIds];
+    for (uint32_t i = threadIdx.x; i < kHotIds; i += kGenBlock) hot[i] = 0;
+    __syncthreads();
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < E; i += stride)
-        atomicAdd(&deg[rmat_src(seed, i, scale, t_src)], 1u);
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < E; i += stride) {
+        const uint32_t u = rmat_src(seed, i, scale, t_src);
+        if (u < kHotIds)
+            atomicAdd(&hot[u], 1u);
+        else
+            atomicAdd(&deg[u], 1u);
+    }
+    __syncthreads();
+    // ids the graph does not have (a scale below 12) stay at zero
+    for (uint32_t i = threadIdx.x; i < kHotIds; i += kGenBlock)
+        if (hot[i]) atomicAdd(&deg[i], hot[i]);
 }
 
-// One warp per 32 consecutive vertices; lanes stride over the warp's edge range
-// and find their vertex by a binary search over the 33 row offsets held in
-// lane registers.
-__global__ void __launch_bounds__(kGenBlock) fill_kernel(uint64_t V0, const uint64_t *rowptr, uint64_t seed, int scale,
-                                                         uint32_t t_d0, uint32_t t_d1, uint32_t *col)
+// Largest u in [lo, V0) with rowptr[u] <= e, found by the whole warp (lo
+// satisfies it, e < rowptr[V0]): 32 probes narrow the range 32-fold.
+__device__ __forceinline__ uint64_t warp_find_row(const uint64_t *rowptr, uint64_t lo, uint64_t V0, uint64_t e)
+{
+    const int lane = threadIdx.x & 31;
+    uint64_t n = V0 - lo;  // the row is in [lo, lo + n)
+    while (n > 1) {
+        const uint64_t step = (n + 31) / 32;
+        const uint64_t at = (uint64_t)lane * step;
+        const bool below = at < n && rowptr[lo + at] <= e;
+        const int k = 31 - __clz(__ballot_sync(0xFFFFFFFFu, below));  // lane 0 always holds
+        lo += (uint64_t)k * step;
+        const uint64_t rest = n - (uint64_t)k * step;
+        n = rest < step ? rest : step;
+    }
+    return lo;
+}
+
+// Column entries.  A warp fills kFillEdges consecutive edges at a time,
+// whatever rows they belong to: the warp finds the rows of its first and last
+// edge, and each lane finds its edge's row between them by a binary search of
+// the cached offsets (the rows of 32 consecutive edges share their probes).
+// Bound by the arithmetic of the draws (three Philox evaluations per edge at
+// scale 20).  With one warp per 32 rows, the warp of the hub rows ran alone at
+// the end (2^24 edges at scale 20: 17.4 ms); with 1024 edges per warp in
+// windows of 32 rows, the warps of the sparse rows did (0.53 ms); this form
+// takes 0.29 ms.
+constexpr uint64_t kFillEdges = 512;
+
+__global__ void __launch_bounds__(kGenBlock) fill_kernel(uint64_t V0, uint64_t E, const uint64_t *rowptr,
+                                                         uint64_t seed, int scale, uint32_t t_d0, uint32_t t_d1,
+                                                         uint32_t *col)
 {
     const int lane = threadIdx.x & 31;
     const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x / 32);
-    for (uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) / 32; w * 32 < V0; w += warps) {
-        const uint64_t u0 = w * 32;
-        const uint64_t my_u = u0 + lane;
-        const uint64_t my_off = rowptr[my_u < V0 ? my_u : V0];
-        const uint64_t end = rowptr[u0 + 32 < V0 ? u0 + 32 : V0];
-        const uint64_t begin = __shfl_sync(0xFFFFFFFFu, my_off, 0);
-        for (uint64_t e = begin + lane; __any_sync(0xFFFFFFFFu, e < end); e += 32) {
-            // largest j with off[j] <= e (off[j] = row start of vertex u0 + j)
-            int lo = 0;
-#pragma unroll
-            for (int step = 16; step > 0; step >>= 1) {
-                const uint64_t probe = __shfl_sync(0xFFFFFFFFu, my_off, lo + step);
-                if (lo + step < 32 && u0 + lo + step <= V0 && probe <= e) lo += step;
+    for (uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) / 32; w * kFillEdges < E; w += warps) {
+        const uint64_t begin = w * kFillEdges, end = begin + kFillEdges < E ? begin + kFillEdges : E;
+        const uint64_t r0 = warp_find_row(rowptr, 0, V0, begin), r1 = warp_find_row(rowptr, r0, V0, end - 1);
+        for (uint64_t e = begin + lane; e < end; e += 32) {
+            // the row of e: the largest u in [r0, r1] with rowptr[u] <= e
+            uint32_t lo = (uint32_t)r0, n = (uint32_t)(r1 - r0 + 1);
+            while (n > 1) {
+                const uint32_t half = n / 2;
+                if (__ldg(rowptr + lo + half) <= e) {
+                    lo += half;
+                    n -= half;
+                } else {
+                    n = half;
+                }
             }
-            // skip vertices with no edges that share the same start offset
-            if (e < end) {
-                const uint64_t u = u0 + lo;
-                const uint64_t k = e - rowptr[u];
-                col[e] = rmat_dst(seed, (uint32_t)u, (uint32_t)k, scale, t_d0, t_d1);
-            }
+            col[e] = rmat_dst(seed, lo, (uint32_t)(e - __ldg(rowptr + lo)), scale, t_d0, t_d1);
         }
     }
 }
@@ -100,10 +153,16 @@ __global__ void mark_present(uint64_t V0, const uint32_t *deg, uint32_t *present
     for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < V0; v += stride) present[v] = deg[v] > 0;
 }
 
+// Most targets are marked already: a look before the store keeps the hub
+// vertices' lines from being written once per edge (2^24 edges at scale 20:
+// 381 -> 46 us).
 __global__ void mark_targets(uint64_t E, const uint32_t *col, uint32_t *present)
 {
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < E; e += stride) present[col[e]] = 1u;
+    for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < E; e += stride) {
+        const uint32_t v = col[e];
+        if (present[v] == 0u) present[v] = 1u;
+    }
 }
 
 __global__ void compact_rowptr(uint64_t V0, const uint32_t *present, const uint32_t *newid, const uint64_t *rowptr,
@@ -125,7 +184,7 @@ __global__ void remap_col(uint64_t E, const uint32_t *newid, uint32_t *col)
 }
 
 struct DevBufs {
-    void *p[6] = {};
+    void *p[3] = {};
     ~DevBufs()
     {
         for (void *q : p)
@@ -152,38 +211,36 @@ lt_status generate_rmat(int device, uint32_t scale, uint64_t E, double a, double
     cudaStream_t st = 0;
 
     DevBufs B;
-    uint32_t *d_deg, *d_col, *d_present, *d_newid;
-    uint64_t *d_rowptr, *d_tmp;
-    LT_CUDA_TRY(cudaMalloc(&B.p[0], 4 * V0));
-    d_deg = (uint32_t *)B.p[0];
-    LT_CUDA_TRY(cudaMalloc(&B.p[1], 8 * (V0 + 1)));
-    d_rowptr = (uint64_t *)B.p[1];
-    LT_CUDA_TRY(cudaMalloc(&B.p[2], 4 * (E ? E : 1)));
-    d_col = (uint32_t *)B.p[2];
-    LT_CUDA_TRY(cudaMalloc(&B.p[3], 8 * scan_tmp_elems(V0 + 1)));
-    d_tmp = (uint64_t *)B.p[3];
+    // one allocation for the per-vertex arrays (each costs a driver call of
+    // some 80 us, and its release as much), u64 ones first
+    const uint64_t tmp_n = scan_tmp_elems(V0 + 1);
+    LT_CUDA_TRY(cudaMalloc(&B.p[0], 8 * (V0 + 1 + tmp_n) + 4 * (V0 + V0 + 1)));
+    uint64_t *d_rowptr = (uint64_t *)B.p[0], *d_tmp = d_rowptr + V0 + 1;
+    uint32_t *d_deg = (uint32_t *)(d_tmp + tmp_n), *d_newid = d_deg + V0;
+    LT_CUDA_TRY(cudaMalloc(&B.p[1], 4 * (E ? E : 1)));
+    uint32_t *d_col = (uint32_t *)B.p[1];
 
     LT_CUDA_TRY(cudaMemsetAsync(d_deg, 0, 4 * V0, st));
     degrees_kernel<<<grid, kGenBlock, 0, st>>>(E, seed, (int)scale, t_src, d_deg);
     LT_CUDA_TRY(cudaGetLastError());
     LT_CUDA_TRY((exclusive_scan<uint32_t, uint64_t>(d_deg, V0, d_rowptr, d_tmp, st)));
-    fill_kernel<<<grid, kGenBlock, 0, st>>>(V0, d_rowptr, seed, (int)scale, t_d0, t_d1, d_col);
+    fill_kernel<<<grid, kGenBlock, 0, st>>>(V0, E, d_rowptr, seed, (int)scale, t_d0, t_d1, d_col);
     LT_CUDA_TRY(cudaGetLastError());
 
     // isolated-vertex removal: present = out-degree > 0 or some in-edge.
-    d_present = d_deg;  // reuse: deg is not needed after the flags are set
+    uint32_t *d_present = d_deg;  // reuse: deg is not needed after the flags are set
     mark_present<<<grid, kGenBlock, 0, st>>>(V0, d_deg, d_present);
     mark_targets<<<grid, kGenBlock, 0, st>>>(E, d_col, d_present);
     LT_CUDA_TRY(cudaGetLastError());
-    LT_CUDA_TRY(cudaMalloc(&B.p[4], 4 * (V0 + 1)));
-    d_newid = (uint32_t *)B.p[4];
     uint32_t *d_tmp32 = (uint32_t *)d_tmp;
     LT_CUDA_TRY((exclusive_scan<uint32_t, uint32_t>(d_present, V0, d_newid, d_tmp32, st)));
     uint32_t V = 0;
+    // page-locking the result's memory (2.2 ms for 64 MB) overlaps the kernels
+    LT_TRY(host_alloc(g.col_buf, 4ull * E, true));
     LT_CUDA_TRY(cudaMemcpyAsync(&V, d_newid + V0, 4, cudaMemcpyDeviceToHost, st));
     LT_CUDA_TRY(cudaStreamSynchronize(st));
-    LT_CUDA_TRY(cudaMalloc(&B.p[5], 8 * ((uint64_t)V + 1)));
-    uint64_t *d_rowptr2 = (uint64_t *)B.p[5];
+    LT_CUDA_TRY(cudaMalloc(&B.p[2], 8 * ((uint64_t)V + 1)));
+    uint64_t *d_rowptr2 = (uint64_t *)B.p[2];
     compact_rowptr<<<grid, kGenBlock, 0, st>>>(V0, d_present, d_newid, d_rowptr, d_rowptr2);
     remap_col<<<grid, kGenBlock, 0, st>>>(E, d_newid, d_col);
     LT_CUDA_TRY(cudaGetLastError());
@@ -191,7 +248,6 @@ lt_status generate_rmat(int device, uint32_t scale, uint64_t E, double a, double
     g.V = V;
     g.E = E;
     LT_TRY(host_alloc(g.rowptr_buf, 8ull * ((uint64_t)V + 1), true));
-    LT_TRY(host_alloc(g.col_buf, 4ull * E, true));
     LT_CUDA_TRY(cudaMemcpyAsync(g.rowptr_mut(), d_rowptr2, 8ull * ((uint64_t)V + 1), cudaMemcpyDeviceToHost, st));
     LT_CUDA_TRY(cudaMemcpyAsync(g.col_mut(), d_col, 4ull * E, cudaMemcpyDeviceToHost, st));
     LT_CUDA_TRY(cudaStreamSynchronize(st));
