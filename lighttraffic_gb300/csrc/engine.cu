@@ -101,14 +101,16 @@ lt_status walk_launch(int app, int start, const uint64_t *d_rowptr, const uint32
     a.W = W;
     a.length = length;
     a.run = run;
-    a.seed = seed;
-    a.thr = app == kWalk ? 0 : threshold53(prob);
+    a.keys = round_keys(seed);
+    a.lim = limit53(app == kWalk ? 0 : threshold53(prob));
+    a.by_v = mod_n(V);
     a.counts = d_counts;
     a.endpoints = d_endpoints;
     a.paths = d_paths;
     a.next = (uint64_t *)d_scratch;
     a.stats = d_stats;
     LT_CUDA_TRY(cudaMemsetAsync(d_scratch, 0, kScratchBytes, st));
+    cudaDeviceGetAttribute(&a.sms, cudaDevAttrMultiProcessorCount, device);
     const int grid = whole_grid(app, start, device, ctas_per_sm, layout);
     LT_CUDA_TRY(launch_walk_whole(a, app, start, grid, st, layout));
     return LT_OK;

@@ -74,6 +74,42 @@ LT_HD Rand4 philox4x32_10(uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3, ui
     return Rand4{c0, c1, c2, c3};
 }
 
+// The ten round keys of one seed.  A kernel whose walkers share a seed takes
+// them as an argument: its draws then read them as constant operands instead
+// of adding the Weyl increments in every round.
+struct RoundKeys {
+    uint32_t k0[10], k1[10];
+};
+
+inline RoundKeys round_keys(uint64_t seed)
+{
+    RoundKeys k;
+    for (int r = 0; r < 10; r++) {
+        k.k0[r] = (uint32_t)seed + (uint32_t)r * 0x9E3779B9u;
+        k.k1[r] = (uint32_t)(seed >> 32) + (uint32_t)r * 0xBB67AE85u;
+    }
+    return k;
+}
+
+LT_HD Rand4 philox4x32_10(uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3, const RoundKeys &k)
+{
+    constexpr uint32_t M0 = 0xD2511F53u, M1 = 0xCD9E8D57u;
+#pragma unroll
+    for (int r = 0; r < 10; r++) {
+        const uint64_t p0 = (uint64_t)M0 * c0, p1 = (uint64_t)M1 * c2;
+        c0 = (uint32_t)(p1 >> 32) ^ c1 ^ k.k0[r];
+        c1 = (uint32_t)p1;
+        c2 = (uint32_t)(p0 >> 32) ^ c3 ^ k.k1[r];
+        c3 = (uint32_t)p0;
+    }
+    return Rand4{c0, c1, c2, c3};
+}
+
+LT_HD Rand4 walk_draw(const RoundKeys &k, uint32_t c0, uint32_t tag, uint32_t run, uint64_t idx)
+{
+    return philox4x32_10(c0, tag | (run << 8), (uint32_t)idx, (uint32_t)(idx >> 32), k);
+}
+
 LT_HD Rand4 walk_draw(uint64_t seed, uint32_t c0, uint32_t tag, uint32_t run, uint64_t idx)
 {
     return philox4x32_10(c0, tag | (run << 8), (uint32_t)idx, (uint32_t)(idx >> 32), (uint32_t)seed,
@@ -84,6 +120,16 @@ LT_HD uint64_t r64_of(const Rand4 &r) { return ((uint64_t)r.x0 << 32) | r.x1; }
 LT_HD uint64_t m53_hi(const Rand4 &r) { return (((uint64_t)r.x0 << 32) | r.x1) >> 11; }
 LT_HD uint64_t m53_of(const Rand4 &r) { return (((uint64_t)r.x2 << 32) | r.x3) >> 11; }
 
+// m53 < thr as one 64-bit comparison: thr = floor(p 2^53) as x <= (thr << 11)
+// - 1 on the unshifted words (thr <= 2^53; never for thr = 0).
+struct Limit53 {
+    uint64_t last;
+    uint32_t some;  // thr > 0
+};
+inline Limit53 limit53(uint64_t thr) { return Limit53{(thr << 11) - 1u, thr != 0 ? 1u : 0u}; }
+LT_HD bool below_hi(const Rand4 &r, const Limit53 &l) { return l.some && (((uint64_t)r.x0 << 32) | r.x1) <= l.last; }
+LT_HD bool below(const Rand4 &r, const Limit53 &l) { return l.some && (((uint64_t)r.x2 << 32) | r.x3) <= l.last; }
+
 // floor(p * 2^53) for a float probability widened to double.
 inline uint64_t threshold53(float p)
 {
@@ -91,17 +137,6 @@ inline uint64_t threshold53(float p)
     if (!(d > 0.0)) return 0;
     if (d >= 1.0) return (uint64_t)1 << 53;
     return (uint64_t)(d * 9007199254740992.0);
-}
-
-// x mod d for 0 < d < 2^16: long division in base 2^16 with three 32-bit
-// remainders (every partial value stays below 2^32).
-LT_HD uint32_t mod64_small(uint64_t x, uint32_t d)
-{
-    const uint32_t hi = (uint32_t)(x >> 32), lo = (uint32_t)x;
-    uint32_t r = hi % d;
-    r = ((r << 16) | (lo >> 16)) % d;
-    r = ((r << 16) | (lo & 0xFFFFu)) % d;
-    return r;
 }
 
 LT_HD float rcp_f32(float d)
@@ -113,7 +148,50 @@ LT_HD float rcp_f32(float d)
 #endif
 }
 
-// x mod d for 2^16 <= d < 2^32 without 64-bit division: reduce the high word
+// 1 / d with a relative error of at most 2^-23 (PTX rcp.approx)
+LT_HD float rcp_approx_f32(float d)
+{
+#ifdef __CUDA_ARCH__
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+    return r;
+#else
+    return 1.0f / d;
+#endif
+}
+
+// x mod d for 0 < d <= 2^20 by folding: with m close below 2^32 / d, e = 2^32 -
+// m d is congruent to 2^32 and below 2 d, so hi 2^32 + lo = hi e + lo (mod d).
+// Three folds bring x below 2^32 + e, one more below 2^32 (d <= 2^20: the
+// folds' high words are below 2^32, 2^21, 2^10 + 1 and 2), and one
+// multiplication by m leaves less than 3 d.
+//
+// m: a single-precision reciprocal scaled down by 2^-22 (so that it never
+// exceeds 2^32 / d; its relative error stays below 2^-21) and one Newton step
+// in integers, after which floor(2^32 / d) - 1 <= m <= 2^32 / d.
+//
+// Most of it is multiply-adds: the walk kernels are bound by the integer ALU,
+// which three native 32-bit remainders (d < 2^16) kept busy instead.
+constexpr uint32_t kFoldMax = 1u << 20;
+
+LT_HD uint32_t mod64_fold(uint32_t hi, uint32_t lo, uint32_t d)
+{
+    const uint32_t m0 = (uint32_t)(rcp_approx_f32((float)d) * 4294966272.0f);
+    const uint32_t m = m0 + mulhi32(m0, 0u - m0 * d);
+    const uint32_t e = 0u - m * d;
+    uint64_t y = (uint64_t)hi * e + lo;
+    y = (uint64_t)(uint32_t)(y >> 32) * e + (uint32_t)y;
+    y = (uint64_t)(uint32_t)(y >> 32) * e + (uint32_t)y;
+    const uint32_t w = (uint32_t)(y >> 32) * e + (uint32_t)y;
+    uint32_t r = w - mulhi32(w, m) * d;
+    // r < 3 d: the unsigned minimum takes the subtraction only where it does not wrap
+    uint32_t t = r - d;
+    r = t < r ? t : r;
+    t = r - d;
+    return t < r ? t : r;
+}
+
+// x mod d for 2^16 <= d < 2^32 (used above 2^20) without 64-bit division: reduce the high word
 // (32-bit remainder), estimate the quotient of the remaining t = r1 2^32 + lo
 // (t < d 2^32) in single precision, then correct in integers.  The estimate's
 // relative error is below 2^-21, so after the first correction |r| < 1024 d;
@@ -143,10 +221,25 @@ LT_HD uint64_t mod_u64(uint64_t r, uint64_t n)
 {
     if ((n >> 32) == 0) {
         const uint32_t d = (uint32_t)n;
-        return d <= 0xFFFFu ? mod64_small(r, d) : mod64_large(r, d);
+        return d <= kFoldMax ? mod64_fold((uint32_t)(r >> 32), (uint32_t)r, d) : mod64_large(r, d);
     }
     return r % n;
 }
+
+// r % n for an n known before the launch (the vertex count): inv =
+// floor((2^64 - 1) / n) gives a quotient at most one too small.
+struct ModN {
+    uint64_t inv;
+    uint32_t n;
+};
+inline ModN mod_n(uint32_t n) { return ModN{UINT64_MAX / n, n}; }
+#ifdef __CUDACC__
+__device__ __forceinline__ uint32_t mod_by(const ModN &m, uint64_t x)
+{
+    const uint64_t rem = x - __umul64hi(x, m.inv) * m.n;
+    return (uint32_t)(rem >= m.n ? rem - m.n : rem);
+}
+#endif
 
 // PPR walk length (src/walk/SingleSource.h:11-18): step = 2, then one more
 // for every draw with U > prob.
@@ -161,6 +254,62 @@ LT_HD uint32_t ppr_length(uint64_t seed, uint32_t run, uint64_t idx, uint64_t th
         step++;
     }
 }
+
+#ifdef __CUDACC__
+// ppr_length for the lanes with `need`, by the whole warp (every lane calls
+// it, converged; 0 for the others).  While more than 16 lengths are open each
+// lane draws for its own walker; the open ones then get 2, 4, ... lanes each,
+// which take their next draws in parallel.  A warp's longest walk would
+// otherwise set the number of rounds: 12 on average for 32 walks at stop
+// probability 0.15, against 6 here.
+__device__ __forceinline__ uint32_t warp_ppr_length(bool need, const RoundKeys &keys, uint32_t run, uint64_t idx,
+                                                    const Limit53 &lim)
+{
+    const unsigned full = 0xFFFFFFFFu, lane = threadIdx.x & 31u;
+    uint32_t t = 0, len = 0;
+    bool open = need;
+    unsigned m = __ballot_sync(full, open);
+    while (__popc(m) > 16) {
+        if (open) {
+            const Rand4 r = walk_draw(keys, t, kTagInit, run, idx);
+            const bool a = below_hi(r, lim);
+            if (a || below(r, lim)) {
+                len = 2u + 2u * t + (a ? 0u : 1u);
+                open = false;
+            }
+            t++;
+        }
+        m = __ballot_sync(full, open);
+    }
+    while (m) {
+        const uint32_t n = (uint32_t)__popc(m);
+        const uint32_t lg = 31u - (uint32_t)__clz((int)(32u / n)), g = 1u << lg;
+        // lane of the (lane >> lg)-th open walker (the last one for lanes left over)
+        const uint32_t want = (lane >> lg) < n ? lane >> lg : n - 1u;
+        uint32_t src = 0;
+#pragma unroll
+        for (uint32_t b = 16; b > 0; b >>= 1)
+            if ((uint32_t)__popc(m & ((1u << (src + b)) - 1u)) <= want) src += b;
+        const uint32_t wt = __shfl_sync(full, t, src) + (lane & (g - 1u));
+        const uint64_t wi = __shfl_sync(full, idx, src);
+        const Rand4 r = walk_draw(keys, wt, kTagInit, run, wi);
+        const bool a = below_hi(r, lim);
+        const unsigned ends = __ballot_sync(full, a || below(r, lim)), at_a = __ballot_sync(full, a);
+        if (open) {
+            const uint32_t first = ((uint32_t)__popc(m & ((1u << lane) - 1u))) << lg;
+            const unsigned mine = (ends >> first) & (g == 32u ? full : (1u << g) - 1u);
+            if (mine) {
+                const uint32_t f = (uint32_t)__ffs((int)mine) - 1u;
+                len = 2u + 2u * (t + f) + ((at_a >> (first + f)) & 1u ? 0u : 1u);
+                open = false;
+            }
+            t += g;
+        }
+        m = __ballot_sync(full, open);
+    }
+    return len;
+}
+#endif
 
 LT_HD uint32_t start_vertex(int start, uint32_t source, uint32_t V, uint64_t seed, uint32_t run, uint64_t idx)
 {

@@ -17,6 +17,7 @@
 //    the read-only path; counters are u64 reductions resolved in L2.  Column
 //    loads are evict-first, row offsets and counters evict-last (mem.cuh).
 #include <algorithm>
+#include <type_traits>
 
 #include "common.h"
 #include "lt_core.cuh"
@@ -30,33 +31,45 @@ namespace {
 constexpr unsigned kFull = 0xFFFFFFFFu;
 // idle lanes a warp waits for before refilling them (all lanes: always): the
 // refill sits on the warp's critical path and PPR's geometric walk lengths
-// would otherwise trigger one nearly every iteration
-constexpr int kRefillMin = 24;
+// would otherwise trigger one nearly every iteration (2|V| PPR walks on
+// RMAT 2^20 / 2^24, whole call: 24 242 us, 16 234, 12 238, 8 253)
+constexpr int kRefillMin = 16;
 
 struct Hints {
     uint64_t keep, stream;
 };
-__device__ __forceinline__ uint32_t ldg_u32(const uint32_t *p, const Hints &h) { return ld_nc_stream_u32(p, h.stream); }
 
 // first edge and degree of v
 template <int L>
-__device__ __forceinline__ void row_range(const WholeArgs &a, uint32_t v, const Hints &h, uint64_t &first,
-                                          uint64_t &deg)
+struct Row {
+    using Edge = typename std::conditional<L == kLayoutWide, uint64_t, uint32_t>::type;
+    Edge first, deg;
+};
+
+template <int L>
+__device__ __forceinline__ Row<L> row_range(const WholeArgs &a, uint32_t v, const Hints &h)
 {
-    if (L == kLayoutPacked) {
+    Row<L> r;
+    if constexpr (L == kLayoutPacked) {
         // the even words never change during a launch (only the counters
         // beside them do), so the read-only path serves them
-        const uint32_t f = ld_nc_u32(a.rows + 2ull * v, h.keep);
-        first = f;
-        deg = ld_nc_u32(a.rows + 2ull * v + 2, h.keep) - f;
-    } else if (L == kLayoutCompact) {
-        const uint32_t f = ld_nc_u32(a.rowptr32 + v, h.keep);
-        first = f;
-        deg = ld_nc_u32(a.rowptr32 + v + 1, h.keep) - f;
+        r.first = ld_nc_u32(a.rows + 2ull * v, h.keep);
+        r.deg = ld_nc_u32(a.rows + 2ull * v + 2, h.keep) - r.first;
+    } else if constexpr (L == kLayoutCompact) {
+        r.first = ld_nc_u32(a.rowptr32 + v, h.keep);
+        r.deg = ld_nc_u32(a.rowptr32 + v + 1, h.keep) - r.first;
     } else {
-        first = ld_nc_u64(a.rowptr + v, h.keep);
-        deg = ld_nc_u64(a.rowptr + v + 1, h.keep) - first;
+        r.first = ld_nc_u64(a.rowptr + v, h.keep);
+        r.deg = ld_nc_u64(a.rowptr + v + 1, h.keep) - r.first;
     }
+    return r;
+}
+
+// the neighbour that draw r picks from a row that is not empty
+template <int L>
+__device__ __forceinline__ uint32_t pick(const WholeArgs &a, const Row<L> &row, const Rand4 &r, const Hints &h)
+{
+    return ld_nc_stream64_u32(a.col + row.first + mod_u64(r64_of(r), row.deg), h.stream);
 }
 
 template <int L>
@@ -71,134 +84,161 @@ __device__ __forceinline__ void count1(const WholeArgs &a, uint32_t v, const Hin
 }
 
 template <int APP, int START, int C>
-__global__ void __launch_bounds__(kWholeBlock) walk_whole_kernel(WholeArgs a)
+__global__ void __launch_bounds__(kWholeBlock, 8) walk_whole_kernel(const __grid_constant__ WholeArgs a)
 {
     const int lane = threadIdx.x & 31;
-    const unsigned lt_mask = (1u << lane) - 1u;
     const Hints h{l2_policy_evict_last(), l2_policy_evict_first()};
 
     uint32_t cur = 0, step = 0;
     uint64_t idx = 0;
     bool active = false;
+    // walkers no longer to be had: the counter has passed W
     bool exhausted = false;
-    uint32_t hop = 0;  // hops taken (walk app path position)
-    uint64_t n_upd = 0, n_mov = 0, n_tel = 0;
+    // the first walkers are dealt out without the counter, 32 to each warp,
+    // the warps of the same number in their CTAs before the next ones, so
+    // that few walkers spread over all SMs
+    const uint64_t dealt = (uint64_t)gridDim.x * kWholeBlock;
+    bool first_deal = true;
+    uint32_t n_mov = 0, n_end = 0;  // hops taken; walks that ended at a vertex without out-edges
+    Rand4 r{};                      // PageRank: the draw of the walker's next step
 
     while (true) {
-        const unsigned idle = __ballot_sync(kFull, !active);
-        if (idle != 0u && !exhausted && (__popc(idle) >= kRefillMin || idle == kFull)) {
-            const int leader = __ffs(idle) - 1;
-            unsigned long long base = 0;
-            if (lane == leader) base = atomicAdd((unsigned long long *)a.next, (unsigned long long)__popc(idle));
-            base = __shfl_sync(kFull, base, leader);
-            if (base + __popc(idle) >= a.W) exhausted = true;
+        const unsigned busy = __ballot_sync(kFull, active);
+        if (__popc(busy) <= 32 - kRefillMin && !exhausted) {
+            const unsigned idle = ~busy;
+            uint64_t base;
+            if (first_deal) {
+                base = 32ull * ((uint64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x);
+                exhausted = dealt >= a.W;
+                first_deal = false;
+            } else {
+                unsigned long long got = 0;
+                if (lane == 0) got = atomicAdd((unsigned long long *)a.next, (unsigned long long)__popc(idle));
+                base = dealt + __shfl_sync(kFull, got, 0);
+                exhausted = base + __popc(idle) >= a.W;
+            }
+            bool fresh = false;
             if (!active) {
-                const uint64_t my = base + __popc(idle & lt_mask);
+                const uint64_t my = base + __popc(idle & ((1u << lane) - 1u));
                 if (my < a.W) {
+                    fresh = active = true;
                     idx = my;
-                    cur = start_vertex(START, a.source, a.V, a.seed, a.run, idx);
-                    if (APP == kPPR) {
-                        step = ppr_length(a.seed, a.run, idx, a.thr);
-                    } else {
-                        step = a.length;
-                    }
-                    hop = 0;
+                    if (START == kStartSource)
+                        cur = a.source;
+                    else if (START == kStartPerVertex)
+                        cur = mod_by(a.by_v, idx);
+                    else
+                        cur = mod_by(a.by_v, r64_of(walk_draw(a.keys, 0, kTagInit, a.run, idx)));
+                    step = a.length;
                     if (APP == kWalk && a.paths) a.paths[idx * (uint64_t)(a.length + 1)] = cur;
-                    active = true;
                 }
             }
-        }
-        if (__ballot_sync(kFull, active) == 0u) {
-            if (exhausted) break;
-            continue;
+            if (APP == kPPR) {
+                const uint32_t len = warp_ppr_length(fresh, a.keys, a.run, idx, a.lim);
+                if (fresh) step = len;
+            }
+            if (APP == kPageRank && fresh) r = walk_draw(a.keys, step, kTagStep, a.run, idx);
+        } else if (busy == 0u) {
+            break;
         }
         if (!active) continue;
 
-        const uint32_t s = step;
-        n_upd++;
+        // The draws do not depend on the graph: they are made between the
+        // row's loads and their first use.
         if (APP == kPPR) {
-            // app/ppr.cu:22-42
-            if (s == 1) {
-                count1<C>(a, cur, h);
-                active = false;
+            // app/ppr.cu:22-42; step >= 2 here, and a walk whose step comes
+            // down to 1 is counted right away
+            const Row<C> row = row_range<C>(a, cur, h);
+            r = walk_draw(a.keys, step, kTagStep, a.run, idx);
+            if (row.deg > 0) {
+                cur = pick<C>(a, row, r, h);
+                n_mov++;
+                step--;
             } else {
-                step = s - 1;
-                uint64_t first, deg;
-                row_range<C>(a, cur, h, first, deg);
-                if (deg > 0) {
-                    const Rand4 r = walk_draw(a.seed, s, kTagStep, a.run, idx);
-                    cur = ldg_u32(a.col + first + mod_u64(r64_of(r), deg), h);
-                    n_mov++;
-                } else {
-                    count1<C>(a, cur, h);
-                    active = false;
-                }
+                step = 1;
             }
+            active = step != 1;
+            if (!active) count1<C>(a, cur, h);
         } else if (APP == kPageRank) {
             // app/pagerank.cu:26-44; a vertex without out-edges teleports.
             count1<C>(a, cur, h);
-            if (s == 1) {
+            step--;
+            if (step == 0) {
                 active = false;
             } else {
-                step = s - 1;
-                const Rand4 r = walk_draw(a.seed, s, kTagStep, a.run, idx);
-                const uint64_t r64 = r64_of(r);
-                bool tele = m53_of(r) >= a.thr;
-                if (!tele) {
-                    uint64_t first, deg;
-                    row_range<C>(a, cur, h, first, deg);
-                    if (deg > 0) {
-                        cur = ldg_u32(a.col + first + mod_u64(r64, deg), h);
-                        n_mov++;
-                    } else {
-                        tele = true;
-                    }
-                }
-                if (tele) {
-                    cur = (uint32_t)mod_u64(r64, a.V);
-                    n_tel++;
+                const Rand4 now = r;
+                Row<C> row{};
+                if (below(now, a.lim)) row = row_range<C>(a, cur, h);
+                r = walk_draw(a.keys, step, kTagStep, a.run, idx);
+                if (row.deg > 0) {
+                    cur = pick<C>(a, row, now, h);
+                    n_mov++;
+                } else {
+                    cur = mod_by(a.by_v, r64_of(now));
                 }
             }
         } else {
             // app/genericwalk.cu:22-32
-            uint64_t first, deg;
-            row_range<C>(a, cur, h, first, deg);
-            uint32_t *path = a.paths ? a.paths + idx * (uint64_t)(a.length + 1) : nullptr;
-            if (deg > 0) {
-                const Rand4 r = walk_draw(a.seed, s, kTagStep, a.run, idx);
-                cur = ldg_u32(a.col + first + mod_u64(r64_of(r), deg), h);
+            const Row<C> row = row_range<C>(a, cur, h);
+            r = walk_draw(a.keys, step, kTagStep, a.run, idx);
+            uint32_t *path = a.paths ? a.paths + idx * (uint64_t)(a.length + 1) + (a.length - step) : nullptr;
+            if (row.deg > 0) {
+                cur = pick<C>(a, row, r, h);
                 n_mov++;
-                hop++;
-                if (path) path[hop] = cur;
-                step = s - 1;
+                if (path) path[1] = cur;
+                step--;
             } else {
-                if (path) {
-                    for (uint32_t h = hop + 1; h <= a.length; h++) path[h] = kInvalidNode;
-                }
+                if (path)
+                    for (uint32_t k = 1; k <= step; k++) path[k] = kInvalidNode;
+                n_end++;
                 step = 0;
             }
-            if (step == 0) active = false;
+            active = step != 0;
         }
         if (!active && a.endpoints) a.endpoints[idx] = cur;
     }
 
-    // Warp-reduce the statistics, one atomic per warp.
+    // Statistics: one atomic per CTA and counter (one per warp would queue
+    // some 30 000 atomics on one line at the end of every launch).  A PPR
+    // walk makes one update per hop and one that ends it, a PageRank walk
+    // a.length updates of which all but the last hop or teleport, a generic
+    // walk one per hop and one where it ends early.
+    if (!a.stats) return;
+    __shared__ unsigned long long s_mov, s_end;
+    if (threadIdx.x == 0) s_mov = s_end = 0;
+    __syncthreads();
+    uint64_t w_mov = n_mov, w_end = n_end;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
-        n_upd += __shfl_down_sync(kFull, n_upd, o);
-        n_mov += __shfl_down_sync(kFull, n_mov, o);
-        n_tel += __shfl_down_sync(kFull, n_tel, o);
+        w_mov += __shfl_down_sync(kFull, w_mov, o);
+        if (APP == kWalk) w_end += __shfl_down_sync(kFull, w_end, o);
     }
-    if (lane == 0 && a.stats) {
-        atomicAdd((unsigned long long *)&a.stats[0], (unsigned long long)n_upd);
-        atomicAdd((unsigned long long *)&a.stats[1], (unsigned long long)n_mov);
-        atomicAdd((unsigned long long *)&a.stats[2], (unsigned long long)n_tel);
+    if (lane == 0 && w_mov + w_end) {
+        atomicAdd(&s_mov, (unsigned long long)w_mov);
+        if (APP == kWalk) atomicAdd(&s_end, (unsigned long long)w_end);
     }
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    unsigned long long upd = APP == kWalk ? s_mov + s_end : APP == kPPR ? s_mov : 0, tel = 0;
+    if (APP == kPageRank) tel = 0ull - s_mov;
+    if (blockIdx.x == 0) {
+        if (APP == kPPR) upd += a.W;
+        if (APP == kPageRank) {
+            upd += a.W * a.length;
+            tel += a.W * (a.length - 1);
+        }
+    }
+    if (upd) atomicAdd((unsigned long long *)&a.stats[0], upd);
+    if (s_mov) atomicAdd((unsigned long long *)&a.stats[1], s_mov);
+    if (tel) atomicAdd((unsigned long long *)&a.stats[2], tel);
 }
 
 template <int APP, int START, int C>
 cudaError_t launch_t(const WholeArgs &a, int grid, cudaStream_t st)
 {
+    // no more CTAs than have walkers, but one per SM
+    const uint64_t need = std::max<uint64_t>(a.sms, (a.W + kWholeBlock - 1) / kWholeBlock);
+    if ((uint64_t)grid > need) grid = (int)need;
     walk_whole_kernel<APP, START, C><<<grid, kWholeBlock, 0, st>>>(a);
     return cudaGetLastError();
 }

@@ -4,6 +4,8 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "lt_core.cuh"
+
 namespace lt {
 
 constexpr int kWholeBlock = 256;
@@ -16,8 +18,6 @@ struct WholeArgs {
     uint64_t W;              // walkers in this pass
     uint32_t length;         // PageRank / walk length
     uint32_t run;            // epoch index (random stream selector)
-    uint64_t seed;
-    uint64_t thr;            // floor(p 2^53): PPR stop prob or PageRank alpha
     uint64_t *counts;        // u64[V] or null (walk app)
     uint32_t *endpoints;     // u32[W] or null
     uint32_t *paths;         // u32[W*(length+1)] or null (walk app)
@@ -33,6 +33,10 @@ struct WholeArgs {
     // of v (u32), rows[2v+1] = v's counter (u32).  The row offsets an update
     // reads and the counter it increments share one 32-byte sector.
     uint32_t *rows;
+    int sms;                 // SMs of the device
+    RoundKeys keys;          // of the seed
+    Limit53 lim;             // of floor(p 2^53): PPR stop prob or PageRank alpha
+    ModN by_v;               // remainders by V
 };
 
 enum Layout : int { kLayoutWide = 0, kLayoutCompact = 1, kLayoutPacked = 2 };
