@@ -36,6 +36,7 @@ lt_status grow(void **p, uint64_t &cap, uint64_t need_bytes)
 
 // Scratch layout of the resident step kernel: the next-walker counter.
 constexpr size_t kScratchBytes = 256;
+constexpr size_t kClearBytes = kScratchBytes + 256;  // and the engine's statistics behind it
 
 }  // namespace
 
@@ -49,13 +50,27 @@ __global__ void narrow_kernel(uint32_t *dst, const uint64_t *src, uint64_t n)
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) dst[i] = (uint32_t)src[i];
 }
 
-__global__ void widen_kernel(uint64_t *dst, const uint32_t *src, uint64_t n)
+// Counters widened to u64 (dst: device or mapped host memory) and the pass's
+// three statistics to mapped host memory.
+__global__ void widen_kernel(uint64_t *dst, const uint32_t *src, uint64_t n, uint64_t *host_stats, const uint64_t *stats)
 {
+    if (blockIdx.x == 0 && threadIdx.x < 3 && host_stats) host_stats[threadIdx.x] = stats[threadIdx.x];
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) dst[i] = src[i];
 }
 
 unsigned stream_blocks(uint64_t n, int sms) { return (unsigned)std::min<uint64_t>((n + 255) / 256, (uint64_t)sms * 8); }
+
+// The device's view of page-locked host memory, null where p is something else.
+uint64_t *mapped(uint64_t *p)
+{
+    cudaPointerAttributes at{};
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    return at.type == cudaMemoryTypeHost ? (uint64_t *)at.devicePointer : nullptr;
+}
 
 // Counter updates of one launch: one per walk (PPR), one per step (PageRank).
 uint64_t count_updates(int app, uint64_t W, uint32_t length)
@@ -71,7 +86,7 @@ lt_status walk_launch(int app, int start, const uint64_t *d_rowptr, const uint32
                       uint32_t V, uint32_t source, uint64_t W, uint32_t length, float prob, uint32_t run,
                       uint64_t seed, uint64_t *d_counts, uint32_t *d_counts32, uint32_t *d_endpoints,
                       uint32_t *d_paths, void *d_scratch, uint64_t *d_stats, cudaStream_t st, int ctas_per_sm,
-                      uint32_t *d_rows = nullptr)
+                      uint32_t *d_rows = nullptr, bool scratch_clear = false)
 {
     const int layout = d_rows ? kLayoutPacked : d_rowptr32 ? kLayoutCompact : kLayoutWide;
     if (app < kPPR || app > kWalk) return fail(LT_ERR_INVALID, "unknown app %d", app);
@@ -104,13 +119,15 @@ lt_status walk_launch(int app, int start, const uint64_t *d_rowptr, const uint32
     a.keys = round_keys(seed);
     a.lim = limit53(app == kWalk ? 0 : threshold53(prob));
     a.by_v = mod_n(V);
+    // twice the mean length, capped where the float would not fit
+    a.long_len = app == kPPR ? (uint32_t)std::min(1e9, 2.0 / prob) + 1u : 0u;
     a.counts = d_counts;
     a.endpoints = d_endpoints;
     a.paths = d_paths;
     a.next = (uint64_t *)d_scratch;
     a.stats = d_stats;
-    LT_CUDA_TRY(cudaMemsetAsync(d_scratch, 0, kScratchBytes, st));
-    cudaDeviceGetAttribute(&a.sms, cudaDevAttrMultiProcessorCount, device);
+    if (!scratch_clear) LT_CUDA_TRY(cudaMemsetAsync(d_scratch, 0, kScratchBytes, st));
+    a.sms = whole_sms(device);
     const int grid = whole_grid(app, start, device, ctas_per_sm, layout);
     LT_CUDA_TRY(launch_walk_whole(a, app, start, grid, st, layout));
     return LT_OK;
@@ -234,19 +251,25 @@ lt_status engine_create(lt_graph *g, const lt_engine_cfg &cfg, lt_engine **out)
         return bail(fail(LT_ERR_CUDA, "stream / event creation failed"));
     if ((e->resident && (cudaMalloc(&e->d_rowptr, 8ull * ((uint64_t)g->V + 1)) != cudaSuccess ||
                          cudaMalloc(&e->d_col, 4ull * (g->E ? g->E : 1)) != cudaSuccess)) ||
-        cudaMalloc(&e->d_counts, 8ull * g->V) != cudaSuccess ||
-        cudaMalloc(&e->d_scratch, walk_scratch_bytes()) != cudaSuccess ||
-        cudaMalloc(&e->d_stats, 64) != cudaSuccess) {
+        cudaMalloc(&e->d_counts, 8ull * g->V) != cudaSuccess) {
         cudaGetLastError();
         return bail(fail(LT_ERR_NOMEM, "device allocation for the resident graph failed"));
     }
-    // compact layout of the resident graph: u32 row offsets and counters
-    if (e->resident && g->E < (1ull << 32)) {
-        if (cudaMalloc(&e->d_rowptr32, 4ull * ((uint64_t)g->V + 1)) != cudaSuccess ||
-            cudaMalloc(&e->d_counts32, 4ull * g->V) != cudaSuccess) {
-            cudaGetLastError();
-            return bail(fail(LT_ERR_NOMEM, "device allocation for the compact row offsets failed"));
-        }
+    // compact layout of the resident graph: u32 row offsets and counters.
+    // Scratch, statistics and u32 counters lie together: one memset clears
+    // them.
+    const bool compact = e->resident && g->E < (1ull << 32);
+    if (cudaMalloc(&e->d_scratch, kClearBytes + (compact ? 4ull * g->V : 0)) != cudaSuccess ||
+        (compact && cudaMalloc(&e->d_rowptr32, 4ull * ((uint64_t)g->V + 1)) != cudaSuccess)) {
+        cudaGetLastError();
+        return bail(fail(LT_ERR_NOMEM, "device allocation for the compact row offsets failed"));
+    }
+    e->d_stats = (uint64_t *)((uint8_t *)e->d_scratch + kScratchBytes);
+    if (compact) e->d_counts32 = (uint32_t *)((uint8_t *)e->d_scratch + kClearBytes);
+    {
+        const lt_status s = host_alloc(e->h_stats, 64, true);
+        if (s != LT_OK) return bail(s);
+        e->h_stats_dev = mapped((uint64_t *)e->h_stats.ptr);
     }
     if (!e->resident) {
         lt_status s = ooc_create(e, &e->ooc);
@@ -263,9 +286,10 @@ void engine_destroy(lt_engine *e)
     if (e->s_compute) cudaStreamSynchronize(e->s_compute);
     if (e->ooc) ooc_destroy(e->ooc);
     if (e->batch) batch_destroy(e->batch);
-    for (void *p : {(void *)e->d_rowptr, (void *)e->d_col, (void *)e->d_counts, e->d_scratch, (void *)e->d_stats,
-                    (void *)e->d_endpoints, (void *)e->d_paths, (void *)e->d_rowptr32, (void *)e->d_counts32})
+    for (void *p : {(void *)e->d_rowptr, (void *)e->d_col, (void *)e->d_counts, e->d_scratch, (void *)e->d_endpoints,
+                    (void *)e->d_paths, (void *)e->d_rowptr32})
         if (p) cudaFree(p);
+    host_free(e->h_stats);
     if (e->ev_k0) cudaEventDestroy(e->ev_k0);
     if (e->ev_k1) cudaEventDestroy(e->ev_k1);
     for (cudaStream_t s : {e->s_compute, e->s_copy, e->s_copyback})
@@ -342,38 +366,46 @@ lt_status engine_run(lt_engine *e, int app, int start, uint32_t source, uint64_t
     // compact layout while every counter total of the call fits 32 bits
     const uint64_t upd = count_updates(app, W, length);
     const bool compact = e->d_rowptr32 && (upd == 0 || upd <= (((1ull << 32) - 1) / runs));
-    if (app != kWalk) {
-        if (compact)
-            LT_CUDA_TRY(cudaMemsetAsync(e->d_counts32, 0, 4ull * g.V, st));
-        else
-            LT_CUDA_TRY(cudaMemsetAsync(e->d_counts, 0, 8ull * g.V, st));
-    }
-    LT_CUDA_TRY(cudaMemsetAsync(e->d_stats, 0, 64, st));
+    const bool cnt = app != kWalk;
+    LT_CUDA_TRY(cudaMemsetAsync(e->d_scratch, 0, kClearBytes + (cnt && compact ? 4ull * g.V : 0), st));
+    if (cnt && !compact) LT_CUDA_TRY(cudaMemsetAsync(e->d_counts, 0, 8ull * g.V, st));
     if (endpoints_out) LT_TRY(grow((void **)&e->d_endpoints, e->endpoints_cap, 4 * W));
     if (paths_out) LT_TRY(grow((void **)&e->d_paths, e->paths_cap, 4 * W * ((uint64_t)length + 1)));
     LT_CUDA_TRY(cudaEventRecord(e->ev_k0, st));
     for (uint32_t r = 0; r < runs; r++) {
-        const bool cnt = app != kWalk;
         LT_TRY(walk_launch(app, start, compact ? nullptr : e->d_rowptr, compact ? e->d_rowptr32 : nullptr, e->d_col,
                            g.V, source, W, length, prob, run_base + r, e->cfg.seed,
                            cnt && !compact ? e->d_counts : nullptr, cnt && compact ? e->d_counts32 : nullptr,
                            endpoints_out ? e->d_endpoints : nullptr, paths_out ? e->d_paths : nullptr, e->d_scratch,
-                           e->d_stats, st, e->cfg.ctas_per_sm));
+                           e->d_stats, st, e->cfg.ctas_per_sm, nullptr, r == 0));
         e->stats.kernel_launches++;
         e->stats.computing_calls++;
     }
-    if (compact && app != kWalk) {
-        widen_kernel<<<stream_blocks(g.V, e->sms), 256, 0, st>>>(e->d_counts, e->d_counts32, g.V);
+    uint64_t *hs = (uint64_t *)e->h_stats.ptr;
+    bool counts_done = false;
+    if (compact && cnt) {
+        // straight into the caller's page-locked memory where that is what it
+        // is (both of its ends): a copy after the kernel costs 9 us more at
+        // V = 47 000 and 13 us at V = 4.6 M
+        uint64_t *dst = e->d_counts, *host_stats = e->h_stats_dev;
+        if (counts_out) {
+            uint64_t *first = mapped(counts_out), *last = mapped(counts_out + (g.V - 1));
+            counts_done = first && last == first + (g.V - 1);
+            if (counts_done) dst = first;
+        }
+        widen_kernel<<<stream_blocks(g.V, e->sms), 256, 0, st>>>(dst, e->d_counts32, g.V, host_stats, e->d_stats);
         LT_CUDA_TRY(cudaGetLastError());
         e->stats.kernel_launches++;
+        if (!host_stats) LT_CUDA_TRY(cudaMemcpyAsync(hs, e->d_stats, 24, cudaMemcpyDeviceToHost, st));
+    } else {
+        LT_CUDA_TRY(cudaMemcpyAsync(hs, e->d_stats, 24, cudaMemcpyDeviceToHost, st));
     }
     LT_CUDA_TRY(cudaEventRecord(e->ev_k1, st));
-    if (counts_out) LT_CUDA_TRY(cudaMemcpyAsync(counts_out, e->d_counts, 8ull * g.V, cudaMemcpyDeviceToHost, st));
+    if (counts_out && !counts_done)
+        LT_CUDA_TRY(cudaMemcpyAsync(counts_out, e->d_counts, 8ull * g.V, cudaMemcpyDeviceToHost, st));
     if (endpoints_out) LT_CUDA_TRY(cudaMemcpyAsync(endpoints_out, e->d_endpoints, 4 * W, cudaMemcpyDeviceToHost, st));
     if (paths_out)
         LT_CUDA_TRY(cudaMemcpyAsync(paths_out, e->d_paths, 4 * W * ((uint64_t)length + 1), cudaMemcpyDeviceToHost, st));
-    uint64_t hs[3] = {0, 0, 0};
-    LT_CUDA_TRY(cudaMemcpyAsync(hs, e->d_stats, sizeof hs, cudaMemcpyDeviceToHost, st));
     LT_CUDA_TRY(cudaStreamSynchronize(st));
     float kms = 0;
     cudaEventElapsedTime(&kms, e->ev_k0, e->ev_k1);

@@ -36,7 +36,9 @@ struct lt_engine {
 
     uint64_t *d_counts = nullptr;  // u64[V]
     void *d_scratch = nullptr;     // lt_walk_scratch_bytes()
-    uint64_t *d_stats = nullptr;   // u64[3]
+    uint64_t *d_stats = nullptr;   // u64[3], behind the scratch
+    lt::HostBuf h_stats;           // page-locked u64[3] and its device view
+    uint64_t *h_stats_dev = nullptr;
     uint32_t *d_endpoints = nullptr;
     uint64_t endpoints_cap = 0;
     uint32_t *d_paths = nullptr;

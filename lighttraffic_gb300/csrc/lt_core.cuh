@@ -255,62 +255,6 @@ LT_HD uint32_t ppr_length(uint64_t seed, uint32_t run, uint64_t idx, uint64_t th
     }
 }
 
-#ifdef __CUDACC__
-// ppr_length for the lanes with `need`, by the whole warp (every lane calls
-// it, converged; 0 for the others).  While more than 16 lengths are open each
-// lane draws for its own walker; the open ones then get 2, 4, ... lanes each,
-// which take their next draws in parallel.  A warp's longest walk would
-// otherwise set the number of rounds: 12 on average for 32 walks at stop
-// probability 0.15, against 6 here.
-__device__ __forceinline__ uint32_t warp_ppr_length(bool need, const RoundKeys &keys, uint32_t run, uint64_t idx,
-                                                    const Limit53 &lim)
-{
-    const unsigned full = 0xFFFFFFFFu, lane = threadIdx.x & 31u;
-    uint32_t t = 0, len = 0;
-    bool open = need;
-    unsigned m = __ballot_sync(full, open);
-    while (__popc(m) > 16) {
-        if (open) {
-            const Rand4 r = walk_draw(keys, t, kTagInit, run, idx);
-            const bool a = below_hi(r, lim);
-            if (a || below(r, lim)) {
-                len = 2u + 2u * t + (a ? 0u : 1u);
-                open = false;
-            }
-            t++;
-        }
-        m = __ballot_sync(full, open);
-    }
-    while (m) {
-        const uint32_t n = (uint32_t)__popc(m);
-        const uint32_t lg = 31u - (uint32_t)__clz((int)(32u / n)), g = 1u << lg;
-        // lane of the (lane >> lg)-th open walker (the last one for lanes left over)
-        const uint32_t want = (lane >> lg) < n ? lane >> lg : n - 1u;
-        uint32_t src = 0;
-#pragma unroll
-        for (uint32_t b = 16; b > 0; b >>= 1)
-            if ((uint32_t)__popc(m & ((1u << (src + b)) - 1u)) <= want) src += b;
-        const uint32_t wt = __shfl_sync(full, t, src) + (lane & (g - 1u));
-        const uint64_t wi = __shfl_sync(full, idx, src);
-        const Rand4 r = walk_draw(keys, wt, kTagInit, run, wi);
-        const bool a = below_hi(r, lim);
-        const unsigned ends = __ballot_sync(full, a || below(r, lim)), at_a = __ballot_sync(full, a);
-        if (open) {
-            const uint32_t first = ((uint32_t)__popc(m & ((1u << lane) - 1u))) << lg;
-            const unsigned mine = (ends >> first) & (g == 32u ? full : (1u << g) - 1u);
-            if (mine) {
-                const uint32_t f = (uint32_t)__ffs((int)mine) - 1u;
-                len = 2u + 2u * (t + f) + ((at_a >> (first + f)) & 1u ? 0u : 1u);
-                open = false;
-            }
-            t += g;
-        }
-        m = __ballot_sync(full, open);
-    }
-    return len;
-}
-#endif
-
 LT_HD uint32_t start_vertex(int start, uint32_t source, uint32_t V, uint64_t seed, uint32_t run, uint64_t idx)
 {
     if (start == kStartSource) return source;

@@ -17,11 +17,13 @@
 //    the read-only path; counters are u64 reductions resolved in L2.  Column
 //    loads are evict-first, row offsets and counters evict-last (mem.cuh).
 #include <algorithm>
+#include <atomic>
 #include <type_traits>
 
 #include "common.h"
 #include "lt_core.cuh"
 #include "mem.cuh"
+#include "ppr_pool.cuh"
 #include "walk_whole.h"
 
 namespace lt {
@@ -29,11 +31,12 @@ namespace lt {
 namespace {
 
 constexpr unsigned kFull = 0xFFFFFFFFu;
-// idle lanes a warp waits for before refilling them (all lanes: always): the
-// refill sits on the warp's critical path and PPR's geometric walk lengths
-// would otherwise trigger one nearly every iteration (2|V| PPR walks on
-// RMAT 2^20 / 2^24, whole call: 24 242 us, 16 234, 12 238, 8 253)
+// idle lanes a warp waits for before it asks for more walkers (PPR: for
+// another pool, whose lengths it then draws)
 constexpr int kRefillMin = 16;
+// PPR: idle lanes before a warp takes walkers out of its pool (2|V| walks on
+// RMAT 2^20 / 2^24, whole call: 1 224 us, 4 223, 8 219, 12 222)
+constexpr int kTakeMin = 8;
 
 struct Hints {
     uint64_t keep, stream;
@@ -83,6 +86,31 @@ __device__ __forceinline__ void count1(const WholeArgs &a, uint32_t v, const Hin
         red_add1_u64((unsigned long long *)(a.counts + v), h.keep);
 }
 
+template <int START>
+__device__ __forceinline__ uint32_t first_vertex(const WholeArgs &a, uint64_t idx)
+{
+    if (START == kStartSource) return a.source;
+    if (START == kStartPerVertex) return mod_by(a.by_v, idx);
+    return mod_by(a.by_v, r64_of(walk_draw(a.keys, 0, kTagInit, a.run, idx)));
+}
+
+// Makes the draw here: the compiler would move it behind the branch on the
+// row's degree, where it would wait for the row's loads first.
+template <int APP>
+__device__ __forceinline__ void settle(Rand4 &r)
+{
+    asm volatile("" : "+r"(r.x0), "+r"(r.x1));
+    if (APP == kPageRank) asm volatile("" : "+r"(r.x2), "+r"(r.x3));
+}
+
+// n more walkers for the calling warp: the first one's index past the dealt ones
+__device__ __forceinline__ uint64_t take(uint64_t *next, uint32_t n)
+{
+    unsigned long long got = 0;
+    if ((threadIdx.x & 31) == 0) got = atomicAdd((unsigned long long *)next, (unsigned long long)n);
+    return __shfl_sync(kFull, got, 0);
+}
+
 template <int APP, int START, int C>
 __global__ void __launch_bounds__(kWholeBlock, 8) walk_whole_kernel(const __grid_constant__ WholeArgs a)
 {
@@ -94,51 +122,60 @@ __global__ void __launch_bounds__(kWholeBlock, 8) walk_whole_kernel(const __grid
     bool active = false;
     // walkers no longer to be had: the counter has passed W
     bool exhausted = false;
-    // the first walkers are dealt out without the counter, 32 to each warp,
-    // the warps of the same number in their CTAs before the next ones, so
-    // that few walkers spread over all SMs
-    const uint64_t dealt = (uint64_t)gridDim.x * kWholeBlock;
+    // the first walkers are dealt out without the counter, 32 (PPR: a pool) to
+    // each warp, the warps of the same number in their CTAs before the next
+    // ones, so that few walkers spread over all SMs
+    const uint64_t dealt = (uint64_t)gridDim.x * (APP == kPPR ? kWholeBlock / 32 * a.pool : kWholeBlock);
     bool first_deal = true;
+    // PPR: the warp's pool of walkers with their lengths drawn
+    __shared__ PprPool pools[APP == kPPR ? kWholeBlock / 32 : 1];
+    PprPool &pool = pools[APP == kPPR ? threadIdx.x >> 5 : 0];
+    uint32_t pool_at = 0, pool_n = 0;
+    uint64_t pool_base = 0;
     uint32_t n_mov = 0, n_end = 0;  // hops taken; walks that ended at a vertex without out-edges
     Rand4 r{};                      // PageRank: the draw of the walker's next step
 
     while (true) {
         const unsigned busy = __ballot_sync(kFull, active);
-        if (__popc(busy) <= 32 - kRefillMin && !exhausted) {
-            const unsigned idle = ~busy;
-            uint64_t base;
-            if (first_deal) {
-                base = 32ull * ((uint64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x);
-                exhausted = dealt >= a.W;
+        const int idle = 32 - __popc(busy);
+        const uint32_t rank = __popc(~busy & ((1u << lane) - 1u));  // of an idle lane among them
+        if (APP == kPPR) {
+            if (pool_at == pool_n && idle >= kRefillMin && !exhausted) {
+                pool_base = first_deal ? a.pool * ((uint64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x)
+                                       : dealt + take(a.next, a.pool);
                 first_deal = false;
-            } else {
-                unsigned long long got = 0;
-                if (lane == 0) got = atomicAdd((unsigned long long *)a.next, (unsigned long long)__popc(idle));
-                base = dealt + __shfl_sync(kFull, got, 0);
-                exhausted = base + __popc(idle) >= a.W;
+                exhausted = pool_base + a.pool >= a.W;
+                pool_at = 0;
+                pool_n = pool_base >= a.W ? 0u : (uint32_t)min((uint64_t)a.pool, a.W - pool_base);
+                ppr_pool_fill(pool, pool_n, a.long_len, a.lim, [&](uint32_t t, uint32_t at) {
+                    return walk_draw(a.keys, t, kTagInit, a.run, pool_base + at);
+                });
             }
-            bool fresh = false;
-            if (!active) {
-                const uint64_t my = base + __popc(idle & ((1u << lane) - 1u));
-                if (my < a.W) {
-                    fresh = active = true;
-                    idx = my;
-                    if (START == kStartSource)
-                        cur = a.source;
-                    else if (START == kStartPerVertex)
-                        cur = mod_by(a.by_v, idx);
-                    else
-                        cur = mod_by(a.by_v, r64_of(walk_draw(a.keys, 0, kTagInit, a.run, idx)));
-                    step = a.length;
-                    if (APP == kWalk && a.paths) a.paths[idx * (uint64_t)(a.length + 1)] = cur;
+            if (pool_at < pool_n && idle >= kTakeMin) {
+                if (!active && pool_at + rank < pool_n) {
+                    idx = pool_base + pool.at[pool_at + rank];
+                    step = pool.len[pool_at + rank];
+                    cur = first_vertex<START>(a, idx);
+                    active = true;
                 }
+                pool_at = min(pool_n, pool_at + (uint32_t)idle);
+            } else if (idle == 32 && exhausted) {
+                break;
             }
-            if (APP == kPPR) {
-                const uint32_t len = warp_ppr_length(fresh, a.keys, a.run, idx, a.lim);
-                if (fresh) step = len;
+        } else if (idle >= kRefillMin && !exhausted) {
+            const uint64_t base = first_deal ? 32ull * ((uint64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x)
+                                             : dealt + take(a.next, (uint32_t)idle);
+            exhausted = first_deal ? dealt >= a.W : base + idle >= a.W;
+            first_deal = false;
+            if (!active && base + rank < a.W) {
+                idx = base + rank;
+                cur = first_vertex<START>(a, idx);
+                step = a.length;
+                active = true;
+                if (APP == kWalk && a.paths) a.paths[idx * (uint64_t)(a.length + 1)] = cur;
+                if (APP == kPageRank) r = walk_draw(a.keys, step, kTagStep, a.run, idx);
             }
-            if (APP == kPageRank && fresh) r = walk_draw(a.keys, step, kTagStep, a.run, idx);
-        } else if (busy == 0u) {
+        } else if (idle == 32) {
             break;
         }
         if (!active) continue;
@@ -150,6 +187,7 @@ __global__ void __launch_bounds__(kWholeBlock, 8) walk_whole_kernel(const __grid
             // down to 1 is counted right away
             const Row<C> row = row_range<C>(a, cur, h);
             r = walk_draw(a.keys, step, kTagStep, a.run, idx);
+            settle<APP>(r);
             if (row.deg > 0) {
                 cur = pick<C>(a, row, r, h);
                 n_mov++;
@@ -170,6 +208,7 @@ __global__ void __launch_bounds__(kWholeBlock, 8) walk_whole_kernel(const __grid
                 Row<C> row{};
                 if (below(now, a.lim)) row = row_range<C>(a, cur, h);
                 r = walk_draw(a.keys, step, kTagStep, a.run, idx);
+                settle<APP>(r);
                 if (row.deg > 0) {
                     cur = pick<C>(a, row, now, h);
                     n_mov++;
@@ -181,6 +220,7 @@ __global__ void __launch_bounds__(kWholeBlock, 8) walk_whole_kernel(const __grid
             // app/genericwalk.cu:22-32
             const Row<C> row = row_range<C>(a, cur, h);
             r = walk_draw(a.keys, step, kTagStep, a.run, idx);
+            settle<APP>(r);
             uint32_t *path = a.paths ? a.paths + idx * (uint64_t)(a.length + 1) + (a.length - step) : nullptr;
             if (row.deg > 0) {
                 cur = pick<C>(a, row, r, h);
@@ -239,7 +279,9 @@ cudaError_t launch_t(const WholeArgs &a, int grid, cudaStream_t st)
     // no more CTAs than have walkers, but one per SM
     const uint64_t need = std::max<uint64_t>(a.sms, (a.W + kWholeBlock - 1) / kWholeBlock);
     if ((uint64_t)grid > need) grid = (int)need;
-    walk_whole_kernel<APP, START, C><<<grid, kWholeBlock, 0, st>>>(a);
+    WholeArgs b = a;
+    b.pool = pool_walkers(a.W, (uint64_t)grid * (kWholeBlock / 32));
+    walk_whole_kernel<APP, START, C><<<grid, kWholeBlock, 0, st>>>(b);
     return cudaGetLastError();
 }
 
@@ -279,16 +321,36 @@ int occupancy_c(int app, int start)
 
 }  // namespace
 
+// SMs of the device and resident CTAs per SM of a kernel instance: properties
+// of the device and the code, asked for once (the occupancy query costs a
+// small call some 5 us).
+namespace {
+constexpr int kMaxDevices = 64;
+std::atomic<int> g_sms[kMaxDevices], g_occ[kMaxDevices][3][9];
+}  // namespace
+
+int whole_sms(int device)
+{
+    int n = device < kMaxDevices ? g_sms[device].load(std::memory_order_relaxed) : 0;
+    if (n == 0) {
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device);
+        if (device < kMaxDevices) g_sms[device].store(n, std::memory_order_relaxed);
+    }
+    return n;
+}
+
 int whole_grid(int app, int start, int device, int ctas_per_sm, int layout)
 {
-    int sms = 0;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    int occ = layout == kLayoutPacked    ? occupancy_c<kLayoutPacked>(app, start)
+    int occ = device < kMaxDevices ? g_occ[device][layout][app * 3 + start].load(std::memory_order_relaxed) : 0;
+    if (occ == 0) {
+        occ = layout == kLayoutPacked    ? occupancy_c<kLayoutPacked>(app, start)
               : layout == kLayoutCompact ? occupancy_c<kLayoutCompact>(app, start)
                                          : occupancy_c<kLayoutWide>(app, start);
-    if (occ < 1) occ = 1;
+        if (occ < 1) occ = 1;
+        if (device < kMaxDevices) g_occ[device][layout][app * 3 + start].store(occ, std::memory_order_relaxed);
+    }
     if (ctas_per_sm > 0 && ctas_per_sm < occ) occ = ctas_per_sm;
-    return sms * occ;
+    return whole_sms(device) * occ;
 }
 
 template <int C>

@@ -33,14 +33,17 @@ struct WholeArgs {
     // of v (u32), rows[2v+1] = v's counter (u32).  The row offsets an update
     // reads and the counter it increments share one 32-byte sector.
     uint32_t *rows;
-    int sms;                 // SMs of the device
+    int sms;                 // SMs of the device (set by the launcher)
     RoundKeys keys;          // of the seed
     Limit53 lim;             // of floor(p 2^53): PPR stop prob or PageRank alpha
     ModN by_v;               // remainders by V
+    uint32_t pool;           // PPR: walkers a warp draws lengths for at a time (set by the launcher)
+    uint32_t long_len;       // PPR: walks longer than this begin first in their pool
 };
 
 enum Layout : int { kLayoutWide = 0, kLayoutCompact = 1, kLayoutPacked = 2 };
 
+int whole_sms(int device);
 // Persistent grid size: SMs x resident CTAs (capped by ctas_per_sm when > 0).
 int whole_grid(int app, int start, int device, int ctas_per_sm, int layout = kLayoutWide);
 cudaError_t launch_walk_whole(const WholeArgs &a, int app, int start, int grid, cudaStream_t st,
