@@ -69,17 +69,18 @@ __device__ __forceinline__ uint32_t ld_nc_stream64_u32(const void *a, uint64_t p
     return v;
 }
 
-// counts[i] += 1 without a return value, with an L2 policy.
-__device__ __forceinline__ void red_add1_u64(unsigned long long *a, uint64_t pol)
+// counts[i] += n without a return value, with an L2 policy.
+__device__ __forceinline__ void red_add_u32(unsigned int *a, uint32_t n, uint64_t pol)
 {
-    asm volatile("red.global.add.L2::cache_hint.u64 [%0], 1, %1;" ::"l"(a), "l"(pol) : "memory");
+    asm volatile("red.global.add.L2::cache_hint.u32 [%0], %1, %2;" ::"l"(a), "r"(n), "l"(pol) : "memory");
+}
+__device__ __forceinline__ void red_add_u64(unsigned long long *a, uint64_t n, uint64_t pol)
+{
+    asm volatile("red.global.add.L2::cache_hint.u64 [%0], %1, %2;" ::"l"(a), "l"(n), "l"(pol) : "memory");
 }
 
-// counts[i] += 1 on a u32 counter, with an L2 policy.
-__device__ __forceinline__ void red_add1_u32(unsigned int *a, uint64_t pol)
-{
-    asm volatile("red.global.add.L2::cache_hint.u32 [%0], 1, %1;" ::"l"(a), "l"(pol) : "memory");
-}
+__device__ __forceinline__ void red_add1_u64(unsigned long long *a, uint64_t pol) { red_add_u64(a, 1, pol); }
+__device__ __forceinline__ void red_add1_u32(unsigned int *a, uint64_t pol) { red_add_u32(a, 1, pol); }
 
 // ---- bulk copies global -> shared (the TMA unit's untiled mode) and the
 // mbarriers that count their bytes.  Both addresses and the size must be

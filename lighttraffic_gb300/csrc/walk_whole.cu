@@ -76,14 +76,41 @@ __device__ __forceinline__ uint32_t pick(const WholeArgs &a, const Row<L> &row, 
 }
 
 template <int L>
-__device__ __forceinline__ void count1(const WholeArgs &a, uint32_t v, const Hints &h)
+__device__ __forceinline__ void count_n(const WholeArgs &a, uint32_t v, uint32_t n, const Hints &h)
 {
     if (L == kLayoutPacked)
-        red_add1_u32(a.rows + 2ull * v + 1, h.keep);
+        red_add_u32(a.rows + 2ull * v + 1, n, h.keep);
     else if (L == kLayoutCompact)
-        red_add1_u32(a.counts32 + v, h.keep);
+        red_add_u32(a.counts32 + v, n, h.keep);
     else
-        red_add1_u64((unsigned long long *)(a.counts + v), h.keep);
+        red_add_u64((unsigned long long *)(a.counts + v), n, h.keep);
+}
+template <int L>
+__device__ __forceinline__ void count1(const WholeArgs &a, uint32_t v, const Hints &h)
+{
+    count_n<L>(a, v, 1, h);
+}
+
+// Hub counters of PageRank.  Counter updates crowd the few lines that hold the
+// hubs' counters (RMAT 2^23 / 2^27: 1 % of 92 M updates go to one line), and
+// the L2 slice of such a line, at 105 % of its tag rate against 64 % on
+// average, set the kernel's time.  A CTA therefore counts up to 512 vertices
+// of at least E / 2^13 out-edges in shared memory and adds them up once at its
+// end; a vertex takes its slot at its first visit whose row is read (the first
+// to come keeps it: a hub is likely to be that).  PageRank on RMAT 2^23 / 2^27:
+// 1759 -> 1557 us, u64 on RMAT 2^21 / 4e7: 228 -> 201; 1024 slots from E / 2^14
+// 1561, 128 slots from E / 2^12 1559; serving the hubs' rows from shared
+// memory as well gave nothing.
+constexpr int kHotBits = 9;
+constexpr uint32_t kHotSlots = 1u << kHotBits;
+constexpr uint32_t kHotMinDegree = 64;
+constexpr uint32_t kNoVertex = 0xFFFFFFFFu;
+
+template <int L>
+__device__ __forceinline__ uint32_t hot_degree(const WholeArgs &a)
+{
+    const uint64_t E = L == kLayoutPacked ? a.rows[2ull * a.V] : L == kLayoutCompact ? a.rowptr32[a.V] : a.rowptr[a.V];
+    return (uint32_t)min(0xFFFFFFFFull, max((unsigned long long)kHotMinDegree, (unsigned long long)E >> 13));
 }
 
 template <int START>
@@ -132,6 +159,17 @@ __global__ void __launch_bounds__(kWholeBlock, 8) walk_whole_kernel(const __grid
     PprPool &pool = pools[APP == kPPR ? threadIdx.x >> 5 : 0];
     uint32_t pool_at = 0, pool_n = 0;
     uint64_t pool_base = 0;
+    constexpr bool kHot = APP == kPageRank;
+    __shared__ uint32_t hot_v[kHot ? kHotSlots : 1], hot_n[kHot ? kHotSlots : 1];
+    uint32_t hot_min = 0;
+    if (kHot) {
+        for (uint32_t i = threadIdx.x; i < kHotSlots; i += kWholeBlock) {
+            hot_v[i] = kNoVertex;
+            hot_n[i] = 0;
+        }
+        hot_min = hot_degree<C>(a);
+        __syncthreads();
+    }
     uint32_t n_mov = 0, n_end = 0;  // hops taken; walks that ended at a vertex without out-edges
     Rand4 r{};                      // PageRank: the draw of the walker's next step
 
@@ -199,7 +237,12 @@ __global__ void __launch_bounds__(kWholeBlock, 8) walk_whole_kernel(const __grid
             if (!active) count1<C>(a, cur, h);
         } else if (APP == kPageRank) {
             // app/pagerank.cu:26-44; a vertex without out-edges teleports.
-            count1<C>(a, cur, h);
+            const uint32_t slot = (cur * 0x9E3779B1u) >> (32 - kHotBits);
+            const uint32_t held = *(volatile uint32_t *)&hot_v[slot];
+            if (held == cur)
+                atomicAdd(&hot_n[slot], 1u);
+            else
+                count1<C>(a, cur, h);
             step--;
             if (step == 0) {
                 active = false;
@@ -209,6 +252,7 @@ __global__ void __launch_bounds__(kWholeBlock, 8) walk_whole_kernel(const __grid
                 if (below(now, a.lim)) row = row_range<C>(a, cur, h);
                 r = walk_draw(a.keys, step, kTagStep, a.run, idx);
                 settle<APP>(r);
+                if (held == kNoVertex && row.deg >= hot_min) atomicCAS(&hot_v[slot], kNoVertex, cur);
                 if (row.deg > 0) {
                     cur = pick<C>(a, row, now, h);
                     n_mov++;
@@ -243,6 +287,11 @@ __global__ void __launch_bounds__(kWholeBlock, 8) walk_whole_kernel(const __grid
     // walk makes one update per hop and one that ends it, a PageRank walk
     // a.length updates of which all but the last hop or teleport, a generic
     // walk one per hop and one where it ends early.
+    if (kHot) {
+        __syncthreads();
+        for (uint32_t i = threadIdx.x; i < kHotSlots; i += kWholeBlock)
+            if (hot_n[i]) count_n<C>(a, hot_v[i], hot_n[i], h);
+    }
     if (!a.stats) return;
     __shared__ unsigned long long s_mov, s_end;
     if (threadIdx.x == 0) s_mov = s_end = 0;

@@ -61,3 +61,37 @@ def test_walk_lengths(lt, require_gpu, graph, length, wide):
         got = paths.cpu().numpy().view(np.uint32)
         assert (got[off:off + W * (length + 1)] == want_pa.ravel()).all() and (got[off + W * (length + 1):] == 0).all()
         assert stats.tolist() == [int(x) for x in st]
+
+
+@pytest.mark.parametrize("degree", [63, 64, 80])
+@pytest.mark.parametrize("layout", ["wide", "compact", "packed"])
+def test_pagerank_shared_counters(lt, require_gpu, degree, layout):
+    """More vertices at and around the least degree counted in shared memory than it has slots."""
+    import torch
+    V, W, L = 3001, 20011, 9
+    rng = np.random.default_rng(degree)
+    rp = (np.arange(V + 1, dtype=np.uint64) * np.uint64(degree))
+    col = rng.integers(0, V, V * degree).astype(np.uint32)
+    want, st = oracle.pagerank(rp, col, W, length=L, seed=77, start_mode=1)
+    dev, p = "cuda", torch.cuda.current_stream().cuda_stream
+    d_rp = torch.from_numpy(rp.view(np.int64)).to(dev)
+    d_col = torch.from_numpy(col.view(np.int32)).to(dev)
+    scratch = torch.zeros(lt.lib.lt_walk_scratch_bytes() // 8, dtype=torch.int64, device=dev)
+    stats = torch.zeros(3, dtype=torch.int64, device=dev)
+    tail = (scratch.data_ptr(), stats.data_ptr(), p)
+    args = (V, 0, W, L, ctypes.c_float(0.85), 0, 77)
+    if layout == "packed":
+        rows = torch.empty(2 * (V + 1), dtype=torch.int32, device=dev)
+        counts = torch.zeros(V, dtype=torch.int64, device=dev)
+        lt.check(lt.lib.lt_rows_pack(d_rp.data_ptr(), rows.data_ptr(), V, p))
+        lt.check(lt.lib.lt_walk_device_packed(1, 1, rows.data_ptr(), d_col.data_ptr(), *args, None, None, *tail))
+        lt.check(lt.lib.lt_rows_counts(rows.data_ptr(), counts.data_ptr(), V, p))
+    elif layout == "compact":
+        rows = torch.from_numpy(rp.astype(np.uint32).view(np.int32)).to(dev)
+        counts = torch.zeros(V, dtype=torch.int32, device=dev)
+        lt.check(lt.lib.lt_walk_device_compact(1, 1, rows.data_ptr(), d_col.data_ptr(), *args, counts.data_ptr(), None, None, *tail))
+    else:
+        counts = torch.zeros(V, dtype=torch.int64, device=dev)
+        lt.check(lt.lib.lt_walk_device(1, 1, d_rp.data_ptr(), d_col.data_ptr(), *args, counts.data_ptr(), None, None, *tail))
+    assert (counts.cpu().numpy().astype(np.uint64) == want).all()
+    assert stats.tolist() == [int(x) for x in st]
