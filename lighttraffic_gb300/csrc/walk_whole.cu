@@ -138,7 +138,52 @@ __device__ __forceinline__ uint64_t take(uint64_t *next, uint32_t n)
     return __shfl_sync(kFull, got, 0);
 }
 
-template <int APP, int START, int C>
+// Paths of generic walks.  A lane gathers up to kPathWords vertices of its path
+// in shared memory; the warp writes the segments of its lanes that are full or
+// ended, 16 threads to a segment, so that a store instruction covers two
+// segments instead of 32 scattered words (one L2 request each).  4.7 M walks of
+// 10 hops on RMAT 2^22 / 2^26 637 -> 602 us, 1 M of 40 hops on 2^18 / 2^22 518
+// -> 448 us.  Walks of fewer than kPathGatherMin hops are too short for it
+// (5 hops: 64 -> 75 us, 9: 103 either way) and in a launch that does not fill
+// the chip its instructions cost more than the requests (20 000 walks of 10
+// hops: 30 -> 33 us; 400 000 of 20: 97 -> 101): two walkers per lane of the chip
+// at least.
+constexpr uint32_t kPathWords = 16, kPathStride = kPathWords + 1;  // an odd stride: no bank conflicts
+constexpr uint32_t kPathGatherMin = 10;
+constexpr size_t kPathSmem = 4ull * kWholeBlock * kPathStride;
+
+struct PathSegment {
+    uint32_t *buf;  // of this lane
+    uint32_t *out;  // where buf[0] goes
+    uint32_t n;     // vertices gathered
+};
+
+// Writes the segments of the lanes with `due`; the whole warp, converged.
+__device__ __forceinline__ void path_flush(PathSegment &p, bool due)
+{
+    unsigned m = __ballot_sync(kFull, due && p.n != 0u);
+    __syncwarp();
+    const uint32_t lane = threadIdx.x & 31u, w = lane & (kPathWords - 1u);
+    const uint32_t *warp_buf = p.buf - lane * kPathStride;
+    while (m) {
+        uint32_t src = (uint32_t)__ffs((int)m) - 1u;
+        m &= m - 1u;
+        const bool second = m != 0u;
+        if (lane >= 16u && second) src = (uint32_t)__ffs((int)m) - 1u;
+        if (second) m &= m - 1u;
+        const uint32_t n = __shfl_sync(kFull, p.n, src);
+        uint32_t *out = (uint32_t *)__shfl_sync(kFull, (unsigned long long)p.out, src);
+        if (w < n && (lane < 16u || second)) out[w] = warp_buf[src * kPathStride + w];
+    }
+    __syncwarp();
+    if (due) {
+        p.out += p.n;
+        p.n = 0;
+    }
+}
+
+// GATHER: paths go through shared memory (kWalk only).
+template <int APP, int START, int C, bool GATHER>
 __global__ void __launch_bounds__(kWholeBlock, 8) walk_whole_kernel(const __grid_constant__ WholeArgs a)
 {
     const int lane = threadIdx.x & 31;
@@ -159,6 +204,8 @@ __global__ void __launch_bounds__(kWholeBlock, 8) walk_whole_kernel(const __grid
     PprPool &pool = pools[APP == kPPR ? threadIdx.x >> 5 : 0];
     uint32_t pool_at = 0, pool_n = 0;
     uint64_t pool_base = 0;
+    extern __shared__ uint32_t path_buf[];  // GATHER: kPathSmem bytes
+    PathSegment path{path_buf + threadIdx.x * kPathStride, nullptr, 0};
     constexpr bool kHot = APP == kPageRank;
     __shared__ uint32_t hot_v[kHot ? kHotSlots : 1], hot_n[kHot ? kHotSlots : 1];
     uint32_t hot_min = 0;
@@ -176,6 +223,10 @@ __global__ void __launch_bounds__(kWholeBlock, 8) walk_whole_kernel(const __grid
     while (true) {
         const unsigned busy = __ballot_sync(kFull, active);
         const int idle = 32 - __popc(busy);
+        // ended walks keep their segments until a lane's is full or their lanes
+        // are refilled (or nothing is left to do)
+        if (GATHER && (__any_sync(kFull, path.n == kPathWords) || (exhausted ? idle == 32 : idle >= kRefillMin)))
+            path_flush(path, path.n == kPathWords || !active);
         const uint32_t rank = __popc(~busy & ((1u << lane) - 1u));  // of an idle lane among them
         if (APP == kPPR) {
             if (pool_at == pool_n && idle >= kRefillMin && !exhausted) {
@@ -210,7 +261,13 @@ __global__ void __launch_bounds__(kWholeBlock, 8) walk_whole_kernel(const __grid
                 cur = first_vertex<START>(a, idx);
                 step = a.length;
                 active = true;
-                if (APP == kWalk && a.paths) a.paths[idx * (uint64_t)(a.length + 1)] = cur;
+                if (GATHER) {
+                    path.out = a.paths + idx * (uint64_t)(a.length + 1);
+                    path.buf[0] = cur;
+                    path.n = 1;
+                } else if (APP == kWalk && a.paths) {
+                    a.paths[idx * (uint64_t)(a.length + 1)] = cur;
+                }
                 if (APP == kPageRank) r = walk_draw(a.keys, step, kTagStep, a.run, idx);
             }
         } else if (idle == 32) {
@@ -265,15 +322,25 @@ __global__ void __launch_bounds__(kWholeBlock, 8) walk_whole_kernel(const __grid
             const Row<C> row = row_range<C>(a, cur, h);
             r = walk_draw(a.keys, step, kTagStep, a.run, idx);
             settle<APP>(r);
-            uint32_t *path = a.paths ? a.paths + idx * (uint64_t)(a.length + 1) + (a.length - step) : nullptr;
+            uint32_t *out = !GATHER && a.paths ? a.paths + idx * (uint64_t)(a.length + 1) + (a.length - step) : nullptr;
             if (row.deg > 0) {
                 cur = pick<C>(a, row, r, h);
                 n_mov++;
-                if (path) path[1] = cur;
+                if (GATHER)
+                    path.buf[path.n++] = cur;
+                else if (out)
+                    out[1] = cur;
                 step--;
             } else {
-                if (path)
-                    for (uint32_t k = 1; k <= step; k++) path[k] = kInvalidNode;
+                // the rest of the path (gathered as far as it fits)
+                if (GATHER) {
+                    const uint32_t fits = min(step, kPathWords - path.n);
+                    for (uint32_t k = 0; k < fits; k++) path.buf[path.n + k] = kInvalidNode;
+                    path.n += fits;
+                    for (uint32_t k = fits; k < step; k++) path.out[path.n + (k - fits)] = kInvalidNode;
+                } else if (out) {
+                    for (uint32_t k = 1; k <= step; k++) out[k] = kInvalidNode;
+                }
                 n_end++;
                 step = 0;
             }
@@ -330,7 +397,13 @@ cudaError_t launch_t(const WholeArgs &a, int grid, cudaStream_t st)
     if ((uint64_t)grid > need) grid = (int)need;
     WholeArgs b = a;
     b.pool = pool_walkers(a.W, (uint64_t)grid * (kWholeBlock / 32));
-    walk_whole_kernel<APP, START, C><<<grid, kWholeBlock, 0, st>>>(b);
+    if constexpr (APP == kWalk) {
+        if (a.paths && a.length >= kPathGatherMin && a.W > 2ull * a.sms * kWholeBlock * 8) {
+            walk_whole_kernel<APP, START, C, true><<<grid, kWholeBlock, kPathSmem, st>>>(b);
+            return cudaGetLastError();
+        }
+    }
+    walk_whole_kernel<APP, START, C, false><<<grid, kWholeBlock, 0, st>>>(b);
     return cudaGetLastError();
 }
 
@@ -348,7 +421,7 @@ template <int APP, int START, int C>
 int occupancy_t()
 {
     int n = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, walk_whole_kernel<APP, START, C>, kWholeBlock, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, walk_whole_kernel<APP, START, C, false>, kWholeBlock, 0);
     return n;
 }
 

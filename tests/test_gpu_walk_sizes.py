@@ -1,6 +1,7 @@
 """The resident step kernels where their dealing of walkers and drawing of lengths can go wrong: fewer walkers than
 lanes, one warp, one more, just past the walkers dealt without the counter, stop probabilities that end nearly every
-walk at once or make one walk of a warp far longer than the others, and statistics, against the CPU oracle."""
+walk at once or make one walk of a warp far longer than the others; paths of walks shorter and longer than the segments
+they are gathered in; statistics.  Against the CPU oracle."""
 import ctypes
 
 import numpy as np
@@ -39,12 +40,12 @@ def test_pagerank_walkers(lt, require_gpu, graph, walkers, alpha, start):
     assert (s["updates"], s["moves"], s["teleports"]) == tuple(int(x) for x in st)
 
 
-@pytest.mark.parametrize("length", [1, 2, 31, 32, 33, 80])
+@pytest.mark.parametrize("walkers,length", [(5003, n) for n in (1, 2, 31, 32, 33, 80)] + [(650003, n) for n in (9, 10, 14, 15, 16, 31, 32, 33)])
 @pytest.mark.parametrize("wide", [True, False])
-def test_walk_lengths(lt, require_gpu, graph, length, wide):
+def test_walk_lengths(lt, require_gpu, graph, walkers, length, wide):
     import torch
     rp, col = graph
-    V, W = len(rp) - 1, 5003
+    V, W = len(rp) - 1, walkers
     rows = torch.from_numpy(rp.view(np.int64) if wide else rp.astype(np.uint32).view(np.int32)).cuda()
     d_col = torch.from_numpy(col.view(np.int32)).cuda()
     ep = torch.zeros(W, dtype=torch.int32, device="cuda")
