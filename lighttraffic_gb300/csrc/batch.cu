@@ -7,11 +7,12 @@
 //   prep    : one CTA; woff = scan(walkers), table capacity per query
 //             cap = next_pow2(max(walkers << load_shift, 32)), toff = scan(cap);
 //   clear   : tables to empty;
-//   walk    : persistent, warp-aggregated refill over the global walker
-//             ordinal; a walker finds its query by binary search over woff
-//             (shared memory), is created from (query seed, index) and stepped
-//             with the PPR semantics of app/ppr.cu:22-42 to its endpoint, which
-//             is added to the query's table (linear probing, u32 counts);
+//   walk    : persistent; a warp takes blocks of walker ordinals, cuts them at
+//             query boundaries (search over woff) into pools whose lengths it
+//             draws ahead (ppr_pool.cuh), and steps each walker with the PPR
+//             semantics of app/ppr.cu:22-42 to its endpoint; endpoints are
+//             gathered and added to their queries' tables (linear probing, u32
+//             counts) 32 at a time;
 //   count   : one CTA per query counts its occupied slots;
 //   offsets : exclusive scan of the counts;
 //   compact : one CTA per query writes (vertex, count) pairs in slot order.
@@ -24,6 +25,7 @@
 #include "engine.h"
 #include "lt_core.cuh"
 #include "mem.cuh"
+#include "ppr_pool.cuh"
 #include "scan.cuh"
 
 namespace lt {
@@ -32,13 +34,10 @@ namespace {
 
 constexpr unsigned kFull = 0xFFFFFFFFu;
 constexpr uint32_t kEmpty = 0xFFFFFFFFu;
-// A warp refills its idle lanes only once at least this many are idle (or
-// all of them): a refill (query lookup, walk-length draws) runs on the
-// warp's critical path, and PPR's geometric lengths would otherwise make
-// nearly every iteration a refill.  24 of 32 measured best on c3
-// (70.5 -> 25.0 ms per batch; 16: 31.3, 32: 29.5).
-constexpr int kRefillMin = 24;
-constexpr uint32_t kSmemQueries = 8192;  // up to this many u32 walker offsets go to shared memory
+// idle lanes before a warp draws another pool, and before it takes walkers
+// out of its pool
+constexpr int kRefillMin = 16;
+constexpr int kTakeMin = 8;
 constexpr int kPrepThreads = 1024;
 constexpr int kRowThreads = 256;
 
@@ -51,14 +50,22 @@ struct Header {
     unsigned long long stats[3]; // updates, moves, -
 };
 
+// Written by the host before each launch: the queries of the batch and where
+// its results go (device memory, or the caller's page-locked host memory).
+struct BatchIn {
+    uint64_t n;
+    uint64_t *qout;  // n+1: output offsets
+    uint32_t *out_v, *out_c;
+};
+
 struct BatchArgs {
-    const uint32_t *n_dev;   // queries in the batch (written by the host before each launch)
-    uint32_t smem_queries;   // walker offsets kept in shared memory when n <= smem_queries
+    const BatchIn *in;
     const uint64_t *rowptr;
     const uint32_t *rowptr32;  // compact row offsets when E < 2^32 (else null)
     const uint32_t *col;
     uint32_t V;
-    uint64_t thr;
+    Limit53 lim;           // stop probability
+    uint32_t long_len;     // walks longer than this begin first in their pool
     Header *hdr;
     const uint32_t *src;
     const uint64_t *walkers;
@@ -71,9 +78,6 @@ struct BatchArgs {
     uint32_t *ccount;    // occupied slots per compaction chunk (nch)
     uint64_t *cbase;     // nch+1: exclusive scan of ccount
     uint64_t nch;        // compaction chunks of the table arena
-    uint64_t *qout;      // n+1: output offsets
-    uint32_t *out_v;
-    uint32_t *out_c;
     int load_shift;
 };
 
@@ -85,7 +89,7 @@ __device__ __forceinline__ uint32_t log2_ceil(uint64_t x)
 // Exclusive scans of walkers and table capacities, one CTA.
 __global__ void __launch_bounds__(kPrepThreads) prep_kernel(BatchArgs a)
 {
-    const uint32_t n = *a.n_dev;
+    const uint32_t n = (uint32_t)a.in->n;
     __shared__ unsigned long long warp_w[kPrepThreads / 32], warp_t[kPrepThreads / 32];
     __shared__ unsigned long long carry_w, carry_t;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -184,104 +188,127 @@ __device__ __forceinline__ void table_add(const BatchArgs &a, uint32_t q, uint32
     atomicAdd(&a.hdr->error, 1ull);
 }
 
-__device__ __forceinline__ uint32_t find_query(const uint32_t *s_off, const uint64_t *g_off, bool in_smem, uint32_t n,
-                                               uint64_t g)
-{
-    uint32_t lo = 0, hi = n - 1;
-    while (lo < hi) {
-        const uint32_t mid = lo + (hi - lo + 1) / 2;
-        const uint64_t o = in_smem ? (uint64_t)s_off[mid] : g_off[mid];
-        if (g < o)
-            hi = mid - 1;
-        else
-            lo = mid;
-    }
-    return lo;
-}
+// Endpoints wait here until a warp has 32 of them: added one by one as the
+// walks end, a few lanes' table probes (a load and two atomics in a row) would
+// hold up the hops of the others in nearly every iteration.
+// Threads per SM the registers are sized for: 48 registers without spills.
+// 256 queries of 7.3 M walks on RMAT 2^22 / 2^26: 2048 (32 registers, spilled) 2.6 ms per batch, 1536 1.52, 1280 1.47,
+// 1024 1.53.
+constexpr int kThreadsPerSm = 1280;
+
+struct BatchWarp {
+    PprPool pool;
+    uint2 ends[64];  // (query, vertex)
+};
 
 template <int BLOCK>
-__global__ void __launch_bounds__(BLOCK) batch_walk_kernel(BatchArgs a)
+__global__ void __launch_bounds__(BLOCK, kThreadsPerSm / BLOCK) batch_walk_kernel(BatchArgs a)
 {
-    extern __shared__ uint32_t s_off[];
-    const uint32_t n = (uint32_t)a.hdr->n;
-    const uint64_t W = a.hdr->W;
-    const bool in_smem = n <= a.smem_queries && W < (1ull << 32);
-    if (in_smem)
-        for (uint32_t i = threadIdx.x; i < n; i += BLOCK) s_off[i] = (uint32_t)a.woff[i];
+    __shared__ BatchWarp s_warp[BLOCK / 32];
+    __shared__ unsigned long long s_mov;
+    const uint64_t n = a.hdr->n, W = a.hdr->W;
+    if (threadIdx.x == 0) s_mov = 0;
     __syncthreads();
     if (n == 0) return;
 
     const int lane = threadIdx.x & 31;
-    const unsigned lt_mask = (1u << lane) - 1u;
+    const unsigned below_me = (1u << lane) - 1u;
     const uint64_t keep = l2_policy_evict_last(), stream = l2_policy_evict_first();
-    uint32_t cur = 0, step = 0, q = 0;
+    BatchWarp &sw = s_warp[threadIdx.x >> 5];
+    const uint64_t warps = (uint64_t)gridDim.x * (BLOCK / 32);
+    const uint32_t block = pool_walkers(W, warps);
+    // the warp's block of ordinals: the first one without the counter
+    uint64_t at = block * ((uint64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x), end = min(W, at + block);
+    bool exhausted = at >= W;
+    // its pool: walkers of one query
+    uint32_t pool_at = 0, pool_n = 0, pool_q = 0;
+    uint64_t pool_idx = 0;
+    uint32_t cur = 0, step = 0, q = 0, n_ends = 0, n_mov = 0;
     uint64_t idx = 0, seed = 0;
-    bool active = false, exhausted = false;
-    unsigned long long n_upd = 0, n_mov = 0;
+    bool active = false, ended = false;
 
     while (true) {
-        const unsigned idle = __ballot_sync(kFull, !active);
-        if (idle != 0u && !exhausted && (__popc(idle) >= kRefillMin || idle == kFull)) {
-            const int leader = __ffs(idle) - 1;
-            unsigned long long base = 0;
-            if (lane == leader) base = atomicAdd(&a.hdr->next, (unsigned long long)__popc(idle));
-            base = __shfl_sync(kFull, base, leader);
-            if (base + __popc(idle) >= W) exhausted = true;
-            if (!active) {
-                const uint64_t g = base + __popc(idle & lt_mask);
-                if (g < W) {
-                    q = find_query(s_off, a.woff, in_smem, n, g);
-                    idx = g - a.woff[q];
-                    seed = a.seeds[q];
-                    cur = a.src[q];
-                    step = ppr_length(seed, 0, idx, a.thr);
-                    active = true;
-                }
+        const unsigned over = __ballot_sync(kFull, ended);
+        if (over) {
+            if (ended) sw.ends[n_ends + __popc(over & below_me)] = make_uint2(q, cur);
+            ended = false;
+            n_ends += __popc(over);
+            __syncwarp();
+            if (n_ends >= 32u) {
+                n_ends -= 32u;
+                const uint2 e = sw.ends[n_ends + lane];
+                table_add(a, e.x, e.y);
+                __syncwarp();
             }
         }
-        if (__ballot_sync(kFull, active) == 0u) {
-            if (exhausted) break;
-            continue;
+        const unsigned busy = __ballot_sync(kFull, active);
+        const int idle = 32 - __popc(busy);
+        if (pool_at == pool_n && idle >= kRefillMin && !exhausted) {
+            pool_q = (uint32_t)warp_find_last(a.woff, pool_q, n, at);
+            const uint64_t q_begin = a.woff[pool_q], q_end = a.woff[pool_q + 1], q_seed = a.seeds[pool_q];
+            pool_at = 0;
+            pool_n = (uint32_t)(min(end, q_end) - at);
+            pool_idx = at - q_begin;
+            ppr_pool_fill(sw.pool, pool_n, a.long_len, a.lim, [&](uint32_t t, uint32_t w) {
+                return walk_draw(q_seed, t, kTagInit, 0, pool_idx + w);
+            });
+            at += pool_n;
+            if (at == end) {
+                unsigned long long got = 0;
+                if (lane == 0) got = atomicAdd(&a.hdr->next, (unsigned long long)block);
+                at = block * warps + __shfl_sync(kFull, got, 0);
+                end = min(W, at + block);
+                exhausted = at >= W;
+            }
+        }
+        if (pool_at < pool_n && idle >= kTakeMin) {
+            const uint32_t mine = pool_at + __popc(~busy & below_me);
+            if (!active && mine < pool_n) {
+                idx = pool_idx + sw.pool.at[mine];
+                step = sw.pool.len[mine];
+                q = pool_q;
+                seed = a.seeds[q];
+                cur = a.src[q];
+                active = true;
+            }
+            pool_at = min(pool_n, pool_at + (uint32_t)idle);
+        } else if (idle == 32 && exhausted) {
+            break;
         }
         if (!active) continue;
-        // app/ppr.cu:22-42
-        const uint32_t s = step;
-        n_upd++;
-        bool done = false;
-        if (s == 1) {
-            done = true;
+        // app/ppr.cu:22-42; step >= 2 here, the draw made under the row's loads
+        uint64_t first, deg;
+        if (a.rowptr32) {
+            const uint32_t f = ld_nc_u32(a.rowptr32 + cur, keep);
+            first = f;
+            deg = ld_nc_u32(a.rowptr32 + cur + 1, keep) - f;
         } else {
-            step = s - 1;
-            uint64_t first, deg;
-            if (a.rowptr32) {
-                const uint32_t f = ld_nc_u32(a.rowptr32 + cur, keep);
-                first = f;
-                deg = ld_nc_u32(a.rowptr32 + cur + 1, keep) - f;
-            } else {
-                first = ld_nc_u64(a.rowptr + cur, keep);
-                deg = ld_nc_u64(a.rowptr + cur + 1, keep) - first;
-            }
-            if (deg > 0) {
-                const Rand4 r = walk_draw(seed, s, kTagStep, 0, idx);
-                cur = ld_nc_stream_u32(a.col + first + mod_u64(r64_of(r), deg), stream);
-                n_mov++;
-            } else {
-                done = true;
-            }
+            first = ld_nc_u64(a.rowptr + cur, keep);
+            deg = ld_nc_u64(a.rowptr + cur + 1, keep) - first;
         }
-        if (done) {
-            table_add(a, q, cur);
-            active = false;
+        Rand4 r = walk_draw(seed, step, kTagStep, 0, idx);
+        asm volatile("" : "+r"(r.x0), "+r"(r.x1));  // here, not behind the branch
+        if (deg > 0) {
+            cur = ld_nc_stream64_u32(a.col + first + mod_u64(r64_of(r), deg), stream);
+            n_mov++;
+            step--;
+        } else {
+            step = 1;
         }
+        ended = step == 1;
+        active = !ended;
     }
+    if ((uint32_t)lane < n_ends) table_add(a, sw.ends[lane].x, sw.ends[lane].y);
+    uint64_t w_mov = n_mov;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        n_upd += __shfl_down_sync(kFull, n_upd, o);
-        n_mov += __shfl_down_sync(kFull, n_mov, o);
-    }
-    if (lane == 0) {
-        atomicAdd(&a.hdr->stats[0], n_upd);
-        atomicAdd(&a.hdr->stats[1], n_mov);
+    for (int o = 16; o > 0; o >>= 1) w_mov += __shfl_down_sync(kFull, w_mov, o);
+    if (lane == 0 && w_mov) atomicAdd(&s_mov, (unsigned long long)w_mov);
+    __syncthreads();
+    // one update per hop and one that ends each walk
+    if (threadIdx.x == 0) {
+        const unsigned long long ends = blockIdx.x == 0 ? W : 0;
+        if (s_mov + ends) atomicAdd(&a.hdr->stats[0], s_mov + ends);
+        if (s_mov) atomicAdd(&a.hdr->stats[1], s_mov);
     }
 }
 
@@ -303,51 +330,65 @@ __device__ unsigned block_count(unsigned v, unsigned *sh)
 // plus the occupied slots between that chunk's start and the table.
 constexpr uint64_t kCompactChunk = 4096;
 
+constexpr uint32_t kChunkPer = kCompactChunk / kRowThreads;  // slots per thread (tables are whole multiples of 32)
+
+// The occupied ones of a thread's kChunkPer consecutive slots, as bits.
+__device__ __forceinline__ uint32_t occupied_slots(const uint32_t *keys, uint32_t (&key)[kChunkPer])
+{
+    uint32_t m = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < kChunkPer; k += 4) {
+        const uint4 q = *reinterpret_cast<const uint4 *>(keys + k);
+        key[k] = q.x, key[k + 1] = q.y, key[k + 2] = q.z, key[k + 3] = q.w;
+    }
+#pragma unroll
+    for (uint32_t k = 0; k < kChunkPer; k++) m |= key[k] != kEmpty ? 1u << k : 0u;
+    return m;
+}
+
 __global__ void __launch_bounds__(kRowThreads) chunk_count_kernel(BatchArgs a)
 {
     __shared__ unsigned sh[kRowThreads / 32];
-    const uint64_t T = a.toff[(uint32_t)a.hdr->n];
+    const uint64_t T = a.hdr->T;
     for (uint64_t c = blockIdx.x; c < a.nch; c += gridDim.x) {
-        const uint64_t b = c * kCompactChunk, e = b + kCompactChunk < T ? b + kCompactChunk : T;
-        unsigned cnt = 0;
-        for (uint64_t i = b + threadIdx.x; i < e; i += kRowThreads) cnt += a.keys[i] != kEmpty;
-        const unsigned t = block_count(cnt, sh);
+        const uint64_t i = c * kCompactChunk + threadIdx.x * kChunkPer;
+        uint32_t key[kChunkPer];
+        const unsigned t = block_count(i < T ? __popc(occupied_slots(a.keys + i, key)) : 0, sh);
         if (threadIdx.x == 0) a.ccount[c] = t;
         __syncthreads();
     }
 }
 
+// A chunk's pairs are gathered in shared memory and written as one run: 22 M
+// slots in 5 400 chunks 79 -> 42 us.
 __global__ void __launch_bounds__(kRowThreads) chunk_compact_kernel(BatchArgs a)
 {
-    __shared__ unsigned sh[kRowThreads / 32];
-    const uint64_t T = a.toff[(uint32_t)a.hdr->n];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    __shared__ uint32_t warp_tot[kRowThreads / 32], total;
+    __shared__ uint32_t s_v[kCompactChunk], s_c[kCompactChunk];
+    const uint64_t T = a.hdr->T;
+    uint32_t *out_v = a.in->out_v, *out_c = a.in->out_c;
     for (uint64_t c = blockIdx.x; c < a.nch && c * kCompactChunk < T; c += gridDim.x) {
-        const uint64_t b = c * kCompactChunk, e = b + kCompactChunk < T ? b + kCompactChunk : T;
-        uint64_t base = a.cbase[c];
-        for (uint64_t t0 = b; t0 < e; t0 += kRowThreads) {
-            const uint64_t i = t0 + threadIdx.x;
-            const bool occ = i < e && a.keys[i] != kEmpty;
-            const unsigned m = __ballot_sync(kFull, occ);
-            if (lane == 0) sh[wid] = __popc(m);
-            __syncthreads();
-            unsigned before = 0, total = 0;
-            for (int w = 0; w < kRowThreads / 32; w++) {
-                if (w < wid) before += sh[w];
-                total += sh[w];
+        const uint64_t i = c * kCompactChunk + threadIdx.x * kChunkPer;
+        uint32_t key[kChunkPer];
+        const uint32_t m = i < T ? occupied_slots(a.keys + i, key) : 0u;
+        uint32_t pos = scan_detail::block_exclusive<uint32_t, kRowThreads>(__popc(m), warp_tot, &total);
+#pragma unroll
+        for (uint32_t k = 0; k < kChunkPer; k++)
+            if ((m >> k) & 1u) {
+                s_v[pos] = key[k];
+                s_c[pos++] = a.cnt[i + k];
             }
-            if (occ) {
-                const uint64_t pos = base + before + __popc(m & ((1u << lane) - 1u));
-                a.out_v[pos] = a.keys[i];
-                a.out_c[pos] = a.cnt[i];
-            }
-            base += total;
-            __syncthreads();
+        __syncthreads();
+        const uint64_t base = a.cbase[c];
+        for (uint32_t k = threadIdx.x; k < total; k += kRowThreads) {
+            out_v[base + k] = s_v[k];
+            out_c[base + k] = s_c[k];
         }
+        __syncthreads();
     }
 }
 
-// One warp per query q (and q = n): qout[q] = occupied slots before toff[q].
+// One warp per query q (and q = n): in->qout[q] = occupied slots before toff[q].
 __global__ void query_offsets_kernel(BatchArgs a)
 {
     const uint32_t n = (uint32_t)a.hdr->n;
@@ -359,15 +400,15 @@ __global__ void query_offsets_kernel(BatchArgs a)
         unsigned cnt = 0;
         for (uint64_t i = c * kCompactChunk + lane; i < s; i += 32) cnt += a.keys[i] != kEmpty;
         for (int o = 16; o > 0; o >>= 1) cnt += __shfl_down_sync(kFull, cnt, o);
-        if (lane == 0) a.qout[q] = a.cbase[c] + cnt;
+        if (lane == 0) a.in->qout[q] = a.cbase[c] + cnt;
     }
 }
 
 template <int BLOCK>
-int walk_occupancy(size_t smem)
+int walk_occupancy()
 {
     int occ = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, batch_walk_kernel<BLOCK>, BLOCK, smem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, batch_walk_kernel<BLOCK>, BLOCK, 0);
     return occ < 1 ? 1 : occ;
 }
 
@@ -379,7 +420,7 @@ struct BatchState {
     uint64_t wcap = 0, tcap = 0;
     Header *d_hdr = nullptr;
     uint32_t *d_src = nullptr, *d_tlog = nullptr, *d_keys = nullptr, *d_cnt = nullptr, *d_ccount = nullptr;
-    uint32_t *d_n = nullptr;
+    BatchIn *d_in = nullptr;
     uint64_t *d_walkers = nullptr, *d_seeds = nullptr, *d_woff = nullptr, *d_toff = nullptr, *d_qout = nullptr;
     uint64_t *d_scan_tmp = nullptr, *d_cbase = nullptr;
     uint64_t nch = 0;  // compaction chunks of the table arena
@@ -390,19 +431,19 @@ struct BatchState {
     uint64_t graph_thr = 0;
     BatchTune graph_tune;
     Header h_hdr{};
-    uint32_t h_n = 0;
+    BatchIn h_in{};
 };
 
 namespace {
 
 void free_buffers(BatchState &b)
 {
-    for (void *p : {(void *)b.d_hdr, (void *)b.d_n, (void *)b.d_src, (void *)b.d_tlog, (void *)b.d_keys, (void *)b.d_cnt,
+    for (void *p : {(void *)b.d_hdr, (void *)b.d_in, (void *)b.d_src, (void *)b.d_tlog, (void *)b.d_keys, (void *)b.d_cnt,
                     (void *)b.d_ccount, (void *)b.d_walkers, (void *)b.d_seeds, (void *)b.d_woff, (void *)b.d_toff,
                     (void *)b.d_qout, (void *)b.d_scan_tmp, (void *)b.d_cbase, (void *)b.d_out_v, (void *)b.d_out_c})
         if (p) cudaFree(p);
     b.d_hdr = nullptr;
-    b.d_n = nullptr;
+    b.d_in = nullptr;
     b.d_src = b.d_tlog = b.d_keys = b.d_cnt = b.d_ccount = b.d_out_v = b.d_out_c = nullptr;
     b.d_walkers = b.d_seeds = b.d_woff = b.d_toff = b.d_qout = b.d_scan_tmp = b.d_cbase = nullptr;
     if (b.exec) cudaGraphExecDestroy(b.exec);
@@ -443,7 +484,7 @@ lt_status ensure(BatchState &b, uint32_t n, uint64_t W, uint64_t T)
     b.wcap = wcap;
     b.tcap = tcap;
     LT_TRY(dalloc(&b.d_hdr, 1));
-    LT_TRY(dalloc(&b.d_n, 1));
+    LT_TRY(dalloc(&b.d_in, 1));
     LT_TRY(dalloc(&b.d_src, qcap));
     LT_TRY(dalloc(&b.d_tlog, qcap));
     b.nch = tcap / kCompactChunk + 1;
@@ -465,13 +506,13 @@ lt_status ensure(BatchState &b, uint32_t n, uint64_t W, uint64_t T)
 BatchArgs args_of(lt_engine *e, BatchState &b, uint64_t thr)
 {
     BatchArgs a{};
-    a.n_dev = b.d_n;
-    a.smem_queries = std::min<uint32_t>(b.qcap, kSmemQueries);
+    a.in = b.d_in;
     a.rowptr = e->d_rowptr;
     a.rowptr32 = e->d_rowptr32;
     a.col = e->d_col;
     a.V = e->g->V;
-    a.thr = thr;
+    a.lim = limit53(thr);
+    a.long_len = thr ? (uint32_t)std::min(1e9, 2.0 * 9007199254740992.0 / (double)thr) + 1u : 0xFFFFFFFFu;
     a.hdr = b.d_hdr;
     a.src = b.d_src;
     a.walkers = b.d_walkers;
@@ -484,34 +525,30 @@ BatchArgs args_of(lt_engine *e, BatchState &b, uint64_t thr)
     a.ccount = b.d_ccount;
     a.cbase = b.d_cbase;
     a.nch = b.nch;
-    a.qout = b.d_qout;
-    a.out_v = b.d_out_v;
-    a.out_c = b.d_out_c;
     a.load_shift = b.tune.load_shift;
     return a;
 }
 
 cudaError_t launch_walk(const BatchArgs &a, const BatchTune &t, int sms, cudaStream_t st)
 {
-    const size_t smem = 4ull * a.smem_queries;
     int occ = 1;
     switch (t.block) {
-    case 128: occ = walk_occupancy<128>(smem); break;
-    case 512: occ = walk_occupancy<512>(smem); break;
-    default: occ = walk_occupancy<256>(smem); break;
+    case 128: occ = walk_occupancy<128>(); break;
+    case 512: occ = walk_occupancy<512>(); break;
+    default: occ = walk_occupancy<256>(); break;
     }
     if (t.ctas_per_sm > 0 && t.ctas_per_sm < occ) occ = t.ctas_per_sm;
     const int grid = sms * occ;
     switch (t.block) {
-    case 128: batch_walk_kernel<128><<<grid, 128, smem, st>>>(a); break;
-    case 512: batch_walk_kernel<512><<<grid, 512, smem, st>>>(a); break;
-    default: batch_walk_kernel<256><<<grid, 256, smem, st>>>(a); break;
+    case 128: batch_walk_kernel<128><<<grid, 128, 0, st>>>(a); break;
+    case 512: batch_walk_kernel<512><<<grid, 512, 0, st>>>(a); break;
+    default: batch_walk_kernel<256><<<grid, 256, 0, st>>>(a); break;
     }
     return cudaGetLastError();
 }
 
 // The batch pipeline on `st` for the queries already in the state's buffers
-// (their count in d_n).
+// (their count and the outputs in d_in).
 lt_status enqueue_pipeline(lt_engine *e, BatchState &b, uint64_t thr, cudaStream_t st)
 {
     BatchArgs a = args_of(e, b, thr);
@@ -531,11 +568,11 @@ lt_status enqueue_pipeline(lt_engine *e, BatchState &b, uint64_t thr, cudaStream
 }
 
 // Replay the captured pipeline (capturing it first when the buffers, the
-// stop probability or the tuning changed); n goes to the device first.
-lt_status run_graph(lt_engine *e, BatchState &b, uint32_t n, uint64_t thr, cudaStream_t st)
+// stop probability or the tuning changed); `in` goes to the device first.
+lt_status run_graph(lt_engine *e, BatchState &b, const BatchIn &in, uint64_t thr, cudaStream_t st)
 {
-    b.h_n = n;
-    LT_CUDA_TRY(cudaMemcpyAsync(b.d_n, &b.h_n, 4, cudaMemcpyHostToDevice, st));
+    b.h_in = in;
+    LT_CUDA_TRY(cudaMemcpyAsync(b.d_in, &b.h_in, sizeof(BatchIn), cudaMemcpyHostToDevice, st));
     const bool stale = !b.exec || b.graph_thr != thr || b.graph_tune.block != b.tune.block ||
                        b.graph_tune.ctas_per_sm != b.tune.ctas_per_sm || b.graph_tune.load_shift != b.tune.load_shift;
     if (stale) {
@@ -610,11 +647,7 @@ lt_status batch_run_device(lt_engine *e, uint32_t n, const uint32_t *d_sources, 
     LT_CUDA_TRY(cudaMemcpyAsync(b.d_src, d_sources, 4ull * n, cudaMemcpyDeviceToDevice, st));
     LT_CUDA_TRY(cudaMemcpyAsync(b.d_walkers, d_walkers, 8ull * n, cudaMemcpyDeviceToDevice, st));
     LT_CUDA_TRY(cudaMemcpyAsync(b.d_seeds, d_seeds, 8ull * n, cudaMemcpyDeviceToDevice, st));
-    LT_TRY(run_graph(e, b, n, threshold53(prob), st));
-    LT_CUDA_TRY(cudaMemcpyAsync(d_offsets, b.d_qout, 8ull * (n + 1), cudaMemcpyDeviceToDevice, st));
-    LT_CUDA_TRY(cudaMemcpyAsync(d_vertices, b.d_out_v, 4ull * W, cudaMemcpyDeviceToDevice, st));
-    LT_CUDA_TRY(cudaMemcpyAsync(d_counts, b.d_out_c, 4ull * W, cudaMemcpyDeviceToDevice, st));
-    return LT_OK;
+    return run_graph(e, b, BatchIn{n, d_offsets, d_vertices, d_counts}, threshold53(prob), st);
 }
 
 lt_status batch_run(lt_engine *e, uint32_t n, const uint32_t *sources, const uint64_t *walkers, const uint64_t *seeds,
@@ -642,15 +675,22 @@ lt_status batch_run(lt_engine *e, uint32_t n, const uint32_t *sources, const uin
         std::vector<uint64_t> s(n, e->cfg.seed);
         LT_CUDA_TRY(cudaMemcpy(b.d_seeds, s.data(), 8ull * n, cudaMemcpyHostToDevice));
     }
+    // outputs in page-locked memory are written by the kernels themselves: no
+    // copies, and no wait for the pairs' number before them
+    const BatchIn direct{n, (uint64_t *)mapped_host(out_offsets, 8ull * (n + 1)), (uint32_t *)mapped_host(out_vertices, 4 * W),
+                         (uint32_t *)mapped_host(out_counts, 4 * W)};
+    const bool pinned = direct.qout && direct.out_v && direct.out_c;
     LT_CUDA_TRY(cudaEventRecord(e->ev_k0, st));
-    LT_TRY(run_graph(e, b, n, threshold53(prob), st));
+    LT_TRY(run_graph(e, b, pinned ? direct : BatchIn{n, b.d_qout, b.d_out_v, b.d_out_c}, threshold53(prob), st));
     LT_CUDA_TRY(cudaEventRecord(e->ev_k1, st));
     LT_CUDA_TRY(cudaMemcpyAsync(&b.h_hdr, b.d_hdr, sizeof(Header), cudaMemcpyDeviceToHost, st));
-    LT_CUDA_TRY(cudaMemcpyAsync(out_offsets, b.d_qout, 8ull * (n + 1), cudaMemcpyDeviceToHost, st));
-    LT_CUDA_TRY(cudaStreamSynchronize(st));
-    const uint64_t total = out_offsets[n];
-    LT_CUDA_TRY(cudaMemcpyAsync(out_vertices, b.d_out_v, 4ull * total, cudaMemcpyDeviceToHost, st));
-    LT_CUDA_TRY(cudaMemcpyAsync(out_counts, b.d_out_c, 4ull * total, cudaMemcpyDeviceToHost, st));
+    if (!pinned) {
+        LT_CUDA_TRY(cudaMemcpyAsync(out_offsets, b.d_qout, 8ull * (n + 1), cudaMemcpyDeviceToHost, st));
+        LT_CUDA_TRY(cudaStreamSynchronize(st));
+        const uint64_t total = out_offsets[n];
+        LT_CUDA_TRY(cudaMemcpyAsync(out_vertices, b.d_out_v, 4ull * total, cudaMemcpyDeviceToHost, st));
+        LT_CUDA_TRY(cudaMemcpyAsync(out_counts, b.d_out_c, 4ull * total, cudaMemcpyDeviceToHost, st));
+    }
     LT_CUDA_TRY(cudaStreamSynchronize(st));
     if (b.h_hdr.error) return fail(LT_ERR_CAPACITY, "a per-query table overflowed");
     float ms = 0;

@@ -40,5 +40,8 @@ struct HostBuf {
 };
 lt_status host_alloc(HostBuf &b, size_t bytes, bool want_pinned);
 void host_free(HostBuf &b);
+// The device's address of page-locked host memory [p, p + bytes), null where
+// either end is not page-locked memory of one allocation.
+void *mapped_host(const void *p, size_t bytes);
 
 }  // namespace lt

@@ -61,17 +61,6 @@ __global__ void widen_kernel(uint64_t *dst, const uint32_t *src, uint64_t n, uin
 
 unsigned stream_blocks(uint64_t n, int sms) { return (unsigned)std::min<uint64_t>((n + 255) / 256, (uint64_t)sms * 8); }
 
-// The device's view of page-locked host memory, null where p is something else.
-uint64_t *mapped(uint64_t *p)
-{
-    cudaPointerAttributes at{};
-    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
-        cudaGetLastError();
-        return nullptr;
-    }
-    return at.type == cudaMemoryTypeHost ? (uint64_t *)at.devicePointer : nullptr;
-}
-
 // Counter updates of one launch: one per walk (PPR), one per step (PageRank).
 uint64_t count_updates(int app, uint64_t W, uint32_t length)
 {
@@ -269,7 +258,7 @@ lt_status engine_create(lt_graph *g, const lt_engine_cfg &cfg, lt_engine **out)
     {
         const lt_status s = host_alloc(e->h_stats, 64, true);
         if (s != LT_OK) return bail(s);
-        e->h_stats_dev = mapped((uint64_t *)e->h_stats.ptr);
+        e->h_stats_dev = (uint64_t *)mapped_host(e->h_stats.ptr, 64);
     }
     if (!e->resident) {
         lt_status s = ooc_create(e, &e->ooc);
@@ -389,9 +378,9 @@ lt_status engine_run(lt_engine *e, int app, int start, uint32_t source, uint64_t
         // V = 47 000 and 13 us at V = 4.6 M
         uint64_t *dst = e->d_counts, *host_stats = e->h_stats_dev;
         if (counts_out) {
-            uint64_t *first = mapped(counts_out), *last = mapped(counts_out + (g.V - 1));
-            counts_done = first && last == first + (g.V - 1);
-            if (counts_done) dst = first;
+            uint64_t *out = (uint64_t *)mapped_host(counts_out, 8ull * g.V);
+            counts_done = out != nullptr;
+            if (out) dst = out;
         }
         widen_kernel<<<stream_blocks(g.V, e->sms), 256, 0, st>>>(dst, e->d_counts32, g.V, host_stats, e->d_stats);
         LT_CUDA_TRY(cudaGetLastError());

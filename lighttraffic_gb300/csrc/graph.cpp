@@ -26,6 +26,20 @@ lt_status fail(lt_status s, const char *fmt, ...)
 void clear_error() { g_last_error.clear(); }
 const char *last_error() { return g_last_error.c_str(); }
 
+void *mapped_host(const void *p, size_t bytes)
+{
+    cudaPointerAttributes first{}, last{};
+    const uint8_t *end = (const uint8_t *)p + (bytes ? bytes - 1 : 0);
+    if (!p || cudaPointerGetAttributes(&first, p) != cudaSuccess || cudaPointerGetAttributes(&last, end) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    if (first.type != cudaMemoryTypeHost || last.type != cudaMemoryTypeHost || !first.devicePointer ||
+        (uint8_t *)last.devicePointer - (uint8_t *)first.devicePointer != end - (const uint8_t *)p)
+        return nullptr;
+    return first.devicePointer;
+}
+
 lt_status host_alloc(HostBuf &b, size_t bytes, bool want_pinned)
 {
     host_free(b);

@@ -17,7 +17,7 @@
 
 namespace lt {
 
-constexpr uint32_t kPoolWalkers = 256;
+constexpr uint32_t kPoolWalkers = 256, kPoolMin = 16;
 
 // One warp's pool, in shared memory: walker base + at[i] has length len[i].
 struct PprPool {
@@ -99,10 +99,11 @@ __device__ __forceinline__ void ppr_pool_fill(PprPool &pool, uint32_t n, uint32_
 
 // Walkers per pool when W walkers are shared by `warps` warps: an equal share
 // of W, cut into as few pools as hold it.
-inline uint32_t pool_walkers(uint64_t W, uint64_t warps)
+LT_HD uint32_t pool_walkers(uint64_t W, uint64_t warps)
 {
     const uint64_t rounds = (W + warps * kPoolWalkers - 1) / (warps * kPoolWalkers);
-    return rounds ? (uint32_t)((W + warps * rounds - 1) / (warps * rounds)) : 1u;
+    const uint64_t n = rounds ? (W + warps * rounds - 1) / (warps * rounds) : 0;
+    return n < kPoolMin ? kPoolMin : (uint32_t)n;
 }
 
 }  // namespace lt

@@ -92,24 +92,6 @@ __global__ void __launch_bounds__(kGenBlock) degrees_kernel(uint64_t E, uint64_t
         if (hot[i]) atomicAdd(&deg[i], hot[i]);
 }
 
-// Largest u in [lo, V0) with rowptr[u] <= e, found by the whole warp (lo
-// satisfies it, e < rowptr[V0]): 32 probes narrow the range 32-fold.
-__device__ __forceinline__ uint64_t warp_find_row(const uint64_t *rowptr, uint64_t lo, uint64_t V0, uint64_t e)
-{
-    const int lane = threadIdx.x & 31;
-    uint64_t n = V0 - lo;  // the row is in [lo, lo + n)
-    while (n > 1) {
-        const uint64_t step = (n + 31) / 32;
-        const uint64_t at = (uint64_t)lane * step;
-        const bool below = at < n && rowptr[lo + at] <= e;
-        const int k = 31 - __clz(__ballot_sync(0xFFFFFFFFu, below));  // lane 0 always holds
-        lo += (uint64_t)k * step;
-        const uint64_t rest = n - (uint64_t)k * step;
-        n = rest < step ? rest : step;
-    }
-    return lo;
-}
-
 // Column entries.  A warp fills kFillEdges consecutive edges at a time,
 // whatever rows they belong to: the warp finds the rows of its first and last
 // edge, and each lane finds its edge's row between them by a binary search of
@@ -129,7 +111,7 @@ __global__ void __launch_bounds__(kGenBlock) fill_kernel(uint64_t V0, uint64_t E
     const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x / 32);
     for (uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) / 32; w * kFillEdges < E; w += warps) {
         const uint64_t begin = w * kFillEdges, end = begin + kFillEdges < E ? begin + kFillEdges : E;
-        const uint64_t r0 = warp_find_row(rowptr, 0, V0, begin), r1 = warp_find_row(rowptr, r0, V0, end - 1);
+        const uint64_t r0 = warp_find_last(rowptr, 0, V0, begin), r1 = warp_find_last(rowptr, r0, V0, end - 1);
         for (uint64_t e = begin + lane; e < end; e += 32) {
             // the row of e: the largest u in [r0, r1] with rowptr[u] <= e
             uint32_t lo = (uint32_t)r0, n = (uint32_t)(r1 - r0 + 1);

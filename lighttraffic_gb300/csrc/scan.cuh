@@ -11,6 +11,9 @@ constexpr int kScanBlock = 256;
 constexpr int kScanItems = 8;
 constexpr int kScanTile = kScanBlock * kScanItems;
 
+// up to this many elements one CTA scans them (one launch instead of three)
+constexpr uint64_t kScanOneCta = 4 * 8192;
+
 namespace scan_detail {
 
 // Exclusive prefix sum of one value per thread over a block of BLOCK threads
@@ -97,7 +100,53 @@ __global__ void __launch_bounds__(kScanBlock) tile_scan(const In *in, uint64_t n
     }
 }
 
+// The whole scan by one CTA of 1024 threads, 8 elements of each at a time.
+template <typename In, typename Out>
+__global__ void __launch_bounds__(1024) scan_one(const In *in, uint64_t n, Out *out)
+{
+    __shared__ Out warp_tot[32];
+    __shared__ Out total;
+    Out carry = 0;
+    for (uint64_t t0 = 0; t0 < n; t0 += 8 * 1024) {
+        const uint64_t base = t0 + 8ull * threadIdx.x;
+        Out v[8];
+        Out s = 0;
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            v[k] = base + k < n ? (Out)in[base + k] : Out(0);
+            s += v[k];
+        }
+        Out run = carry + block_exclusive<Out, 1024>(s, warp_tot, &total);
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            if (base + k < n) out[base + k] = run;
+            run += v[k];
+        }
+        carry += total;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) out[n] = carry;
+}
+
 }  // namespace scan_detail
+
+// Largest i in [lo, n) with off[i] <= x, by the whole warp (converged); off is
+// ascending and off[lo] <= x: 32 probes narrow the range 32-fold.
+__device__ __forceinline__ uint64_t warp_find_last(const uint64_t *off, uint64_t lo, uint64_t n, uint64_t x)
+{
+    const int lane = threadIdx.x & 31;
+    uint64_t left = n - lo;  // the answer is in [lo, lo + left)
+    while (left > 1) {
+        const uint64_t step = (left + 31) / 32;
+        const uint64_t at = (uint64_t)lane * step;
+        const bool below = at < left && off[lo + at] <= x;
+        const int k = 31 - __clz(__ballot_sync(0xFFFFFFFFu, below));  // lane 0 always holds
+        lo += (uint64_t)k * step;
+        const uint64_t rest = left - (uint64_t)k * step;
+        left = rest < step ? rest : step;
+    }
+    return lo;
+}
 
 // out[i] = sum(in[0..i)) for i in [0, n]; out has n+1 entries (out[n] = total).
 // tmp must hold ceil(n / kScanTile) + 1 Out values.  In and out may not alias.
@@ -106,6 +155,10 @@ cudaError_t exclusive_scan(const In *in, uint64_t n, Out *out, Out *tmp, cudaStr
 {
     const uint64_t nb = (n + kScanTile - 1) / kScanTile;
     if (nb == 0) return cudaMemsetAsync(out, 0, sizeof(Out), st);
+    if (n <= kScanOneCta) {
+        scan_detail::scan_one<In, Out><<<1, 1024, 0, st>>>(in, n, out);
+        return cudaGetLastError();
+    }
     scan_detail::tile_sums<In, Out><<<(unsigned)nb, kScanBlock, 0, st>>>(in, n, tmp);
     scan_detail::scan_sums<Out><<<1, kScanBlock, 0, st>>>(tmp, nb, out + n);
     scan_detail::tile_scan<In, Out><<<(unsigned)nb, kScanBlock, 0, st>>>(in, n, tmp, out);
