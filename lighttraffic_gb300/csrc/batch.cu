@@ -512,7 +512,7 @@ BatchArgs args_of(lt_engine *e, BatchState &b, uint64_t thr)
     a.col = e->d_col;
     a.V = e->g->V;
     a.lim = limit53(thr);
-    a.long_len = thr ? (uint32_t)std::min(1e9, 2.0 * 9007199254740992.0 / (double)thr) + 1u : 0xFFFFFFFFu;
+    a.long_len = ppr_long_len(thr);
     a.hdr = b.d_hdr;
     a.src = b.d_src;
     a.walkers = b.d_walkers;

@@ -108,8 +108,7 @@ lt_status walk_launch(int app, int start, const uint64_t *d_rowptr, const uint32
     a.keys = round_keys(seed);
     a.lim = limit53(app == kWalk ? 0 : threshold53(prob));
     a.by_v = mod_n(V);
-    // twice the mean length, capped where the float would not fit
-    a.long_len = app == kPPR ? (uint32_t)std::min(1e9, 2.0 / prob) + 1u : 0u;
+    a.long_len = ppr_long_len(threshold53(prob));
     a.counts = d_counts;
     a.endpoints = d_endpoints;
     a.paths = d_paths;

@@ -14,6 +14,7 @@
 //   (0, 1]; the test U > p is done exactly in integers as m53 >= floor(p 2^53).
 #pragma once
 
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -234,12 +235,25 @@ struct ModN {
 };
 inline ModN mod_n(uint32_t n) { return ModN{UINT64_MAX / n, n}; }
 #ifdef __CUDACC__
+// x / n for an x that n divides
+__device__ __forceinline__ uint64_t div_exact(const ModN &m, uint64_t x)
+{
+    const uint64_t q = __umul64hi(x, m.inv);  // or one less than the quotient
+    return q + (x - q * m.n ? 1u : 0u);
+}
 __device__ __forceinline__ uint32_t mod_by(const ModN &m, uint64_t x)
 {
     const uint64_t rem = x - __umul64hi(x, m.inv) * m.n;
     return (uint32_t)(rem >= m.n ? rem - m.n : rem);
 }
 #endif
+
+// PPR walks longer than this begin first in their pool: twice the mean
+// length at stop threshold thr = floor(p 2^53).
+inline uint32_t ppr_long_len(uint64_t thr)
+{
+    return thr ? (uint32_t)std::min(1e9, 2.0 * 9007199254740992.0 / (double)thr) + 1u : 0xFFFFFFFFu;
+}
 
 // PPR walk length (src/walk/SingleSource.h:11-18): step = 2, then one more
 // for every draw with U > prob.

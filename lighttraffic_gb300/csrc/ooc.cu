@@ -74,6 +74,7 @@ enum TimerKind { kTGraph = 0, kTCompute = 1, kTZero = 2, kTBucket = 3 };
 // partition share lines.  With the vertex index on the device a hop reads
 // only its col entry from the host: one 32-byte sector (measured 31.9).
 constexpr uint64_t kZeroCopyBytesPerHop = 62;
+constexpr int kZcSplitCtas = 2;  // CTAs per SM of the zero-copy kernel of a split launch
 constexpr uint64_t kZeroCopyBytesPerHopIndexed = 32;
 
 }  // namespace
@@ -90,6 +91,7 @@ struct Ooc {
 
     uint32_t *d_node_off = nullptr;
     uint64_t *d_edge_off = nullptr;
+    uint16_t *d_map = nullptr;
     unsigned long long *d_rp = nullptr, *d_col = nullptr;
 
     uint8_t *d_arena = nullptr;
@@ -111,7 +113,8 @@ struct Ooc {
     uint64_t work_cap = 0;
     unsigned long long *d_stats = nullptr;
 
-    HostBuf h_ctl;   // pinned mirror of d_ctl
+    HostBuf h_ctl;   // pinned mirror of d_ctl, and its device view
+    uint32_t *h_ctl_dev = nullptr;
     HostBuf h_plan;  // pinned plan block
     HostBuf h_work;  // pinned work list
     // device views of h_plan / h_work (null: not mapped, upload by copy)
@@ -123,8 +126,7 @@ struct Ooc {
     uint8_t *h_planin_dev = nullptr;
     uint64_t planin_words = 0;  // words of one half
     uint64_t plan_passes = 0;
-    cudaEvent_t ev_ctl = nullptr;  // the control block's copy to the host has landed
-    cudaEvent_t ev_steps = nullptr;  // the pass's step kernels have ended
+    cudaEvent_t ev_ctl = nullptr;  // the control block has been written to the host
     cudaEvent_t ev_pre = nullptr, ev_aux = nullptr;  // split launches: inputs ready / cached kernel done
     cudaStream_t s_aux = nullptr;  // split launches: the cached-queue kernel's stream
     // wave runs: the policy has yet to see the last iteration's histograms;
@@ -141,6 +143,12 @@ struct Ooc {
 
     std::vector<Queue> q;
     std::unique_ptr<Policy> policy;
+    // table updates made since the last pass (see set_entry)
+    struct Entry {
+        uint32_t p;
+        unsigned long long rp, col;
+    };
+    std::vector<Entry> entries;
     int32_t prev_loaded = -1, prev_computed = -1;
     uint64_t iteration = 0;
     uint64_t zc_threshold = 0;
@@ -259,27 +267,85 @@ uint64_t host_part_bytes(const Ooc &o, uint32_t p)
 
 uint64_t zc_bytes_per_hop(const Ooc &o) { return o.d_index ? kZeroCopyBytesPerHopIndexed : kZeroCopyBytesPerHop; }
 
-__global__ void set_entry_kernel(unsigned long long *rp, unsigned long long *col, uint32_t p, unsigned long long rv,
-                                 unsigned long long cv)
-{
-    rp[p] = rv;
-    col[p] = cv;
-}
+// Table updates travel as kernel arguments: they are ordered on the compute
+// stream with the kernels that read the table and keep the values of the time
+// they were made.  Only step kernels read the table, so updates wait for the
+// next pass and go with its other preparations (pass_begin).
+constexpr uint32_t kEntriesPerLaunch = 32;
+struct EntryBatch {
+    unsigned long long rp[kEntriesPerLaunch], col[kEntriesPerLaunch];
+    uint32_t p[kEntriesPerLaunch];
+    uint32_t n;
+};
 
-// Table updates travel as kernel arguments, so they are ordered on `st` with
-// the kernels that read the table and capture the values at call time.
-lt_status set_entry(Ooc &o, uint32_t p, cudaStream_t st)
+void set_entry(Ooc &o, uint32_t p)
 {
-    set_entry_kernel<<<1, 1, 0, st>>>(o.d_rp, o.d_col, p, o.h_rp[p], o.h_col[p]);
-    LT_CUDA_TRY(cudaGetLastError());
-    o.e->stats.kernel_launches++;
-    return LT_OK;
+    for (Ooc::Entry &x : o.entries)
+        if (x.p == p) {
+            x.rp = o.h_rp[p];
+            x.col = o.h_col[p];
+            return;
+        }
+    o.entries.push_back({p, o.h_rp[p], o.h_col[p]});
 }
 
 __global__ void upload_kernel(uint32_t *dst, const uint32_t *src, uint64_t n)
 {
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) dst[i] = src[i];
+}
+
+// What precedes a pass's step kernels, in one launch: table updates, the work
+// list and its offsets from mapped pinned memory, the control block cleared.
+__global__ void pass_begin_kernel(unsigned long long *rp, unsigned long long *col, const __grid_constant__ EntryBatch e,
+                                  uint32_t *work, const uint32_t *h_work, uint64_t n_work, uint32_t *off,
+                                  const uint32_t *h_off, uint64_t n_off, uint32_t *ctl, uint32_t n_ctl)
+{
+    const uint64_t first = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (uint64_t)gridDim.x * blockDim.x;
+    if (first < e.n) {
+        rp[e.p[first]] = e.rp[first];
+        col[e.p[first]] = e.col[first];
+    }
+    for (uint64_t i = first; i < n_ctl; i += stride) ctl[i] = 0;
+    for (uint64_t i = first; i < n_work; i += stride) work[i] = h_work[i];
+    for (uint64_t i = first; i < n_off; i += stride) off[i] = h_off[i];
+}
+
+// Launches pass_begin_kernel (several where there are many table updates);
+// n_work words of h_work and, with `offsets`, 2 n_work words of h_woff go up.
+lt_status pass_begin(Ooc &o, const uint32_t *h_work, uint64_t n_work, const uint64_t *h_woff, bool offsets)
+{
+    lt_engine &e = *o.e;
+    auto view = [&](const void *p) {
+        return (const uint32_t *)(o.h_work_dev + ((const uint8_t *)p - (const uint8_t *)o.h_work.ptr));
+    };
+    uint64_t n_off = offsets ? 2 * n_work : 0;
+    if (!o.h_work_dev) {
+        if (n_work) LT_CUDA_TRY(cudaMemcpyAsync(o.d_work, h_work, 4 * n_work, cudaMemcpyHostToDevice, e.s_compute));
+        if (n_off) LT_CUDA_TRY(cudaMemcpyAsync(o.d_work_off, h_woff, 4 * n_off, cudaMemcpyHostToDevice, e.s_compute));
+        n_work = n_off = 0;
+    }
+    size_t done = 0;
+    uint32_t n_ctl = o.cleared_words();
+    do {
+        EntryBatch b{};
+        for (; b.n < kEntriesPerLaunch && done < o.entries.size(); b.n++, done++) {
+            b.p[b.n] = o.entries[done].p;
+            b.rp[b.n] = o.entries[done].rp;
+            b.col[b.n] = o.entries[done].col;
+        }
+        const uint64_t words = std::max<uint64_t>(std::max<uint64_t>(n_work, n_off), n_ctl);
+        const uint64_t blocks = std::max<uint64_t>(1, std::min<uint64_t>((words + 255) / 256, 304));
+        pass_begin_kernel<<<(unsigned)blocks, 256, 0, e.s_compute>>>(
+            o.d_rp, o.d_col, b, o.d_work, n_work ? view(h_work) : nullptr, n_work, (uint32_t *)o.d_work_off,
+            n_off ? view(h_woff) : nullptr, n_off, o.d_ctl, n_ctl);
+        LT_CUDA_TRY(cudaGetLastError());
+        e.stats.kernel_launches++;
+        n_work = n_off = 0;
+        n_ctl = 0;
+    } while (done < o.entries.size());
+    o.entries.clear();
+    return LT_OK;
 }
 
 // Copy `words` u32 words at h_src (inside the pinned buffer hb, whose device
@@ -502,8 +568,8 @@ void uncached_entry(Ooc &o, uint32_t p)
     o.h_col[p] = 0;
 }
 
-// Clear v's table entry on the compute stream.  Kernels enqueued before this
-// point may still read the slot; loads into the slot wait for this point.
+// Clear v's table entry before the next step kernel.  Kernels enqueued before
+// this point may still read the slot; loads into the slot wait for them.
 
 lt_status evict_partition(Ooc &o, uint32_t v)
 {
@@ -511,7 +577,8 @@ lt_status evict_partition(Ooc &o, uint32_t v)
     o.slot_of[v] = -1;
     o.part_in_slot[s] = -1;
     uncached_entry(o, v);
-    return set_entry(o, v, o.e->s_compute);
+    set_entry(o, v);
+    return LT_OK;
 }
 
 int32_t free_slot(Ooc &o)
@@ -557,7 +624,7 @@ lt_status start_load(Ooc &o, uint32_t p, int32_t slot, std::vector<std::pair<uin
         deferred->push_back({p, t.b});
     } else {
         LT_CUDA_TRY(cudaStreamWaitEvent(e.s_compute, t.b, 0));
-        LT_TRY(set_entry(o, p, e.s_compute));
+        set_entry(o, p);
     }
     e.stats.graph_loading_calls++;
     e.stats.h2d_graph_bytes += rp_bytes + 4 * (e1 - e0);
@@ -696,6 +763,7 @@ struct Lazy {
     int mode;           // lt::Start
     uint32_t nb, n;     // per-vertex starts: vertex range
     uint64_t begin, count;
+    uint32_t last = 0;  // wave runs: all walkers of partitions p .. last (see lazy_extend)
 };
 
 Lazy lazy_of(Ooc &o, const RunParams &rp, int32_t p, uint64_t begin, uint64_t count)
@@ -713,6 +781,22 @@ Lazy lazy_of(Ooc &o, const RunParams &rp, int32_t p, uint64_t begin, uint64_t co
         z.n = o.g->node_off[p + 1] - z.nb;
     }
     return z;
+}
+
+// Per-vertex starts: the walkers of consecutive partitions of which none has
+// been created yet are those of one larger vertex range, in the same order
+// (walkers j V + v, j-major), so a pass that has room for all of them creates
+// them together.  One partition's per pass made as many passes as there are
+// partitions: PageRank of 7e5 walkers over 70 partitions 71 -> 15 passes, 5.5 ->
+// 1.9 ms.
+void lazy_extend(const Ooc &o, uint32_t p, uint64_t room, Lazy &lz)
+{
+    lz.last = p;
+    if (lz.mode != kStartPerVertex || lz.begin != 0 || lz.count != o.q[p].lazy_total) return;
+    auto fresh = [&](uint32_t x) { return o.q[x].lazy_next == 0 && o.q[x].lazy_total > 0; };
+    while (lz.last + 1 < o.P && fresh(lz.last + 1) && lz.count + o.q[lz.last + 1].lazy_total <= room)
+        lz.count += o.q[++lz.last].lazy_total;
+    lz.n = o.g->node_off[lz.last + 1] - lz.nb;
 }
 
 lt_status step_and_bucket_parts(Ooc &o, const RunParams &rp, const std::vector<uint32_t> &parts, int32_t p,
@@ -790,6 +874,9 @@ lt_status step_and_bucket_parts(Ooc &o, const RunParams &rp, const std::vector<u
     // walkers that read only device memory, mixed into warps waiting on host
     // reads, would move at the host reads' pace (c2: 0.935 -> 0.909 s and
     // 0.952 -> 0.934 s per run; two CTAs per SM for the cached kernel: 0.973).
+    // 512 lanes per SM keep the host link full; more only take issue slots
+    // and cache from the cached kernel (PPR of 8.4 M walks on RMAT 2^24 / 2^28
+    // with 14 of 35 partitions: 4 CTAs per SM 10.1 ms, 3 9.17, 2 9.14, 1 9.14).
     auto in_group = [&](uint32_t x) { return o.zc_mask_any && ((o.zc_mask[x >> 5] >> (x & 31)) & 1u); };
     std::vector<uint32_t> order;
     uint64_t nw_a = 0, walkers_a = 0;  // the cached part of a split launch
@@ -821,10 +908,7 @@ lt_status step_and_bucket_parts(Ooc &o, const RunParams &rp, const std::vector<u
             }
         }
     }
-    if (nw) {
-        LT_TRY(upload(o, o.d_work, o.h_work, o.h_work_dev, h_work, nw));
-        if (multi) LT_TRY(upload(o, o.d_work_off, o.h_work, o.h_work_dev, h_woff, 2 * nw));
-    }
+    LT_TRY(pass_begin(o, h_work, nw, h_woff, multi));
     // Plan the bucketing pass on the device, right behind the step kernel,
     // when the free chunks provably hold every arrival: at most n_in walkers
     // leave, which need at most ceil(n_in / kChunk) chunks plus one per
@@ -834,7 +918,7 @@ lt_status step_and_bucket_parts(Ooc &o, const RunParams &rp, const std::vector<u
     const uint64_t n_in = n_chunk_walkers + G;
     const uint64_t need_max = (n_in + kChunk - 1) / kChunk + std::min<uint64_t>(o.P, n_in);
     bool dev_plan = false;
-    if (o.P <= kSmemPartMax && o.h_planin_dev && !e.cfg.host_plan) {
+    if (o.P <= kSmemPartMax && o.h_planin_dev && o.h_ctl_dev && !e.cfg.host_plan) {
         uint64_t free_after = o.free_chunks.size();
         for (uint32_t x : parts) free_after += o.q[x].dev_chunks.size();
         dev_plan = need_max <= free_after && need_max + o.P <= o.plan_cap;
@@ -869,11 +953,13 @@ lt_status step_and_bucket_parts(Ooc &o, const RunParams &rp, const std::vector<u
         pa.plan_chunks = o.d_planbuf + 2ull * o.P;
         pa.plan_cap = o.plan_cap;
         pa.err = o.ctl_bucket_err();
+        pa.ctl = o.d_ctl;
+        pa.ctl_host = o.h_ctl_dev;
+        pa.ctl_words = (uint32_t)o.ctl_words;
     }
-    LT_CUDA_TRY(cudaMemsetAsync(o.d_ctl, 0, 4ull * o.cleared_words(), e.s_compute));
 
     StepArgs a{};
-    a.t = PartTable{o.d_node_off, o.d_edge_off, o.d_rp, o.d_col, o.P};
+    a.t = PartTable{o.d_node_off, o.d_edge_off, o.d_rp, o.d_col, o.P, o.d_map};
     a.arena = o.d_arena;
     a.work_chunks = o.d_work;
     a.n_chunk_walkers = n_chunk_walkers;
@@ -889,8 +975,11 @@ lt_status step_and_bucket_parts(Ooc &o, const RunParams &rp, const std::vector<u
     a.source = rp.source;
     a.length = rp.length;
     a.run = rp.run;
-    a.seed = e.cfg.seed;
-    a.thr = rp.thr;
+    a.keys = round_keys(e.cfg.seed);
+    a.lim = limit53(rp.thr);
+    a.by_v = mod_n(g.V);
+    if (lz.n) a.by_lazy = mod_n(lz.n);
+    a.long_len = ppr_long_len(rp.thr);
     a.counts = rp.counts;
     a.endpoints = rp.endpoints;
     a.paths = rp.paths;
@@ -953,7 +1042,7 @@ lt_status step_and_bucket_parts(Ooc &o, const RunParams &rp, const std::vector<u
         e.stats.computing_calls++;
         e.stats.kernel_launches++;
         e.stats.split_launches++;
-        grid -= e.sms;
+        grid = std::min(grid - e.sms, kZcSplitCtas * e.sms);
     }
     Ooc::Timed t{ev_get(o), ev_get(o), zc_launch ? kTZero : kTCompute};
     // NVTX ranges name the launch kind for profilers (ncu --nvtx-include)
@@ -965,7 +1054,6 @@ lt_status step_and_bucket_parts(Ooc &o, const RunParams &rp, const std::vector<u
     LT_CUDA_TRY(cudaEventRecord(t.b, e.s_compute));
     o.timed.push_back(t);
     if (split) LT_CUDA_TRY(cudaStreamWaitEvent(e.s_compute, o.ev_aux, 0));
-    LT_CUDA_TRY(cudaEventRecord(o.ev_steps, e.s_compute));
     if (zc_launch)
         e.stats.zerocopy_calls++;
     else
@@ -974,19 +1062,14 @@ lt_status step_and_bucket_parts(Ooc &o, const RunParams &rp, const std::vector<u
     if (deferred) {
         for (auto &d : *deferred) {
             LT_CUDA_TRY(cudaStreamWaitEvent(e.s_compute, d.second, 0));
-            LT_TRY(set_entry(o, d.first, e.s_compute));
+            set_entry(o, d.first);
         }
         deferred->clear();
     }
     uint32_t *h_hist = (uint32_t *)o.h_ctl.ptr;
     if (dev_plan) {
-        // the control block goes to the host on the copy-back stream as soon
-        // as the step kernel ends; plan and bucketing follow the kernel on the
-        // compute stream while the host reads it
-        if (!o.ev_ctl) LT_CUDA_TRY(cudaEventCreateWithFlags(&o.ev_ctl, cudaEventDisableTiming));
-        LT_CUDA_TRY(cudaStreamWaitEvent(e.s_copyback, o.ev_steps, 0));
-        LT_CUDA_TRY(cudaMemcpyAsync(h_hist, o.d_ctl, 4ull * o.ctl_words, cudaMemcpyDeviceToHost, e.s_copyback));
-        LT_CUDA_TRY(cudaEventRecord(o.ev_ctl, e.s_copyback));
+        // the plan kernel writes the control block to mapped host memory; the
+        // host reads it while the bucketing runs
         ScatterArgs sa{};
         sa.in_cur = a.out_cur;
         sa.in_step = a.out_step;
@@ -1006,6 +1089,7 @@ lt_status step_and_bucket_parts(Ooc &o, const RunParams &rp, const std::vector<u
         LT_CUDA_TRY(cudaEventRecord(tb.a, e.s_compute));
         nvtxRangePushA("bucketing");
         cudaError_t bucketed = launch_plan(pa, e.s_compute);
+        if (bucketed == cudaSuccess) bucketed = cudaEventRecord(o.ev_ctl, e.s_compute);
         if (bucketed == cudaSuccess) bucketed = launch_scatter(sa, e.device, e.s_compute);
         nvtxRangePop();
         LT_CUDA_TRY(bucketed);
@@ -1049,7 +1133,12 @@ lt_status step_and_bucket_parts(Ooc &o, const RunParams &rp, const std::vector<u
             refresh(o, x);
         }
     }
-    if (qp) {
+    if (qp && lz.last > (uint32_t)p) {
+        for (uint32_t x = (uint32_t)p; x <= lz.last; x++) {
+            o.q[x].lazy_next = o.q[x].lazy_total;
+            refresh(o, x);
+        }
+    } else if (qp) {
         qp->lazy_next += G;
         refresh(o, (uint32_t)p);
     }
@@ -1219,7 +1308,7 @@ lt_status process(Ooc &o, const RunParams &rp, uint32_t p)
             if (e.cfg.pipeline) LT_TRY(overlap_load(o, rp, p, pending.front().second));
             for (auto &d : pending) {
                 LT_CUDA_TRY(cudaStreamWaitEvent(e.s_compute, d.second, 0));
-                LT_TRY(set_entry(o, d.first, e.s_compute));
+                set_entry(o, d.first);
             }
         }
         o.prev_loaded = (int32_t)p;
@@ -1306,7 +1395,7 @@ lt_status publish_all(Ooc &o, WaveState &w)
     lt_engine &e = *o.e;
     for (auto &d : w.inflight) {
         LT_CUDA_TRY(cudaStreamWaitEvent(e.s_compute, d.second, 0));
-        LT_TRY(set_entry(o, d.first, e.s_compute));
+        set_entry(o, d.first);
         w.loading[d.first] = 0;
     }
     w.inflight.clear();
@@ -1353,7 +1442,7 @@ lt_status wave_step(Ooc &o, const RunParams &rp, WaveState &w, bool &done)
             for (auto &d : inflight) {
                 const cudaError_t q = cudaEventQuery(d.second);
                 if (q == cudaSuccess) {
-                    LT_TRY(set_entry(o, d.first, e.s_compute));
+                    set_entry(o, d.first);
                     loading[d.first] = 0;
                 } else {
                     if (q != cudaErrorNotReady) LT_CUDA_TRY(q);
@@ -1554,7 +1643,7 @@ lt_status wave_step(Ooc &o, const RunParams &rp, WaveState &w, bool &done)
             // iteration's kernel instead of overlapping it
             for (auto &d : inflight) {
                 LT_CUDA_TRY(cudaStreamWaitEvent(e.s_compute, d.second, 0));
-                LT_TRY(set_entry(o, d.first, e.s_compute));
+                set_entry(o, d.first);
                 loading[d.first] = 0;
             }
             inflight.clear();
@@ -1660,7 +1749,7 @@ lt_status wave_step(Ooc &o, const RunParams &rp, WaveState &w, bool &done)
             // (copies finish in the order they were issued on the copy stream)
             o.zc_mask_any = false;
             LT_CUDA_TRY(cudaEventSynchronize(inflight.front().second));
-            LT_TRY(set_entry(o, inflight.front().first, e.s_compute));
+            set_entry(o, inflight.front().first);
             loading[inflight.front().first] = 0;
             inflight.erase(inflight.begin());
             return LT_OK;
@@ -1677,7 +1766,8 @@ lt_status wave_step(Ooc &o, const RunParams &rp, WaveState &w, bool &done)
             return LT_OK;
         }
         w.stalls = 0;
-        const Lazy lz = lazy_p >= 0 ? lazy_of(o, rp, lazy_p, o.q[lazy_p].lazy_next, G) : Lazy{};
+        Lazy lz = lazy_p >= 0 ? lazy_of(o, rp, lazy_p, o.q[lazy_p].lazy_next, G) : Lazy{};
+        if (lazy_p >= 0 && G > 0) lazy_extend(o, (uint32_t)lazy_p, wave_lazy_budget(o, chunks, walkers, UINT64_MAX), lz);
         e.stats.host_sched_ms += now_ms() - t_sched;
         LT_TRY(step_and_bucket_parts(o, rp, parts, lazy_p, lz, false, nullptr));
         o.zc_mask_any = false;
@@ -1703,7 +1793,7 @@ lt_status wave_run(Ooc &o, const RunParams &rp, bool &stop)
             lt_engine &e = *o.e;
             for (auto &d : w.inflight) {
                 LT_CUDA_TRY(cudaStreamWaitEvent(e.s_compute, d.second, 0));
-                LT_TRY(set_entry(o, d.first, e.s_compute));
+                set_entry(o, d.first);
             }
             LT_CUDA_TRY(cudaStreamSynchronize(e.s_compute));
             return LT_OK;
@@ -1783,13 +1873,15 @@ lt_status ooc_create(lt_engine *e, Ooc **out)
     lt_status s = dalloc(&o->d_slots, (uint64_t)o->K * o->slot_stride);
     if (s == LT_OK) s = dalloc(&o->d_node_off, o->P + 1);
     if (s == LT_OK) s = dalloc(&o->d_edge_off, o->P + 1);
+    if (s == LT_OK) s = dalloc(&o->d_map, kPartMapN + 2);
     if (s == LT_OK) s = dalloc(&o->d_rp, o->P);
     if (s == LT_OK) s = dalloc(&o->d_col, o->P);
     if (s == LT_OK) s = dalloc(&o->d_ctl, o->ctl_words);
     if (s == LT_OK) s = dalloc(&o->d_stats, 8);
     if (s == LT_OK) s = host_alloc(o->h_ctl, 4 * o->ctl_words, true);
+    if (s == LT_OK) o->h_ctl_dev = (uint32_t *)mapped_host(o->h_ctl.ptr, 4 * o->ctl_words);
     if (s == LT_OK && (cudaStreamCreateWithFlags(&o->s_aux, cudaStreamNonBlocking) != cudaSuccess ||
-                       cudaEventCreateWithFlags(&o->ev_steps, cudaEventDisableTiming) != cudaSuccess ||
+                       cudaEventCreateWithFlags(&o->ev_ctl, cudaEventDisableTiming) != cudaSuccess ||
                        cudaEventCreateWithFlags(&o->ev_pre, cudaEventDisableTiming) != cudaSuccess ||
                        cudaEventCreateWithFlags(&o->ev_aux, cudaEventDisableTiming) != cudaSuccess))
         s = fail(LT_ERR_CUDA, "stream / event creation failed");
@@ -1805,6 +1897,13 @@ lt_status ooc_create(lt_engine *e, Ooc **out)
         cudaMemset(o->d_rp, 0, 8ull * o->P) != cudaSuccess || cudaMemset(o->d_col, 0, 8ull * o->P) != cudaSuccess ||
         cudaMemset(o->d_ctl, 0, 4ull * o->ctl_words) != cudaSuccess)
         return bail(fail(LT_ERR_CUDA, "partition table upload failed"));
+    if (o->P <= kSmemPartMax) {
+        std::vector<uint16_t> map(kPartMapN + 2, (uint16_t)(o->P - 1));
+        const uint32_t shift = part_map_shift(g.V);
+        for (uint32_t b = 0; b < kPartMapN && ((uint64_t)b << shift) < g.V; b++) map[b] = (uint16_t)g.find_partition(b << shift);
+        if (cudaMemcpy(o->d_map, map.data(), 2 * map.size(), cudaMemcpyHostToDevice) != cudaSuccess)
+            return bail(fail(LT_ERR_CUDA, "partition map upload failed"));
+    }
     o->slot_of.assign(o->P, -1);
     o->part_in_slot.assign(o->K, -1);
     o->last_used.assign(o->P, 0);
@@ -1856,7 +1955,7 @@ void ooc_destroy(Ooc *o)
 {
     if (!o) return;
     drain_timers(*o, true);
-    for (void *p : {(void *)o->d_index, (void *)o->d_slots, (void *)o->d_node_off, (void *)o->d_edge_off, (void *)o->d_rp, (void *)o->d_col,
+    for (void *p : {(void *)o->d_index, (void *)o->d_slots, (void *)o->d_node_off, (void *)o->d_edge_off, (void *)o->d_map, (void *)o->d_rp, (void *)o->d_col,
                     (void *)o->d_arena, (void *)o->d_out, (void *)o->d_ctl, (void *)o->d_planbuf, (void *)o->d_work,
                     (void *)o->d_work_off, (void *)o->d_stats})
         if (p) cudaFree(p);
@@ -1869,7 +1968,7 @@ void ooc_destroy(Ooc *o)
     if (o->d_tier) cudaFree(o->d_tier);
     if (o->ev_tier) cudaEventDestroy(o->ev_tier);
     if (o->ev_ctl) cudaEventDestroy(o->ev_ctl);
-    for (cudaEvent_t ev : {o->ev_steps, o->ev_pre, o->ev_aux})
+    for (cudaEvent_t ev : {o->ev_pre, o->ev_aux})
         if (ev) cudaEventDestroy(ev);
     if (o->s_aux) cudaStreamDestroy(o->s_aux);
     for (cudaEvent_t ev : o->ev_free) cudaEventDestroy(ev);
@@ -2996,7 +3095,7 @@ void serve_close(lt_server *s)
         if (s->wave) {
             // loads still in flight: let them land and publish them
             cudaStreamSynchronize(s->e->s_copy);
-            for (auto &d : s->wave->inflight) set_entry(*s->o, d.first, s->e->s_compute);
+            for (auto &d : s->wave->inflight) set_entry(*s->o, d.first);
             cudaStreamSynchronize(s->e->s_compute);
         }
         drain_timers(*s->o, true);

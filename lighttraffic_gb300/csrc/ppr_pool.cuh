@@ -25,11 +25,11 @@ struct PprPool {
     uint32_t len[kPoolWalkers];
 };
 
-// Fills the pool with walkers base .. base + n - 1 (n <= kPoolWalkers); the
-// whole warp, converged.  Draw is a callable (t, at) -> Rand4: draw t of the
+// Fills the pool with walkers base .. base + n - 1 (n at most its
+// arrays' size); the whole warp, converged.  Draw is a callable (t, at) -> Rand4: draw t of the
 // init draws of walker base + at.
-template <typename Draw>
-__device__ __forceinline__ void ppr_pool_fill(PprPool &pool, uint32_t n, uint32_t long_len, const Limit53 &lim,
+template <typename Pool, typename Draw>
+__device__ __forceinline__ void ppr_pool_fill(Pool &pool, uint32_t n, uint32_t long_len, const Limit53 &lim,
                                               const Draw &draw)
 {
     const unsigned full = 0xFFFFFFFFu, lane = threadIdx.x & 31u, below_me = (1u << lane) - 1u;

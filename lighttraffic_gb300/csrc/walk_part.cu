@@ -25,6 +25,7 @@
 
 #include "lt_core.cuh"
 #include "mem.cuh"
+#include "ppr_pool.cuh"
 #include "scan.cuh"
 #include "walk_part.h"
 
@@ -33,25 +34,10 @@ namespace lt {
 namespace {
 
 constexpr unsigned kFull = 0xFFFFFFFFu;
-// idle lanes a warp waits for before refilling them (all lanes: always): the
-// refill sits on the warp's critical path and PPR's geometric walk lengths
-// would otherwise trigger one nearly every iteration (also in zero-copy
-// launches, where refills are short beside host reads: on c2, thresholds 8
-// and 2 there made runs 4 % and 6 % slower)
-constexpr int kRefillMin = 24;
-
-__device__ __forceinline__ uint32_t find_part(const uint32_t *off, uint32_t P, uint32_t v)
-{
-    uint32_t lo = 0, hi = P - 1;
-    while (lo < hi) {
-        const uint32_t mid = lo + (hi - lo + 1) / 2;
-        if (v < off[mid])
-            hi = mid - 1;
-        else
-            lo = mid;
-    }
-    return lo;
-}
+// idle lanes a warp waits for before it takes more walkers, and before it
+// draws another pool of PPR lengths
+constexpr int kTakeMin = 8;
+constexpr int kRefillMin = 16;
 
 // Row offsets stay in L2 (evict-last), column entries stream (evict-first).
 __device__ __forceinline__ uint64_t ld_u64(unsigned long long addr, uint64_t keep)
@@ -63,35 +49,6 @@ __device__ __forceinline__ uint32_t ld_u32(unsigned long long addr, uint64_t str
     return ld_nc_stream_u32(reinterpret_cast<const void *>(addr), stream);
 }
 
-// Row of vertex cur in the lane's readable partition [nb, ne): the address of
-// its first column entry and its degree.  Row offsets are u64 global edge
-// offsets (rowptr slices in the slots, the reference's layout), or, with the
-// compact device-resident index (a.rp32), u32 offsets relative to the
-// partition's first edge; eb is then the partition's edge count, which ends
-// the last vertex's row.
-// hot: the vertex carries the tier mark (compact index only).
-__device__ __forceinline__ void row_at(bool rp32, unsigned long long rp, unsigned long long col, uint64_t eb,
-                                       uint32_t cur, uint32_t nb, uint32_t ne, uint64_t keep,
-                                       unsigned long long &first_addr, uint64_t &deg, bool &hot)
-{
-    const uint32_t rel = cur - nb;
-    if (rp32) {
-        const uint32_t lo_m = ld_nc_u32(reinterpret_cast<const void *>(rp + 4ull * rel), keep);
-        const uint32_t hi = cur + 1 < ne
-                                ? ld_nc_u32(reinterpret_cast<const void *>(rp + 4ull * (rel + 1)), keep) & ~kHotMark
-                                : (uint32_t)eb;
-        const uint32_t lo = lo_m & ~kHotMark;
-        first_addr = col + 4ull * lo;
-        deg = hi - lo;
-        hot = (lo_m & kHotMark) != 0;
-    } else {
-        hot = false;
-        const uint64_t first = ld_u64(rp + 8ull * rel, keep);
-        deg = ld_u64(rp + 8ull * (rel + 1), keep) - first;
-        first_addr = col + 4ull * (first - eb);
-    }
-}
-
 // Address of the first column entry of marked vertex v in the tier.
 __device__ __forceinline__ unsigned long long hot_first(const StepArgs &a, uint32_t v, uint64_t keep)
 {
@@ -100,47 +57,94 @@ __device__ __forceinline__ unsigned long long hot_first(const StepArgs &a, uint3
     return (unsigned long long)(a.hot_pool + ld_nc_u32(a.hot_off + rank, keep));
 }
 
-// Row of the next update in the lane's readable range; a marked vertex of a
-// zero-copy partition is read from the tier instead of host memory.
-template <bool HOT>
-__device__ __forceinline__ void row_of(const StepArgs &a, unsigned long long rp, unsigned long long col, uint64_t eb,
-                                       uint32_t cur, uint32_t nb, uint32_t ne, bool zc, uint64_t keep,
-                                       unsigned long long &first_addr, uint64_t &deg, bool &zc_read)
+// What a warp keeps in shared memory: its pool of drawn PPR lengths, the
+// walkers that have left (written out 32 at a time: one reservation and
+// 128-byte stores instead of an atomic on one address in nearly every
+// iteration), and, serving, the walks that have ended.
+constexpr uint32_t kPartPool = 128;
+template <bool POOL, bool SERVE>
+struct PartWarp {
+    struct {
+        uint32_t at[POOL ? kPartPool : 1], len[POOL ? kPartPool : 1];
+    } pool;
+    uint32_t cur[64], step[64], idx[64], dest[64], q[SERVE ? 64 : 1];
+    uint2 ends[SERVE ? 64 : 1];  // (query slot, vertex)
+    // its block of input ordinals, the ordinal its pool begins at (of a queued
+    // walker, or of one to be created) and the work chunk holding that
+    uint64_t at, end, base;
+    uint32_t work, exits;
+};
+
+// Shared-memory copy of the partition table of one launch (P <= kSmemPartMax).
+struct SmemTable {
+    const uint32_t *off;            // P + 1
+    uint32_t *hist, *visit;         // P
+    const uint32_t *zc;             // zero-copy mask
+    const unsigned long long *col;  // P: column address, bit 0: zero-copy, 0: unreadable (RP32, P <= kColTableMax)
+    const uint16_t *map;            // kPartMapN + 1
+};
+
+// The partition of v: between the partitions of the first vertices of v's
+// block of 2^map_shift vertices and of the next one.
+__device__ __forceinline__ uint32_t find_part(const StepArgs &a, const SmemTable &t, bool in_smem, uint32_t v)
 {
-    bool marked;
-    row_at(a.rp32, rp, col, eb, cur, nb, ne, keep, first_addr, deg, marked);
-    zc_read = zc;
-    if (HOT && marked && zc) {
-        first_addr = hot_first(a, cur, keep);
-        zc_read = false;
+    uint32_t lo = 0, hi = a.t.P - 1;
+    if (in_smem) {
+        const uint32_t b = v >> a.map_shift;
+        lo = t.map[b];
+        hi = t.map[b + 1];
     }
+    while (lo < hi) {
+        const uint32_t mid = lo + (hi - lo + 1) / 2;
+        if (v < t.off[mid])
+            hi = mid - 1;
+        else
+            lo = mid;
+    }
+    return lo;
 }
 
-// A PPR walk ends at v: count it (single run) or add it to the query's table
-// (linear probing, u32 counts) and mark one more walker of the query done.
-__device__ __forceinline__ void ppr_count(const StepArgs &a, uint32_t qs, uint32_t v)
+// Walker index of lazily created ordinal t.
+__device__ __forceinline__ uint32_t lazy_id(const StepArgs &a, uint64_t t)
 {
-    if (!a.q_seed) {
-        red_add1_u64((unsigned long long *)&a.counts[v], l2_policy_evict_last());
-        return;
-    }
-    const uint64_t base = a.q_toff[qs];
-    const uint64_t mask = (1ull << a.q_tlog[qs]) - 1;
-    uint64_t slot = ((uint64_t)(v * 0x9E3779B1u)) & mask;
-    bool added = false;
-    for (uint64_t probe = 0; probe <= mask && !added; probe++) {
-        uint32_t *k = &a.q_keys[base + slot];
-        uint32_t old = *(volatile uint32_t *)k;
-        if (old == 0xFFFFFFFFu) old = atomicCAS(k, 0xFFFFFFFFu, v);
-        if (old == 0xFFFFFFFFu || old == v) {
-            atomicAdd(&a.q_cnt[base + slot], 1u);
-            added = true;
+    if (a.lazy_mode != kStartPerVertex) return (uint32_t)t;
+    const uint32_t rem = mod_by(a.by_lazy, t);
+    return (uint32_t)(div_exact(a.by_lazy, t - rem) * a.V + a.lazy_nb + rem);
+}
+
+__device__ __forceinline__ void count1(const StepArgs &a, uint32_t v, uint64_t keep)
+{
+    red_add1_u64((unsigned long long *)&a.counts[v], keep);
+}
+
+// A finished walk's endpoints of 32 lanes (or fewer) go to their queries'
+// tables (linear probing, u32 counts); then each query has that many more
+// walkers done.
+__device__ __forceinline__ void serve_count(const StepArgs &a, bool have, uint2 e)
+{
+    const unsigned all = __ballot_sync(kFull, have);
+    if (have) {
+        const uint64_t base = a.q_toff[e.x];
+        const uint64_t mask = (1ull << a.q_tlog[e.x]) - 1;
+        uint64_t slot = ((uint64_t)(e.y * 0x9E3779B1u)) & mask;
+        bool added = false;
+        for (uint64_t probe = 0; probe <= mask && !added; probe++) {
+            uint32_t *k = &a.q_keys[base + slot];
+            uint32_t old = *(volatile uint32_t *)k;
+            if (old == 0xFFFFFFFFu) old = atomicCAS(k, 0xFFFFFFFFu, e.y);
+            if (old == 0xFFFFFFFFu || old == e.y) {
+                atomicAdd(&a.q_cnt[base + slot], 1u);
+                added = true;
+            }
+            slot = (slot + 1) & mask;
         }
-        slot = (slot + 1) & mask;
+        if (!added) atomicAdd(a.q_error, 1ull);
+        __threadfence();
+        const unsigned same = __match_any_sync(all, e.x);
+        if ((threadIdx.x & 31) == (unsigned)__ffs((int)same) - 1u)
+            atomicAdd(&a.q_done[e.x], (unsigned long long)__popc(same));
     }
-    if (!added) atomicAdd(a.q_error, 1ull);
-    __threadfence();
-    atomicAdd(&a.q_done[qs], 1ull);
+    __syncwarp();
 }
 
 // Resident CTAs per SM the register budget is sized for: PPR fits 48
@@ -150,269 +154,372 @@ __device__ __forceinline__ void ppr_count(const StepArgs &a, uint32_t qs, uint32
 template <int APP>
 constexpr int part_min_blocks() { return APP == kPPR ? 5 : 6; }
 
-// HOT: the hot-vertex tier is on (a.hot_on); a separate instance, so that
-// runs without the tier keep the registers of the kernel without it.
-template <int APP, bool HOT>
-__global__ void __launch_bounds__(kPartBlock, part_min_blocks<APP>()) walk_part_kernel(StepArgs a)
+// HOT: the hot-vertex tier is on (a.hot_on); SERVE: query mode (a.q_seed);
+// RP32: row offsets are u32 offsets from the partition's first edge, all
+// partitions' back to back at a.zc_rp_base.  Separate instances keep the
+// registers of the others.
+template <int APP, bool HOT, bool SERVE, bool RP32>
+__global__ void __launch_bounds__(kPartBlock, part_min_blocks<APP>()) walk_part_kernel(const __grid_constant__ StepArgs a)
 {
-    extern __shared__ uint32_t smem[];
+    extern __shared__ __align__(16) uint32_t smem[];
+    __shared__ PartWarp<APP == kPPR && !SERVE, SERVE> s_warp[kPartBlock / 32];
     const uint32_t P = a.t.P;
     const bool in_smem = P <= kSmemPartMax;
-    uint32_t *s_off = smem;
-    uint32_t *s_hist = smem + (P + 1);
-    uint32_t *s_visit = s_hist + P;
-    uint32_t *s_zc = s_visit + P;
+    const bool col_table = RP32 && P <= kColTableMax;
+    SmemTable t{a.t.node_off, a.hist, a.visits, nullptr, nullptr, nullptr};
     if (in_smem) {
-        for (uint32_t i = threadIdx.x; i <= P; i += blockDim.x) s_off[i] = a.t.node_off[i];
-        for (uint32_t i = threadIdx.x; i < P; i += blockDim.x) {
+        uint32_t *s_off = smem + (col_table ? 2 * P : 0), *s_hist = s_off + P + 1, *s_visit = s_hist + P;
+        uint32_t *s_zc = s_visit + P;
+        uint16_t *s_map = reinterpret_cast<uint16_t *>(s_zc + (P + 31) / 32);
+        unsigned long long *s_col = reinterpret_cast<unsigned long long *>(smem);
+        for (uint32_t i = threadIdx.x; i <= P; i += kPartBlock) s_off[i] = a.t.node_off[i];
+        for (uint32_t i = threadIdx.x; i < P; i += kPartBlock) {
             s_hist[i] = 0;
             s_visit[i] = 0;
+            if (col_table) {
+                unsigned long long c = *(volatile const unsigned long long *)&a.t.rp_addr[i] ? a.t.col_addr[i] : 0ull;
+                if (i == a.zc_part)
+                    c = a.zc_col | 1ull;
+                else if (c == 0ull && ((a.zc_mask[i >> 5] >> (i & 31)) & 1u))
+                    c = (a.zc_col_base + 4ull * a.t.edge_off[i]) | 1ull;
+                s_col[i] = c;
+            }
         }
-        for (uint32_t i = threadIdx.x; i < (P + 31) / 32; i += blockDim.x) s_zc[i] = a.zc_mask[i];
+        for (uint32_t i = threadIdx.x; i < (P + 31) / 32; i += kPartBlock) s_zc[i] = a.zc_mask[i];
+        for (uint32_t i = threadIdx.x; i <= kPartMapN / 2; i += kPartBlock)
+            reinterpret_cast<uint32_t *>(s_map)[i] = reinterpret_cast<const uint32_t *>(a.t.map)[i];
+        t = SmemTable{s_off, s_hist, s_visit, s_zc, s_col, s_map};
     }
     __syncthreads();
-    const uint32_t *off = in_smem ? s_off : a.t.node_off;
-    uint32_t *hist = in_smem ? s_hist : a.hist;
-    uint32_t *visit = in_smem ? s_visit : a.visits;
 
     const int lane = threadIdx.x & 31;
-    const unsigned lt_mask = (1u << lane) - 1u;
+    const unsigned below_me = (1u << lane) - 1u;
     const uint64_t total = a.n_chunk_walkers + a.lazy_count;
     const uint64_t keep = l2_policy_evict_last(), stream = l2_policy_evict_first();
+    PartWarp<APP == kPPR && !SERVE, SERVE> &sw = s_warp[threadIdx.x >> 5];
 
-    uint32_t cur = 0, step = 0, idx = 0, hop = 0, qs = 0;
-    uint64_t seed = a.seed;
-    bool active = false, exhausted = false;
-    // cached readable partition of the lane
+    // the warp's block of input ordinals (the first one without the counter),
+    // of which [pool_at, pool_n) are at hand: queued walkers, or walkers to be
+    // created (PPR: with their lengths drawn)
+    const uint64_t dealt = (uint64_t)a.block * ((threadIdx.x >> 5) * gridDim.x + blockIdx.x);
+    bool exhausted = dealt >= total, pool_lazy = false;
+    uint32_t pool_at = 0, pool_n = 0;
+    if (lane == 0) {
+        sw.at = dealt;
+        sw.end = min(dealt + a.block, total);
+        sw.work = sw.exits = 0;
+    }
+    __syncwarp();
+
+    uint32_t cur = 0, step = 0, idx = 0, qs = 0;
+    uint64_t seed = 0;  // SERVE: of the lane's query
+    bool active = false, emit = false, ended = false;
+    uint32_t dest = 0;
+    Rand4 r{};  // PageRank: the draw of the walker's next step
+    // readable range of the lane's partition.  The empty range (1, 0) makes
+    // the next look-up count as an entry into its partition, (2, 1) does not.
     uint32_t cp_nb = 1, cp_ne = 0;
-    unsigned long long cp_rp = 0, cp_col = 0;
-    uint64_t cp_eb = 0;
+    unsigned long long cp_rp = 0, cp_col = 0;  // cp_rp: !RP32, or HOT's one-vertex ranges
+    uint64_t cp_eb = 0;                        // !RP32: the partition's first edge
     bool cp_zc = false;
-    // per-thread statistics of this launch (a launch makes far fewer than
-    // 2^32 updates per thread); widened in the warp reduction at the end
-    uint32_t n_upd = 0, n_mov = 0, n_tel = 0, n_zc = 0, n_exit = 0, n_fin = 0;
+    // statistics of this launch (a thread makes far fewer than 2^32 updates)
+    // n_end: teleports (PageRank), walks that ended early (generic)
+    uint32_t n_mov = 0, n_zc = 0, n_fin = 0, n_end = 0;
+    uint32_t n_out = 0, n_ends = 0;  // walkers / ended walks gathered by the warp
+
+    auto draw = [&](uint32_t s) {
+        return SERVE ? walk_draw(seed, s, kTagStep, a.run, idx) : walk_draw(a.keys, s, kTagStep, a.run, idx);
+    };
+    auto write_out = [&](uint32_t first, uint32_t n) {
+        unsigned long long base = 0;
+        if (lane == 0) base = atomicAdd(a.out_n, (unsigned long long)n);
+        base = __shfl_sync(kFull, base, 0);
+        if ((uint32_t)lane < n) {
+            const uint64_t pos = base + lane;
+            a.out_cur[pos] = sw.cur[first + lane];
+            a.out_step[pos] = sw.step[first + lane];
+            a.out_idx[pos] = sw.idx[first + lane];
+            a.out_dest[pos] = sw.dest[first + lane];
+            a.out_q[pos] = SERVE ? sw.q[first + lane] : 0u;
+        }
+        if (lane == 0) sw.exits += n;
+        __syncwarp();
+    };
 
     while (true) {
-        const unsigned idle = __ballot_sync(kFull, !active);
-        if (idle != 0u && !exhausted && (__popc(idle) >= kRefillMin || idle == kFull)) {
-            const int leader = __ffs(idle) - 1;
-            unsigned long long base = 0;
-            if (lane == leader) base = atomicAdd(a.next, (unsigned long long)__popc(idle));
-            base = __shfl_sync(kFull, base, leader);
-            if (base + __popc(idle) >= total) exhausted = true;
-            if (!active) {
-                const uint64_t my = base + __popc(idle & lt_mask);
-                if (my < a.n_chunk_walkers) {
+        const unsigned left = __ballot_sync(kFull, emit);
+        if (left) {
+            if (emit) {
+                const uint32_t k = n_out + __popc(left & below_me);
+                sw.cur[k] = cur;
+                sw.step[k] = step;
+                sw.idx[k] = idx;
+                sw.dest[k] = dest;
+                if (SERVE) sw.q[k] = qs;
+                atomicAdd(&t.hist[dest], 1u);
+                emit = false;
+            }
+            n_out += __popc(left);
+            __syncwarp();
+            if (n_out >= 32u) {
+                n_out -= 32u;
+                write_out(n_out, 32u);
+            }
+        }
+        if (SERVE) {
+            const unsigned over = __ballot_sync(kFull, ended);
+            if (over) {
+                if (ended) sw.ends[n_ends + __popc(over & below_me)] = make_uint2(qs, cur);
+                ended = false;
+                n_ends += __popc(over);
+                __syncwarp();
+                if (n_ends >= 32u) {
+                    n_ends -= 32u;
+                    serve_count(a, true, sw.ends[n_ends + lane]);
+                }
+            }
+        }
+        const unsigned busy = __ballot_sync(kFull, active);
+        const int idle = 32 - __popc(busy);
+        if (pool_at == pool_n && idle >= kRefillMin && !exhausted) {
+            uint64_t at = sw.at;
+            const uint64_t end = sw.end;
+            pool_at = 0;
+            pool_lazy = at >= a.n_chunk_walkers;
+            const uint64_t base = pool_lazy ? at - a.n_chunk_walkers + a.lazy_begin : at;
+            uint32_t work = sw.work;
+            if (pool_lazy) {
+                pool_n = (uint32_t)(end - at);
+                if (APP == kPPR && !SERVE)
+                    ppr_pool_fill(sw.pool, pool_n, a.long_len, a.lim, [&](uint32_t d, uint32_t w) {
+                        return walk_draw(a.keys, d, kTagInit, a.run, lazy_id(a, base + w));
+                    });
+            } else {
+                pool_n = (uint32_t)(min(end, (uint64_t)a.n_chunk_walkers) - at);
+                if (a.work_off) work = (uint32_t)warp_find_last(a.work_off, work, a.n_work, at);
+            }
+            at += pool_n;
+            if (at == end) {
+                unsigned long long got = 0;
+                if (lane == 0) got = atomicAdd(a.next, (unsigned long long)a.block);
+                at = (uint64_t)a.block * gridDim.x * (kPartBlock / 32) + __shfl_sync(kFull, got, 0);
+            }
+            exhausted = at >= total;
+            __syncwarp();
+            if (lane == 0) {
+                sw.at = at;
+                sw.end = at < end ? end : min(at + a.block, total);
+                sw.base = base;
+                sw.work = work;
+            }
+            __syncwarp();
+        }
+        if (pool_at < pool_n && idle >= kTakeMin) {
+            const uint32_t mine = pool_at + __popc(~busy & below_me);
+            if (!active && mine < pool_n) {
+                active = true;
+                const uint64_t pool_base = sw.base;
+                if (!pool_lazy) {
+                    const uint64_t my = pool_base + mine;
                     uint32_t wi, j;
                     if (!a.work_off) {
                         wi = (uint32_t)(my / kChunk);
                         j = (uint32_t)(my % kChunk);
                     } else {
-                        uint32_t lo = 0, hi = a.n_work - 1;
-                        while (lo < hi) {
-                            const uint32_t mid = lo + (hi - lo + 1) / 2;
-                            if (my < a.work_off[mid])
-                                hi = mid - 1;
-                            else
-                                lo = mid;
-                        }
-                        wi = lo;
-                        j = (uint32_t)(my - a.work_off[lo]);
+                        wi = sw.work;
+                        while (wi + 1 < a.n_work && a.work_off[wi + 1] <= my) wi++;
+                        j = (uint32_t)(my - a.work_off[wi]);
                     }
-                    const uint32_t k = a.work_chunks[wi];
-                    const uint32_t *c = reinterpret_cast<const uint32_t *>(a.arena + (uint64_t)k * kChunkBytes);
+                    const uint32_t *c =
+                        reinterpret_cast<const uint32_t *>(a.arena + (uint64_t)a.work_chunks[wi] * kChunkBytes);
                     cur = c[j];
                     step = c[kChunk + j];
                     idx = c[2 * kChunk + j];
-                    qs = c[3 * kChunk + j];
                     // A walker taken from a queue chunk was counted as
-                    // entering its partition when it was staged there; the
-                    // empty range (2, 1) forces its lookup and marks it as
-                    // not a new entry (counting it again would rank uncached
-                    // partitions by the walkers that queued at them, i.e.
-                    // by the cache state).  (1, 0) is the plain empty range.
+                    // entering its partition when it was staged there
+                    // (counting it again would rank uncached partitions by
+                    // the walkers that queued at them, i.e. by the cache
+                    // state).
                     cp_nb = 2;
                     cp_ne = 1;
-                    if (a.q_seed) seed = a.q_seed[qs];
-                    active = true;
-                } else if (my < total) {
-                    const uint64_t t = a.lazy_begin + (my - a.n_chunk_walkers);
-                    if (a.lazy_mode == kStartPerVertex) {
-                        idx = (uint32_t)per_vertex_id(t, a.lazy_nb, a.lazy_n, a.V);
-                        cur = a.lazy_nb + (uint32_t)(t % a.lazy_n);
-                    } else {
-                        idx = (uint32_t)t;
-                        cur = start_vertex(a.lazy_mode, a.source, a.V, a.seed, a.run, idx);
+                    if (SERVE) {
+                        qs = c[3 * kChunk + j];
+                        seed = a.q_seed[qs];
                     }
-                    qs = 0;
-                    seed = a.seed;
-                    step = APP == kPPR ? ppr_length(a.seed, a.run, idx, a.thr) : a.length;
+                } else {
+                    const uint32_t w = APP == kPPR && !SERVE ? sw.pool.at[mine] : mine;
+                    idx = lazy_id(a, pool_base + w);
+                    if (a.lazy_mode == kStartPerVertex)
+                        cur = a.lazy_nb + mod_by(a.by_lazy, pool_base + w);
+                    else if (a.lazy_mode == kStartSource)
+                        cur = a.source;
+                    else
+                        cur = mod_by(a.by_v, r64_of(walk_draw(a.keys, 0, kTagInit, a.run, idx)));
+                    step = APP == kPPR && !SERVE ? sw.pool.len[mine] : a.length;
                     if (APP == kWalk && a.paths) a.paths[(uint64_t)idx * (a.length + 1)] = cur;
-                    active = true;
+                    // the lane's range holds from its previous walker
                 }
-                hop = a.length - step;
+                if (APP == kPageRank) r = draw(step);
             }
-        }
-        if (__ballot_sync(kFull, active) == 0u) {
-            if (exhausted) break;
-            continue;
-        }
-
-        // Does the next update read the graph, and is the walker's partition readable?
-        Rand4 r{};
-        bool need_graph = false, emit = false;
-        uint32_t dest = 0;
-        if (active) {
-            if (APP == kPPR) {
-                need_graph = step >= 2;
-            } else if (APP == kPageRank) {
-                if (step >= 2) {
-                    r = walk_draw(seed, step, kTagStep, a.run, idx);
-                    need_graph = m53_of(r) < a.thr;
-                }
-            } else {
-                need_graph = true;
-            }
-            if (need_graph && (cur < cp_nb || cur >= cp_ne)) {
-                const uint32_t p = find_part(off, P, cur);
-                if (!(cp_nb == 2 && cp_ne == 1)) atomicAdd(&visit[p], 1u);
-                unsigned long long rp, col = 0;
-                if (p == a.zc_part) {
-                    rp = a.zc_rp | 1ull;
-                    col = a.zc_col;
-                } else {
-                    rp = *(volatile const unsigned long long *)&a.t.rp_addr[p];
-                    if (rp != 0ull) {
-                        col = *(volatile const unsigned long long *)&a.t.col_addr[p];
-                    } else if (in_smem && ((s_zc[p >> 5] >> (p & 31)) & 1u)) {
-                        rp = (a.zc_rp_base + (a.rp32 ? 4ull : 8ull) * off[p]) | 1ull;
-                        col = a.zc_col_base + 4ull * a.t.edge_off[p];
-                    }
-                }
-                bool hot = false;
-                if (HOT && rp == 0ull) {
-                    // unreadable partition: a marked vertex is read from the
-                    // tier, as a one-vertex readable range of the lane
-                    const uint32_t lo_m = ld_nc_u32(reinterpret_cast<const void *>(a.zc_rp_base + 4ull * cur), keep);
-                    if (lo_m & kHotMark) {
-                        const uint32_t lo = lo_m & ~kHotMark;
-                        cp_eb = cur + 1 < off[p + 1]
-                                    ? ld_nc_u32(reinterpret_cast<const void *>(a.zc_rp_base + 4ull * (cur + 1)), keep) &
-                                          ~kHotMark
-                                    : a.t.edge_off[p + 1] - a.t.edge_off[p];
-                        cp_nb = cur;
-                        cp_ne = cur + 1;
-                        cp_rp = a.zc_rp_base + 4ull * cur;
-                        cp_col = hot_first(a, cur, keep) - 4ull * lo;
-                        cp_zc = false;
-                        hot = true;
-                    }
-                }
-                if (hot) {
-                } else if (rp == 0ull) {
-                    emit = true;
-                    dest = p;
-                    cp_nb = 1;
-                    cp_ne = 0;
-                } else {
-                    cp_nb = off[p];
-                    cp_ne = off[p + 1];
-                    cp_rp = rp & ~1ull;
-                    cp_col = col;
-                    cp_eb = a.rp32 ? a.t.edge_off[p + 1] - a.t.edge_off[p] : a.t.edge_off[p];
-                    cp_zc = (rp & 1ull) != 0;
-                }
-            }
-        }
-        const unsigned em = __ballot_sync(kFull, emit);
-        if (em != 0u) {
-            const int leader = __ffs(em) - 1;
-            unsigned long long base = 0;
-            if (lane == leader) base = atomicAdd(a.out_n, (unsigned long long)__popc(em));
-            base = __shfl_sync(kFull, base, leader);
-            if (emit) {
-                const uint64_t pos = base + __popc(em & lt_mask);
-                a.out_cur[pos] = cur;
-                a.out_step[pos] = step;
-                a.out_idx[pos] = idx;
-                a.out_dest[pos] = dest;
-                a.out_q[pos] = qs;
-                atomicAdd(&hist[dest], 1u);
-                active = false;
-                n_exit++;
-            }
+            pool_at = min(pool_n, pool_at + (uint32_t)idle);
+        } else if (idle == 32 && exhausted && pool_at == pool_n) {
+            break;
         }
         if (!active) continue;
 
-        const uint32_t s = step;
-        n_upd++;
+        // Does the next update read the graph, and is the walker's partition readable?
+        const bool need_graph = APP != kPageRank || (step >= 2 && below(r, a.lim));
+        if (need_graph && (cur < cp_nb || cur >= cp_ne)) {
+            const uint32_t p = find_part(a, t, in_smem, cur);
+            if (!(cp_nb == 2 && cp_ne == 1)) atomicAdd(&t.visit[p], 1u);
+            unsigned long long rp = 1ull, col = 0;
+            if (col_table) {
+                col = t.col[p];
+                cp_zc = (col & 1ull) != 0;
+                rp = col;
+                col &= ~1ull;
+            } else if (p == a.zc_part) {
+                rp = a.zc_rp;
+                col = a.zc_col;
+                cp_zc = true;
+            } else {
+                rp = *(volatile const unsigned long long *)&a.t.rp_addr[p];
+                cp_zc = false;
+                if (rp != 0ull) {
+                    col = *(volatile const unsigned long long *)&a.t.col_addr[p];
+                } else if (in_smem && ((t.zc[p >> 5] >> (p & 31)) & 1u)) {
+                    rp = a.zc_rp_base + (RP32 ? 4ull : 8ull) * t.off[p];
+                    col = a.zc_col_base + 4ull * a.t.edge_off[p];
+                    cp_zc = true;
+                }
+            }
+            bool hot = false;
+            if (HOT && rp == 0ull) {
+                // unreadable partition: a marked vertex is read from the
+                // tier, as a one-vertex readable range of the lane
+                const uint32_t lo_m = ld_nc_u32(reinterpret_cast<const void *>(a.zc_rp_base + 4ull * cur), keep);
+                if (lo_m & kHotMark) {
+                    cp_nb = cur;
+                    cp_ne = cur + 1;
+                    cp_col = hot_first(a, cur, keep) - 4ull * (lo_m & ~kHotMark);
+                    cp_zc = false;
+                    hot = true;
+                }
+            }
+            if (hot) {
+            } else if (rp == 0ull) {
+                emit = true;
+                active = false;
+                dest = p;
+                cp_nb = 1;
+                cp_ne = 0;
+                continue;
+            } else {
+                cp_nb = t.off[p];
+                cp_ne = t.off[p + 1];
+                cp_col = col;
+                if (!RP32) {
+                    cp_rp = rp;
+                    cp_eb = a.t.edge_off[p];
+                }
+            }
+        }
+
+        // The row: first column entry and degree.  With RP32 the partition's
+        // edge count ends its last vertex's row.
+        unsigned long long fa = 0;
+        uint64_t deg = 0;
+        bool zc_read = cp_zc;
+        if (need_graph) {
+            if (RP32) {
+                const uint32_t lo_m = ld_nc_u32(reinterpret_cast<const void *>(a.zc_rp_base + 4ull * cur), keep);
+                uint32_t hi;
+                if (cur + 1 < cp_ne) {
+                    hi = ld_nc_u32(reinterpret_cast<const void *>(a.zc_rp_base + 4ull * (cur + 1)), keep);
+                } else {
+                    const uint32_t p = find_part(a, t, in_smem, cur);
+                    hi = HOT && cur + 1 < t.off[p + 1]
+                             ? ld_nc_u32(reinterpret_cast<const void *>(a.zc_rp_base + 4ull * (cur + 1)), keep)
+                             : (uint32_t)(a.t.edge_off[p + 1] - a.t.edge_off[p]);
+                }
+                if (APP == kPageRank) count1(a, cur, keep);
+                if (APP != kPageRank) {
+                    r = draw(step);
+                    asm volatile("" : "+r"(r.x0), "+r"(r.x1));  // here, under the loads
+                }
+                const uint32_t lo = lo_m & ~kHotMark;
+                fa = cp_col + 4ull * lo;
+                deg = (hi & ~kHotMark) - lo;
+                if (HOT && (lo_m & kHotMark) && cp_zc) {
+                    // a marked vertex of a zero-copy partition: from the tier
+                    fa = hot_first(a, cur, keep);
+                    zc_read = false;
+                }
+            } else {
+                const uint32_t rel = cur - cp_nb;
+                const uint64_t first = ld_u64(cp_rp + 8ull * rel, keep);
+                const uint64_t next = ld_u64(cp_rp + 8ull * (rel + 1), keep);
+                if (APP == kPageRank) count1(a, cur, keep);
+                if (APP != kPageRank) {
+                    r = draw(step);
+                    asm volatile("" : "+r"(r.x0), "+r"(r.x1));
+                }
+                deg = next - first;
+                fa = cp_col + 4ull * (first - cp_eb);
+            }
+        } else if (APP == kPageRank) {
+            count1(a, cur, keep);
+        }
+
         bool done = false;
         if (APP == kPPR) {
-            // app/ppr.cu:22-42
-            if (s == 1) {
-                ppr_count(a, qs, cur);
-                done = true;
+            // app/ppr.cu:22-42; step >= 2 here, and a walk whose step comes
+            // down to 1 is counted right away
+            if (deg > 0) {
+                cur = ld_u32(fa + 4ull * mod_u64(r64_of(r), deg), stream);
+                n_mov++;
+                n_zc += zc_read;
+                step--;
             } else {
-                step = s - 1;
-                unsigned long long fa;
-                uint64_t deg;
-                bool zc_read;
-                row_of<HOT>(a, cp_rp, cp_col, cp_eb, cur, cp_nb, cp_ne, cp_zc, keep, fa, deg, zc_read);
-                if (deg > 0) {
-                    const Rand4 q = walk_draw(seed, s, kTagStep, a.run, idx);
-                    cur = ld_u32(fa + 4ull * mod_u64(r64_of(q), deg), stream);
-                    n_mov++;
-                    n_zc += zc_read;
-                } else {
-                    ppr_count(a, qs, cur);
-                    done = true;
-                }
+                step = 1;
+            }
+            done = step == 1;
+            if (done) {
+                if (SERVE)
+                    ended = true;
+                else
+                    red_add1_u64((unsigned long long *)&a.counts[cur], keep);
             }
         } else if (APP == kPageRank) {
             // app/pagerank.cu:26-44; a vertex without out-edges teleports.
-            red_add1_u64((unsigned long long *)&a.counts[cur], keep);
-            if (s == 1) {
-                done = true;
-            } else {
-                step = s - 1;
+            step--;
+            done = step == 0;
+            if (!done) {
                 const uint64_t r64 = r64_of(r);
-                bool tele = !need_graph;
-                if (!tele) {
-                    unsigned long long fa;
-                    uint64_t deg;
-                    bool zc_read;
-                    row_of<HOT>(a, cp_rp, cp_col, cp_eb, cur, cp_nb, cp_ne, cp_zc, keep, fa, deg, zc_read);
-                    if (deg > 0) {
-                        cur = ld_u32(fa + 4ull * mod_u64(r64, deg), stream);
-                        n_mov++;
-                        n_zc += zc_read;
-                    } else {
-                        tele = true;
-                    }
+                if (deg > 0) {
+                    cur = ld_u32(fa + 4ull * mod_u64(r64, deg), stream);
+                    n_mov++;
+                    n_zc += zc_read;
+                } else {
+                    cur = mod_by(a.by_v, r64);
+                    n_end++;
                 }
-                if (tele) {
-                    cur = (uint32_t)mod_u64(r64, a.V);
-                    n_tel++;
-                }
+                r = draw(step);
+                asm volatile("" : "+r"(r.x0), "+r"(r.x1), "+r"(r.x2), "+r"(r.x3));
             }
         } else {
             // app/genericwalk.cu:22-32
-            unsigned long long fa;
-            uint64_t deg;
-            bool zc_read;
-            row_of<HOT>(a, cp_rp, cp_col, cp_eb, cur, cp_nb, cp_ne, cp_zc, keep, fa, deg, zc_read);
-            uint32_t *path = a.paths ? a.paths + (uint64_t)idx * (a.length + 1) : nullptr;
+            uint32_t *path = a.paths ? a.paths + (uint64_t)idx * (a.length + 1) + (a.length - step) : nullptr;
             if (deg > 0) {
-                const Rand4 q = walk_draw(seed, s, kTagStep, a.run, idx);
-                cur = ld_u32(fa + 4ull * mod_u64(r64_of(q), deg), stream);
+                cur = ld_u32(fa + 4ull * mod_u64(r64_of(r), deg), stream);
                 n_mov++;
                 n_zc += zc_read;
-                hop++;
-                if (path) path[hop] = cur;
-                step = s - 1;
+                if (path) path[1] = cur;
+                step--;
             } else {
                 if (path)
-                    for (uint32_t h = hop + 1; h <= a.length; h++) path[h] = kInvalidNode;
+                    for (uint32_t k = 1; k <= step; k++) path[k] = kInvalidNode;
+                n_end++;
                 step = 0;
             }
             done = step == 0;
@@ -423,32 +530,47 @@ __global__ void __launch_bounds__(kPartBlock, part_min_blocks<APP>()) walk_part_
             if (a.endpoints) a.endpoints[idx] = cur;
         }
     }
+    if (n_out) write_out(0, n_out);
+    if (SERVE && n_ends) serve_count(a, (uint32_t)lane < n_ends, sw.ends[lane]);
 
-    uint64_t w_upd = n_upd, w_mov = n_mov, w_tel = n_tel, w_zc = n_zc, w_exit = n_exit, w_fin = n_fin;
+    // Statistics: one atomic per CTA and counter.  A PPR walk makes one update
+    // per hop and one that ends it, a PageRank walk one per hop, teleport and
+    // end, a generic walk one per hop and one where it ends early.
+    __shared__ unsigned long long s_stats[5];
+    if (threadIdx.x < 5) s_stats[threadIdx.x] = 0;
+    __syncthreads();
+    uint64_t w_mov = n_mov, w_zc = n_zc, w_fin = n_fin, w_upd = n_end;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
-        w_upd += __shfl_down_sync(kFull, w_upd, o);
         w_mov += __shfl_down_sync(kFull, w_mov, o);
-        w_tel += __shfl_down_sync(kFull, w_tel, o);
         w_zc += __shfl_down_sync(kFull, w_zc, o);
-        w_exit += __shfl_down_sync(kFull, w_exit, o);
         w_fin += __shfl_down_sync(kFull, w_fin, o);
+        w_upd += __shfl_down_sync(kFull, w_upd, o);
     }
     if (lane == 0) {
-        atomicAdd(&a.stats[0], (unsigned long long)w_upd);
-        atomicAdd(&a.stats[1], (unsigned long long)w_mov);
-        atomicAdd(&a.stats[2], (unsigned long long)w_tel);
-        atomicAdd(&a.stats[3], (unsigned long long)w_zc);
-        atomicAdd(&a.stats[4], (unsigned long long)w_exit);
-        atomicAdd(&a.stats[5], (unsigned long long)w_fin);
+        if (w_upd) atomicAdd(&s_stats[0], (unsigned long long)w_upd);
+        if (w_mov) atomicAdd(&s_stats[1], (unsigned long long)w_mov);
+        if (w_zc) atomicAdd(&s_stats[2], (unsigned long long)w_zc);
+        if (sw.exits) atomicAdd(&s_stats[3], (unsigned long long)sw.exits);
+        if (w_fin) atomicAdd(&s_stats[4], (unsigned long long)w_fin);
     }
-    if (in_smem) {
-        __syncthreads();
-        for (uint32_t i = threadIdx.x; i < P; i += blockDim.x) {
-            if (s_hist[i]) atomicAdd(&a.hist[i], s_hist[i]);
-            if (s_visit[i]) atomicAdd(&a.visits[i], s_visit[i]);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const unsigned long long end_n = s_stats[0], mov = s_stats[1], fin = s_stats[4];
+        const unsigned long long tel = APP == kPageRank ? end_n : 0ull;
+        const unsigned long long upd = mov + (APP == kPageRank ? tel + fin : APP == kPPR ? fin : end_n);
+        if (upd) atomicAdd(&a.stats[0], upd);
+        if (mov) atomicAdd(&a.stats[1], mov);
+        if (tel) atomicAdd(&a.stats[2], tel);
+        if (s_stats[2]) atomicAdd(&a.stats[3], s_stats[2]);
+        if (s_stats[3]) atomicAdd(&a.stats[4], s_stats[3]);
+        if (fin) atomicAdd(&a.stats[5], fin);
+    }
+    if (in_smem)
+        for (uint32_t i = threadIdx.x; i < P; i += kPartBlock) {
+            if (t.hist[i]) atomicAdd(&a.hist[i], t.hist[i]);
+            if (t.visit[i]) atomicAdd(&a.visits[i], t.visit[i]);
         }
-    }
 }
 
 // Tile of kScatterItems walkers per thread.
@@ -695,6 +817,7 @@ __global__ void __launch_bounds__(kPlanBlock) plan_kernel(PlanArgs a)
     __shared__ uint32_t tot_new, tot_slots;
     const uint32_t P = a.P;
     const uint32_t per = (P + kPlanBlock - 1) / kPlanBlock;
+    for (uint32_t i = threadIdx.x; i < a.ctl_words; i += kPlanBlock) a.ctl_host[i] = a.ctl[i];
     uint32_t h[kPerMax], fill[kPerMax], tail[kPerMax], nnew[kPerMax];
     uint32_t my_new = 0, my_slots = 0;
 #pragma unroll
@@ -748,56 +871,93 @@ __global__ void inject_kernel(InjectArgs a)
     }
 }
 
-template <int APP>
+template <int APP, bool HOT, bool SERVE, bool RP32>
+cudaError_t launch_part(const StepArgs &a, int grid, size_t smem, cudaStream_t st)
+{
+    walk_part_kernel<APP, HOT, SERVE, RP32><<<grid, kPartBlock, smem, st>>>(a);
+    return cudaGetLastError();
+}
+
+template <int APP, bool HOT, bool SERVE, bool RP32>
 int occ_part(size_t smem)
 {
-    if (smem > 48 * 1024) {
-        cudaFuncSetAttribute(walk_part_kernel<APP, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        cudaFuncSetAttribute(walk_part_kernel<APP, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    }
+    if (smem > 16 * 1024)
+        cudaFuncSetAttribute(walk_part_kernel<APP, HOT, SERVE, RP32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)smem);
     int n = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, walk_part_kernel<APP, false>, kPartBlock, smem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, walk_part_kernel<APP, HOT, SERVE, RP32>, kPartBlock, smem);
     return n;
+}
+
+// The instances' common occupancy (and their shared-memory limits set).
+template <int APP>
+int occ_app(size_t smem)
+{
+    int n = std::min(occ_part<APP, false, false, true>(smem), occ_part<APP, false, false, false>(smem));
+    n = std::min(n, occ_part<APP, true, false, true>(smem));
+    if (APP == kPPR) {
+        n = std::min(n, occ_part<kPPR, false, true, true>(smem));
+        n = std::min(n, occ_part<kPPR, false, true, false>(smem));
+        n = std::min(n, occ_part<kPPR, true, true, true>(smem));
+    }
+    return n;
+}
+
+template <int APP>
+cudaError_t launch_app(const StepArgs &a, int grid, size_t smem, cudaStream_t st)
+{
+    if (a.rp32) return a.hot_on ? launch_part<APP, true, false, true>(a, grid, smem, st)
+                                : launch_part<APP, false, false, true>(a, grid, smem, st);
+    return launch_part<APP, false, false, false>(a, grid, smem, st);
 }
 
 }  // namespace
 
-size_t part_smem(uint32_t P) { return P <= kSmemPartMax ? sizeof(uint32_t) * (3ull * P + 1 + (P + 31) / 32) : 0; }
+size_t part_smem(uint32_t P)
+{
+    if (P > kSmemPartMax) return 0;
+    return (P <= kColTableMax ? 8ull * P : 0) + 4 * (3ull * P + 1 + (P + 31) / 32) + 2 * (kPartMapN + 2);
+}
 
 int part_grid(int app, int /*start*/, int device, size_t smem, int ctas_per_sm)
 {
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    int occ = app == kPPR ? occ_part<kPPR>(smem) : app == kPageRank ? occ_part<kPageRank>(smem) : occ_part<kWalk>(smem);
+    int occ = app == kPPR ? occ_app<kPPR>(smem) : app == kPageRank ? occ_app<kPageRank>(smem) : occ_app<kWalk>(smem);
     if (ctas_per_sm > 0 && ctas_per_sm < occ) occ = ctas_per_sm;
     if (occ < 1) occ = 1;
     return sms * occ;
 }
 
-cudaError_t launch_walk_part(const StepArgs &a, int app, int grid, cudaStream_t st)
+uint32_t part_map_shift(uint32_t V)
 {
-    const size_t smem = part_smem(a.t.P);
-    switch (app) {
-    case kPPR:
-        if (a.hot_on)
-            walk_part_kernel<kPPR, true><<<grid, kPartBlock, smem, st>>>(a);
-        else
-            walk_part_kernel<kPPR, false><<<grid, kPartBlock, smem, st>>>(a);
-        break;
-    case kPageRank:
-        if (a.hot_on)
-            walk_part_kernel<kPageRank, true><<<grid, kPartBlock, smem, st>>>(a);
-        else
-            walk_part_kernel<kPageRank, false><<<grid, kPartBlock, smem, st>>>(a);
-        break;
-    default:
-        if (a.hot_on)
-            walk_part_kernel<kWalk, true><<<grid, kPartBlock, smem, st>>>(a);
-        else
-            walk_part_kernel<kWalk, false><<<grid, kPartBlock, smem, st>>>(a);
-        break;
+    uint32_t shift = 0;
+    while (((uint64_t)V - 1) >> shift >= kPartMapN) shift++;
+    return shift;
+}
+
+cudaError_t launch_walk_part(const StepArgs &args, int app, int grid, cudaStream_t st)
+{
+    const size_t smem = part_smem(args.t.P);
+    StepArgs a = args;
+    const uint64_t total = a.n_chunk_walkers + a.lazy_count;
+    // no more CTAs than have walkers, but half the grid's
+    const uint64_t need = std::max<uint64_t>((uint64_t)grid / 2, (total + kPartBlock - 1) / kPartBlock);
+    if ((uint64_t)grid > need) grid = (int)std::max<uint64_t>(1, need);
+    const uint64_t warps = (uint64_t)grid * (kPartBlock / 32);
+    const uint64_t rounds = std::max<uint64_t>(1, (total + warps * kPartPool - 1) / (warps * kPartPool));
+    a.block = (uint32_t)std::max<uint64_t>(16, (total + warps * rounds - 1) / (warps * rounds));
+    a.map_shift = part_map_shift(a.V);
+    if (app == kPPR && a.q_seed) {
+        if (!a.rp32) return launch_part<kPPR, false, true, false>(a, grid, smem, st);
+        return a.hot_on ? launch_part<kPPR, true, true, true>(a, grid, smem, st)
+                        : launch_part<kPPR, false, true, true>(a, grid, smem, st);
     }
-    return cudaGetLastError();
+    switch (app) {
+    case kPPR: return launch_app<kPPR>(a, grid, smem, st);
+    case kPageRank: return launch_app<kPageRank>(a, grid, smem, st);
+    default: return launch_app<kWalk>(a, grid, smem, st);
+    }
 }
 
 cudaError_t launch_plan(const PlanArgs &a, cudaStream_t st)

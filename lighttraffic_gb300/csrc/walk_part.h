@@ -11,12 +11,16 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "lt_core.cuh"
+
 namespace lt {
 
 constexpr uint32_t kChunk = 8192;                         // walkers per chunk
 constexpr uint64_t kChunkBytes = 16ull * kChunk;           // 128 KiB
 constexpr int kPartBlock = 256;
 constexpr uint32_t kSmemPartMax = 4096;                    // P up to this keeps node_off / histograms in smem
+constexpr uint32_t kColTableMax = 1536;                    // P up to this: column addresses in smem too
+constexpr uint32_t kPartMapN = 2048;                       // blocks of vertices of the partition map
 constexpr uint32_t kZcMaskWords = kSmemPartMax / 32;       // zero-copy set of one launch, one bit per partition
 
 // Device view of the partition table: node / edge ranges of every partition
@@ -32,6 +36,9 @@ struct PartTable {
     const unsigned long long *rp_addr;    // P, 0 = not readable
     const unsigned long long *col_addr;   // P
     uint32_t P;
+    // partition of vertex b << part_map_shift(V) for b < kPartMapN (P - 1
+    // past the last vertex), kPartMapN + 2 entries; P <= kSmemPartMax only
+    const uint16_t *map;
 };
 
 struct StepArgs {
@@ -53,8 +60,11 @@ struct StepArgs {
     uint32_t source;
     uint32_t length;
     uint32_t run;
-    uint64_t seed;
-    uint64_t thr;
+    RoundKeys keys;                // of the seed
+    Limit53 lim;                   // of floor(p 2^53): PPR stop prob or PageRank alpha
+    ModN by_v, by_lazy;            // remainders by V and by lazy_n
+    uint32_t long_len;             // PPR: walks longer than this begin first in their pool
+    uint32_t block, map_shift;     // input ordinals a warp takes at a time; set by the launcher
     uint64_t *counts;
     uint32_t *endpoints;
     uint32_t *paths;
@@ -133,6 +143,10 @@ struct PlanArgs {
     uint32_t *cursor, *win_off, *plan_chunks;  // the ScatterArgs plan
     uint64_t plan_cap;
     unsigned int *err;           // bit 1 set when the stack or the plan buffer is too small
+    // the pass's control block (histogram first), copied to mapped host memory
+    const uint32_t *ctl;
+    uint32_t *ctl_host;
+    uint32_t ctl_words;
 };
 constexpr uint32_t kNoChunk = 0xFFFFFFFFu;
 constexpr uint32_t kHotMark = 0x80000000u;   // tier mark in a device index entry
@@ -148,6 +162,8 @@ struct InjectArgs {
     uint64_t seed, thr;
 };
 
+// log2 of the vertices per block of the partition map
+uint32_t part_map_shift(uint32_t V);
 // Step-kernel grid: SMs x resident CTAs (capped at ctas_per_sm when > 0).
 int part_grid(int app, int start, int device, size_t smem, int ctas_per_sm);
 cudaError_t launch_inject(const InjectArgs &a, int device, cudaStream_t st);
