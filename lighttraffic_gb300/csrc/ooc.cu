@@ -35,6 +35,7 @@
 #include "engine.h"
 #include "lt_core.cuh"
 #include "mlp.h"
+#include "scan.cuh"
 #include "walk_part.h"
 
 namespace lt {
@@ -149,6 +150,8 @@ struct Ooc {
         unsigned long long rp, col;
     };
     std::vector<Entry> entries;
+    // the copy stream waits for every pass submitted so far
+    bool copy_waits = false;
     int32_t prev_loaded = -1, prev_computed = -1;
     uint64_t iteration = 0;
     uint64_t zc_threshold = 0;
@@ -599,10 +602,14 @@ lt_status start_load(Ooc &o, uint32_t p, int32_t slot, std::vector<std::pair<uin
 {
     lt_engine &e = *o.e;
     lt_graph &g = *o.g;
-    cudaEvent_t free_ev = ev_get(o);
-    LT_CUDA_TRY(cudaEventRecord(free_ev, e.s_compute));
-    LT_CUDA_TRY(cudaStreamWaitEvent(e.s_copy, free_ev, 0));
-    o.ev_free.push_back(free_ev);
+    if (!o.copy_waits) {
+        // once for all loads between two passes
+        cudaEvent_t free_ev = ev_get(o);
+        LT_CUDA_TRY(cudaEventRecord(free_ev, e.s_compute));
+        LT_CUDA_TRY(cudaStreamWaitEvent(e.s_copy, free_ev, 0));
+        o.ev_free.push_back(free_ev);
+        o.copy_waits = true;
+    }
 
     const uint64_t n0 = g.node_off[p], n1 = g.node_off[p + 1];
     const uint64_t e0 = g.edge_off[p], e1 = g.edge_off[p + 1];
@@ -746,6 +753,8 @@ lt_status unspill(Ooc &o, uint32_t p, uint64_t max_chunks)
 }
 
 void serve_args(Ooc &o, StepArgs &a);
+void serve_plan_args(Ooc &o, PlanArgs &a);
+void serve_published(Ooc &o, const PlanArgs &a);
 
 struct RunParams {
     int app, start;
@@ -858,6 +867,7 @@ lt_status step_and_bucket_parts(Ooc &o, const RunParams &rp, const std::vector<u
     lt_engine &e = *o.e;
     lt_graph &g = *o.g;
     const double t_submit = now_ms();
+    o.copy_waits = false;
     Queue *qp = p >= 0 ? &o.q[p] : nullptr;
     uint64_t n_chunk_walkers = 0, nw = 0;
     for (uint32_t x : parts) {
@@ -956,6 +966,7 @@ lt_status step_and_bucket_parts(Ooc &o, const RunParams &rp, const std::vector<u
         pa.ctl = o.d_ctl;
         pa.ctl_host = o.h_ctl_dev;
         pa.ctl_words = (uint32_t)o.ctl_words;
+        if (o.serve) serve_plan_args(o, pa);
     }
 
     StepArgs a{};
@@ -1102,6 +1113,7 @@ lt_status step_and_bucket_parts(Ooc &o, const RunParams &rp, const std::vector<u
         const double w0 = now_ms();
         LT_CUDA_TRY(cudaEventSynchronize(o.ev_ctl));
         e.stats.host_wait_ms += now_ms() - w0;
+        if (o.serve) serve_published(o, pa);
     } else {
         LT_CUDA_TRY(cudaMemcpyAsync(h_hist, o.d_ctl, 4ull * o.ctl_words, cudaMemcpyDeviceToHost, e.s_compute));
         e.stats.host_submit_ms += now_ms() - t_submit;
@@ -2713,11 +2725,17 @@ struct lt_server {
     uint64_t thr = 0;
     uint64_t *d_seed = nullptr, *d_toff = nullptr;
     uint32_t *d_tlog = nullptr, *d_keys = nullptr, *d_cnt = nullptr;
-    unsigned long long *d_done = nullptr, *d_err = nullptr, *d_outn = nullptr;
-    uint32_t *d_out_v = nullptr, *d_out_c = nullptr;
+    unsigned long long *d_done = nullptr, *d_err = nullptr;
+    unsigned long long *d_outn = nullptr;  // pair counters of an extraction, zero between two
+    // mapped pinned memory the kernels read and write directly: copies on the
+    // compute stream would queue behind partition loads, or wait for pages
+    lt::HostBuf h_done;      // finished-walker counters, written by each pass's plan kernel
+    bool done_fresh = false;
+    lt::HostBuf h_admit;     // AdmitQuery records, then the chunk ids of their windows
+    cudaEvent_t ev_admit = nullptr;
+    lt::HostBuf h_fin;       // ExtractQuery records, then their pair counts
+    lt::HostBuf h_out;       // pairs of finished queries: vertices, then counts
     uint64_t out_cap = 0;
-    uint64_t *d_meta = nullptr;  // extraction metadata: table base, size, output base and count per finished query
-    lt::HostBuf h_done;
     std::vector<Query *> slots;
     std::deque<Query *> pending;
     std::map<uint64_t, Query *> all;
@@ -2738,39 +2756,101 @@ double serve_now_ms()
 
 namespace {
 
-__global__ void serve_slot_kernel(uint64_t *seed, uint64_t *toff, uint32_t *tlog, unsigned long long *done,
-                                  uint32_t slot, uint64_t sv, uint64_t tv, uint32_t lv)
-{
-    seed[slot] = sv;
-    toff[slot] = tv;
-    tlog[slot] = lv;
-    done[slot] = 0;
-}
+// A query being admitted: its slot's values and where its walkers go.
+struct AdmitQuery {
+    uint64_t seed, toff, walkers;
+    uint32_t tlog, slot, source, cursor;
+    uint64_t plan;  // first chunk id of its window
+};
 
-__global__ void serve_clear_kernel(uint32_t *keys, uint32_t *cnt, uint64_t base, uint64_t n)
+// Queries of one admission, one row of CTAs each: the slot is set, the table
+// cleared and the walkers written to the source partition's queue (walker i
+// at position cursor + i of the chunk window, its length from (seed, i)).
+// One launch for all of them: a burst of 48 took 48 x 3 launches, each with a
+// copy and a wait, some 30 us per query.
+__global__ void __launch_bounds__(256) serve_admit_kernel(const AdmitQuery *queries, const uint32_t *chunks,
+                                                          uint64_t thr, uint8_t *arena, uint64_t *seed, uint64_t *toff,
+                                                          uint32_t *tlog, unsigned long long *done, uint32_t *keys,
+                                                          uint32_t *cnt)
 {
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-        keys[base + i] = 0xFFFFFFFFu;
-        cnt[base + i] = 0;
+    __shared__ AdmitQuery q;
+    if (threadIdx.x < sizeof(AdmitQuery) / 4)
+        reinterpret_cast<uint32_t *>(&q)[threadIdx.x] =
+            reinterpret_cast<const uint32_t *>(queries + blockIdx.y)[threadIdx.x];
+    __syncthreads();
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        seed[q.slot] = q.seed;
+        toff[q.slot] = q.toff;
+        tlog[q.slot] = q.tlog;
+        done[q.slot] = 0;
+    }
+    const uint64_t first = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t i = first; i < 1ull << q.tlog; i += stride) {
+        keys[q.toff + i] = 0xFFFFFFFFu;
+        cnt[q.toff + i] = 0;
+    }
+    for (uint64_t i = first; i < q.walkers; i += stride) {
+        const uint64_t pos = q.cursor + i;
+        const uint32_t chunk = chunks[q.plan + pos / kChunk];
+        uint32_t *c = reinterpret_cast<uint32_t *>(arena + (uint64_t)chunk * kChunkBytes);
+        const uint32_t j = (uint32_t)(pos % kChunk);
+        c[j] = q.source;
+        c[kChunk + j] = ppr_length(q.seed, 0, i, thr);
+        c[2 * kChunk + j] = (uint32_t)i;
+        c[3 * kChunk + j] = q.slot;
     }
 }
 
-// One CTA per finished query: its occupied table slots become (vertex, count)
-// pairs at out + obase[k].
-__global__ void serve_extract_kernel(const uint32_t *keys, const uint32_t *cnt, const uint64_t *tbase,
-                                     const uint64_t *tsize, const uint64_t *obase, unsigned long long *outn,
-                                     uint32_t *out_v, uint32_t *out_c)
+struct ExtractQuery {
+    uint64_t toff, tsize, obase;
+};
+constexpr uint64_t kExtractSlots = 4096;  // table slots a CTA takes at a time
+
+// Finished queries, one row of CTAs each: the occupied table slots become
+// (vertex, count) pairs at out + obase, every kExtractSlots of them with one
+// reservation (one CTA and one atomic per pair for each query: 0.4 ms a
+// launch, the largest 1.1).
+__global__ void __launch_bounds__(256) serve_extract_kernel(const ExtractQuery *queries, const uint32_t *keys,
+                                                            const uint32_t *cnt, unsigned long long *outn,
+                                                            uint32_t *out_v, uint32_t *out_c)
 {
-    const uint32_t k = blockIdx.x;
-    const uint64_t b = tbase[k], n = tsize[k], o = obase[k];
-    for (uint64_t i = threadIdx.x; i < n; i += blockDim.x) {
-        const uint32_t key = keys[b + i];
-        if (key != 0xFFFFFFFFu) {
-            const unsigned long long pos = atomicAdd(&outn[k], 1ull);
-            out_v[o + pos] = key;
-            out_c[o + pos] = cnt[b + i];
+    __shared__ uint32_t warp_tot[8], total;
+    __shared__ uint32_t s_v[kExtractSlots], s_c[kExtractSlots];
+    __shared__ unsigned long long s_base;
+    __shared__ ExtractQuery q;
+    if (threadIdx.x == 0) q = queries[blockIdx.y];
+    __syncthreads();
+    for (uint64_t b = blockIdx.x * kExtractSlots; b < q.tsize; b += gridDim.x * kExtractSlots) {
+        const uint64_t t0 = b + 16ull * threadIdx.x;
+        uint32_t key[16], n = 0;
+#pragma unroll
+        for (int k = 0; k < 16; k++) {
+            key[k] = t0 + k < q.tsize ? keys[q.toff + t0 + k] : 0xFFFFFFFFu;
+            n += key[k] != 0xFFFFFFFFu;
         }
+        uint32_t pos = scan_detail::block_exclusive<uint32_t, 256>(n, warp_tot, &total);
+#pragma unroll
+        for (int k = 0; k < 16; k++)
+            if (key[k] != 0xFFFFFFFFu) {
+                s_v[pos] = key[k];
+                s_c[pos++] = cnt[q.toff + t0 + k];
+            }
+        if (threadIdx.x == 0) s_base = atomicAdd(&outn[blockIdx.y], (unsigned long long)total);
+        __syncthreads();
+        for (uint32_t k = threadIdx.x; k < total; k += 256) {
+            out_v[q.obase + s_base + k] = s_v[k];
+            out_c[q.obase + s_base + k] = s_c[k];
+        }
+        __syncthreads();
+    }
+}
+
+// The pair counters go to the host and back to zero.
+__global__ void serve_outn_kernel(unsigned long long *outn, unsigned long long *host, uint32_t n)
+{
+    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
+        host[i] = outn[i];
+        outn[i] = 0;
     }
 }
 
@@ -2785,6 +2865,17 @@ void serve_args(Ooc &o, StepArgs &a)
     a.q_done = s.d_done;
     a.q_error = s.d_err;
 }
+
+// The plan kernel of a serving pass also publishes the finished-walker
+// counters.
+void serve_plan_args(Ooc &o, PlanArgs &a)
+{
+    lt_server &s = *o.serve;
+    a.done = s.d_done;
+    a.done_host = (unsigned long long *)mapped_host(s.h_done.ptr, s.h_done.bytes);
+    a.n_done = a.done_host ? s.max_active : 0;
+}
+void serve_published(Ooc &o, const PlanArgs &a) { o.serve->done_fresh = a.n_done != 0; }
 
 bool table_alloc(lt_server &s, uint32_t lg, uint64_t &off)
 {
@@ -2820,15 +2911,15 @@ lt_status serve_admit(lt_server &s)
     Ooc &o = *s.o;
     lt_engine &e = *s.e;
     lt_graph &g = *o.g;
+    if (s.pending.empty()) return LT_OK;
+    AdmitQuery *queries = (AdmitQuery *)s.h_admit.ptr;
+    uint32_t *chunks = (uint32_t *)(queries + s.max_active);
+    uint32_t n = 0, slot = 0;
+    uint64_t n_plan = 0, most = 0;
     while (!s.pending.empty()) {
         lt_server::Query *q = s.pending.front();
-        int32_t slot = -1;
-        for (uint32_t i = 0; i < s.max_active; i++)
-            if (!s.slots[i]) {
-                slot = (int32_t)i;
-                break;
-            }
-        if (slot < 0) break;
+        while (slot < s.max_active && s.slots[slot]) slot++;
+        if (slot == s.max_active) break;
         const uint32_t p = g.find_partition(q->source);
         Queue &qp = o.q[p];
         const bool open_tail = !qp.dev_chunks.empty() && qp.tail_fill < kChunk;
@@ -2838,109 +2929,102 @@ lt_status serve_admit(lt_server &s)
         const uint32_t lg = std::max<uint32_t>(5, log2_ceil_host(q->walkers * 2));
         uint64_t toff = 0;
         if (!table_alloc(s, lg, toff)) break;
+        // the last admission's kernel has read its records (long ago)
+        if (n == 0) LT_CUDA_TRY(cudaEventSynchronize(s.ev_admit));
         s.pending.pop_front();
-        q->slot = slot;
+        q->slot = (int32_t)slot;
         q->toff = toff;
         q->tlog = lg;
         q->state = 1;
         s.slots[slot] = q;
         s.live_walkers += q->walkers;
-        serve_slot_kernel<<<1, 1, 0, e.s_compute>>>(s.d_seed, s.d_toff, s.d_tlog, s.d_done, (uint32_t)slot, q->seed,
-                                                   toff, lg);
-        serve_clear_kernel<<<std::max<uint64_t>(1, std::min<uint64_t>((1ull << lg) / 256, 256)), 256, 0,
-                             e.s_compute>>>(s.d_keys, s.d_cnt, toff, 1ull << lg);
         // append the walkers to the source partition's queue
         if (qp.dev_chunks.empty() || qp.tail_fill == kChunk) {
             qp.dev_chunks.push_back(o.free_chunks.back());
             o.free_chunks.pop_back();
             qp.tail_fill = 0;
         }
-        uint32_t *h_chunks = (uint32_t *)o.h_plan.ptr;
-        uint64_t n_plan = 0;
-        h_chunks[n_plan++] = qp.dev_chunks.back();
-        const uint32_t cursor = qp.tail_fill;
+        queries[n++] = AdmitQuery{q->seed, toff, q->walkers, lg, slot, q->source, qp.tail_fill, n_plan};
+        chunks[n_plan++] = qp.dev_chunks.back();
         const uint64_t tot = (uint64_t)qp.tail_fill + q->walkers;
         const uint64_t extra = (tot + kChunk - 1) / kChunk - 1;
         for (uint64_t k = 0; k < extra; k++) {
             const uint32_t c = o.free_chunks.back();
             o.free_chunks.pop_back();
             qp.dev_chunks.push_back(c);
-            h_chunks[n_plan++] = c;
+            chunks[n_plan++] = c;
         }
         qp.tail_fill = (uint32_t)(tot - extra * kChunk);
-        LT_CUDA_TRY(cudaMemcpyAsync(o.d_planbuf, h_chunks, 4 * n_plan, cudaMemcpyHostToDevice, e.s_compute));
-        InjectArgs ia{};
-        ia.arena = o.d_arena;
-        ia.plan_chunks = o.d_planbuf;
-        ia.cursor = cursor;
-        ia.n = q->walkers;
-        ia.source = q->source;
-        ia.qslot = (uint32_t)slot;
-        ia.seed = q->seed;
-        ia.thr = s.thr;
-        LT_CUDA_TRY(launch_inject(ia, e.device, e.s_compute));
-        // the pinned plan block is rewritten by the next admission: let the copy finish
-        LT_CUDA_TRY(cudaStreamSynchronize(e.s_compute));
+        most = std::max(most, std::max<uint64_t>(q->walkers, 1ull << lg));
         refresh(o, p);
     }
+    if (n == 0) return LT_OK;
+    const uint8_t *dev = (const uint8_t *)mapped_host(s.h_admit.ptr, s.h_admit.bytes);
+    if (!dev) return fail(LT_ERR_CUDA, "the admission records are not mapped");
+    const uint32_t *d_chunks = (const uint32_t *)(dev + ((const uint8_t *)chunks - (const uint8_t *)queries));
+    // 2048 items per CTA of the largest query, at most some 16 CTAs per SM in
+    // all; grid rows hold 65 535 queries
+    const uint64_t most_cols = std::max<uint64_t>(1, 16ull * (uint64_t)e.sms / n);
+    const uint64_t cols = std::max<uint64_t>(1, std::min<uint64_t>((most + 2047) / 2048, most_cols));
+    for (uint32_t k = 0; k < n; k += 65535) {
+        serve_admit_kernel<<<dim3((unsigned)cols, std::min<uint32_t>(n - k, 65535)), 256, 0, e.s_compute>>>(
+            (const AdmitQuery *)dev + k, d_chunks, s.thr, o.d_arena, s.d_seed, s.d_toff, s.d_tlog, s.d_done, s.d_keys,
+            s.d_cnt);
+        LT_CUDA_TRY(cudaGetLastError());
+    }
+    LT_CUDA_TRY(cudaEventRecord(s.ev_admit, e.s_compute));
     return LT_OK;
 }
 
 // Extract every active query whose walkers have all finished.
 lt_status serve_complete(lt_server &s, uint32_t &completed)
 {
-    Ooc &o = *s.o;
     lt_engine &e = *s.e;
     completed = 0;
     unsigned long long *h_done = (unsigned long long *)s.h_done.ptr;
-    LT_CUDA_TRY(cudaMemcpyAsync(h_done, s.d_done, 8ull * s.max_active, cudaMemcpyDeviceToHost, e.s_compute));
-    LT_CUDA_TRY(cudaStreamSynchronize(e.s_compute));
+    if (!s.done_fresh) {
+        LT_CUDA_TRY(cudaMemcpyAsync(h_done, s.d_done, 8ull * s.max_active, cudaMemcpyDeviceToHost, e.s_compute));
+        LT_CUDA_TRY(cudaStreamSynchronize(e.s_compute));
+    }
+    s.done_fresh = false;
     std::vector<lt_server::Query *> fin;
-    for (uint32_t i = 0; i < s.max_active; i++)
+    for (uint32_t i = 0; i < s.max_active && fin.size() < 65535; i++)
         if (s.slots[i] && h_done[i] >= s.slots[i]->walkers) fin.push_back(s.slots[i]);
     if (fin.empty()) return LT_OK;
-    std::vector<uint64_t> meta(3 * fin.size());
-    uint64_t obase = 0;
+    ExtractQuery *meta = (ExtractQuery *)s.h_fin.ptr;
+    const unsigned long long *nn = (const unsigned long long *)(meta + s.max_active);
+    uint64_t obase = 0, most = 0;
     for (size_t k = 0; k < fin.size(); k++) {
-        meta[k] = fin[k]->toff;
-        meta[fin.size() + k] = 1ull << fin[k]->tlog;
-        meta[2 * fin.size() + k] = obase;
+        meta[k] = ExtractQuery{fin[k]->toff, 1ull << fin[k]->tlog, obase};
+        most = std::max(most, meta[k].tsize);
         obase += fin[k]->walkers;
     }
     if (obase > s.out_cap) {
         // the output staging grows geometrically (rarely: to the largest
         // batch of finished walkers seen so far)
-        for (void *p : {(void *)s.d_out_v, (void *)s.d_out_c})
-            if (p) cudaFree(p);
-        s.out_cap = std::max<uint64_t>(obase, 2 * s.out_cap);
-        LT_CUDA_TRY(cudaMalloc(&s.d_out_v, 4 * s.out_cap));
-        LT_CUDA_TRY(cudaMalloc(&s.d_out_c, 4 * s.out_cap));
+        const uint64_t cap = std::max<uint64_t>(obase, 2 * s.out_cap);
+        s.out_cap = 0;
+        LT_TRY(host_alloc(s.h_out, 8 * cap, true));
+        s.out_cap = cap;
     }
-    // at most max_active queries finish in one step: the metadata block
-    // allocated at serve_open always holds them
-    uint64_t *d_meta = s.d_meta;
-    unsigned long long *d_n = (unsigned long long *)(d_meta + meta.size());
-    LT_CUDA_TRY(cudaMemcpyAsync(d_meta, meta.data(), 8 * meta.size(), cudaMemcpyHostToDevice, e.s_compute));
-    LT_CUDA_TRY(cudaMemsetAsync(d_n, 0, 8 * fin.size(), e.s_compute));
-    serve_extract_kernel<<<(unsigned)fin.size(), 256, 0, e.s_compute>>>(s.d_keys, s.d_cnt, d_meta, d_meta + fin.size(),
-                                                                          d_meta + 2 * fin.size(), d_n, s.d_out_v,
-                                                                          s.d_out_c);
+    const uint32_t *h_v = (const uint32_t *)s.h_out.ptr, *h_c = h_v + s.out_cap;
+    uint8_t *d_fin = (uint8_t *)mapped_host(s.h_fin.ptr, s.h_fin.bytes);
+    uint32_t *d_v = (uint32_t *)mapped_host(s.h_out.ptr, s.h_out.bytes);
+    if (!d_fin || !d_v) return fail(LT_ERR_CUDA, "the extraction buffers are not mapped");
+    const uint32_t n = (uint32_t)fin.size();
+    const uint64_t cols = std::min<uint64_t>((most + kExtractSlots - 1) / kExtractSlots, 1024);
+    serve_extract_kernel<<<dim3((unsigned)cols, n), 256, 0, e.s_compute>>>((const ExtractQuery *)d_fin, s.d_keys, s.d_cnt,
+                                                                           s.d_outn, d_v, d_v + s.out_cap);
     LT_CUDA_TRY(cudaGetLastError());
-    std::vector<unsigned long long> nn(fin.size());
-    LT_CUDA_TRY(cudaMemcpyAsync(nn.data(), d_n, 8 * fin.size(), cudaMemcpyDeviceToHost, e.s_compute));
+    serve_outn_kernel<<<1, 256, 0, e.s_compute>>>(
+        s.d_outn, (unsigned long long *)(d_fin + sizeof(ExtractQuery) * s.max_active), n);
+    LT_CUDA_TRY(cudaGetLastError());
     LT_CUDA_TRY(cudaStreamSynchronize(e.s_compute));
     const double now = serve_now_ms();
     for (size_t k = 0; k < fin.size(); k++) {
         lt_server::Query *q = fin[k];
-        q->out_v.resize(nn[k]);
-        q->out_c.resize(nn[k]);
-        LT_CUDA_TRY(cudaMemcpyAsync(q->out_v.data(), s.d_out_v + meta[2 * fin.size() + k], 4 * nn[k],
-                                    cudaMemcpyDeviceToHost, e.s_compute));
-        LT_CUDA_TRY(cudaMemcpyAsync(q->out_c.data(), s.d_out_c + meta[2 * fin.size() + k], 4 * nn[k],
-                                    cudaMemcpyDeviceToHost, e.s_compute));
-    }
-    LT_CUDA_TRY(cudaStreamSynchronize(e.s_compute));
-    for (lt_server::Query *q : fin) {
+        q->out_v.assign(h_v + meta[k].obase, h_v + meta[k].obase + nn[k]);
+        q->out_c.assign(h_c + meta[k].obase, h_c + meta[k].obase + nn[k]);
         q->state = 2;
         q->t_done = now;
         s.finished.push_back(q->ticket);
@@ -2949,7 +3033,6 @@ lt_status serve_complete(lt_server &s, uint32_t &completed)
         s.live_walkers -= q->walkers;
         completed++;
     }
-    (void)o;
     return LT_OK;
 }
 
@@ -2983,10 +3066,19 @@ lt_status serve_open(lt_engine *e, uint32_t max_active, uint64_t table_slots, fl
     if (st == LT_OK) st = dalloc(&s->d_err, 1);
     if (st == LT_OK) st = dalloc(&s->d_keys, table_slots);
     if (st == LT_OK) st = dalloc(&s->d_cnt, table_slots);
-    if (st == LT_OK) st = dalloc(&s->d_meta, 4ull * max_active);
+    if (st == LT_OK) st = dalloc(&s->d_outn, max_active);
     if (st == LT_OK) st = host_alloc(s->h_done, 8ull * max_active, true);
+    // windows: every chunk once, and an open one per query
+    if (st == LT_OK)
+        st = host_alloc(s->h_admit, sizeof(AdmitQuery) * (uint64_t)max_active + 4 * ((uint64_t)o.n_chunks + max_active),
+                        true);
+    if (st == LT_OK) st = host_alloc(s->h_fin, (sizeof(ExtractQuery) + 8) * (uint64_t)max_active, true);
+    s->out_cap = 1 << 18;
+    if (st == LT_OK) st = host_alloc(s->h_out, 8 * s->out_cap, true);
     if (st != LT_OK) return bail(st);
-    if (cudaMemset(s->d_done, 0, 8ull * max_active) != cudaSuccess || cudaMemset(s->d_err, 0, 8) != cudaSuccess)
+    if (cudaMemset(s->d_done, 0, 8ull * max_active) != cudaSuccess || cudaMemset(s->d_err, 0, 8) != cudaSuccess ||
+        cudaMemset(s->d_outn, 0, 8ull * max_active) != cudaSuccess ||
+        cudaEventCreateWithFlags(&s->ev_admit, cudaEventDisableTiming) != cudaSuccess)
         return bail(fail(LT_ERR_CUDA, "serving state initialisation failed"));
     reset_queues(o);
     refresh_all(o);
@@ -3104,9 +3196,10 @@ void serve_close(lt_server *s)
         refresh_all(*s->o);
     }
     for (void *p : {(void *)s->d_seed, (void *)s->d_toff, (void *)s->d_tlog, (void *)s->d_keys, (void *)s->d_cnt,
-                    (void *)s->d_done, (void *)s->d_err, (void *)s->d_out_v, (void *)s->d_out_c, (void *)s->d_meta})
+                    (void *)s->d_done, (void *)s->d_err, (void *)s->d_outn})
         if (p) cudaFree(p);
-    host_free(s->h_done);
+    for (HostBuf *b : {&s->h_done, &s->h_admit, &s->h_fin, &s->h_out}) host_free(*b);
+    if (s->ev_admit) cudaEventDestroy(s->ev_admit);
     delete s->wave;
     for (auto &kv : s->all) delete kv.second;
     for (lt_server::Query *q : s->pending)

@@ -818,6 +818,7 @@ __global__ void __launch_bounds__(kPlanBlock) plan_kernel(PlanArgs a)
     const uint32_t P = a.P;
     const uint32_t per = (P + kPlanBlock - 1) / kPlanBlock;
     for (uint32_t i = threadIdx.x; i < a.ctl_words; i += kPlanBlock) a.ctl_host[i] = a.ctl[i];
+    for (uint32_t i = threadIdx.x; i < a.n_done; i += kPlanBlock) a.done_host[i] = a.done[i];
     uint32_t h[kPerMax], fill[kPerMax], tail[kPerMax], nnew[kPerMax];
     uint32_t my_new = 0, my_slots = 0;
 #pragma unroll
@@ -853,21 +854,6 @@ __global__ void __launch_bounds__(kPlanBlock) plan_kernel(PlanArgs a)
         if (!h[j]) continue;
         if (tail[j] != kNoChunk) a.plan_chunks[pos_slot++] = tail[j];
         for (uint32_t c = 0; c < nnew[j]; c++) a.plan_chunks[pos_slot++] = a.stack[pos_new++];
-    }
-}
-
-__global__ void inject_kernel(InjectArgs a)
-{
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += stride) {
-        const uint64_t pos = a.cursor + i;
-        const uint32_t chunk = a.plan_chunks[pos / kChunk];
-        uint32_t *c = reinterpret_cast<uint32_t *>(a.arena + (uint64_t)chunk * kChunkBytes);
-        const uint32_t j = (uint32_t)(pos % kChunk);
-        c[j] = a.source;
-        c[kChunk + j] = ppr_length(a.seed, 0, i, a.thr);
-        c[2 * kChunk + j] = (uint32_t)i;
-        c[3 * kChunk + j] = a.qslot;
     }
 }
 
@@ -964,17 +950,6 @@ cudaError_t launch_plan(const PlanArgs &a, cudaStream_t st)
 {
     if (a.P > kSmemPartMax) return cudaErrorInvalidValue;
     plan_kernel<<<1, kPlanBlock, 0, st>>>(a);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_inject(const InjectArgs &a, int device, cudaStream_t st)
-{
-    if (a.n == 0) return cudaSuccess;
-    int sms = 0;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    uint64_t blocks = (a.n + 255) / 256;
-    if (blocks > (uint64_t)sms * 4) blocks = (uint64_t)sms * 4;
-    inject_kernel<<<(unsigned)blocks, 256, 0, st>>>(a);
     return cudaGetLastError();
 }
 

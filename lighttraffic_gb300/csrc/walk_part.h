@@ -147,26 +147,18 @@ struct PlanArgs {
     const uint32_t *ctl;
     uint32_t *ctl_host;
     uint32_t ctl_words;
+    // serving: the finished-walker counters, likewise
+    const unsigned long long *done;
+    unsigned long long *done_host;
+    uint32_t n_done;
 };
 constexpr uint32_t kNoChunk = 0xFFFFFFFFu;
 constexpr uint32_t kHotMark = 0x80000000u;   // tier mark in a device index entry
-
-// Walkers of newly admitted queries: walker i of query slot q (i < n) goes to
-// position cursor + i of the chunk window, with PPR length from (seed, i).
-struct InjectArgs {
-    uint8_t *arena;
-    const uint32_t *plan_chunks;
-    uint32_t cursor;
-    uint64_t n;
-    uint32_t source, qslot;
-    uint64_t seed, thr;
-};
 
 // log2 of the vertices per block of the partition map
 uint32_t part_map_shift(uint32_t V);
 // Step-kernel grid: SMs x resident CTAs (capped at ctas_per_sm when > 0).
 int part_grid(int app, int start, int device, size_t smem, int ctas_per_sm);
-cudaError_t launch_inject(const InjectArgs &a, int device, cudaStream_t st);
 size_t part_smem(uint32_t P);
 cudaError_t launch_walk_part(const StepArgs &a, int app, int grid, cudaStream_t st);
 cudaError_t launch_scatter(const ScatterArgs &a, int device, cudaStream_t st);
