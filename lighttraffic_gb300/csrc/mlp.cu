@@ -10,12 +10,21 @@
 //                  h = relu(x W1 + b1), y = h . W2 + b2 by a warp reduction;
 //   mlp_backward : one CTA per hidden unit j; threads stride over rows and
 //                  accumulate dL/dW1[:, j], dL/db1[j], dL/dW2[j] (and dL/db2,
-//                  the loss in CTA 0), then a fixed-order tree reduction;
-//                  L = mean (y - t)^2;
-//   mlp_sgd      : v = mu v + g, w -= lr v;
-//   pol_iter / pol_features / pol_labels / pol_demand: the policy's visit
-//                  ring and moving average, feature rows, residual targets
-//                  with the moving-average baseline loss, and forecasts.
+//                  the loss in CTA 0), then a fixed-order tree reduction of
+//                  all sums at once; L = mean (y - t)^2; then the SGD step of
+//                  its own parameters, v = mu v + g, w -= lr v;
+//   pol_step     : one warp per partition: visit ring and moving average,
+//                  feature row, residual target and the network on the row
+//                  that is trained on;
+//   pol_forecast : the network on the new rows, and the forecasts, written to
+//                  page-locked memory.
+// What bounds them is the launches: a few hundred rows make a few us of work,
+// and the host waits for nothing, so the policy costs what its calls cost.  One
+// kernel per stage (visits, features, targets, forward, backward, SGD, forward,
+// forecast, copy) took 9 launches and 3 events for two iterations; the row-wise
+// stages need nothing of another row, so three kernels and one event do: 42 ->
+// 36 us of host time per iteration while serving (70 partitions), a burst of
+// queries 6.15 -> 6.02 ms.
 #include "mlp.h"
 
 #include <algorithm>
@@ -31,13 +40,9 @@ constexpr int F = kMlpIn, H = kMlpHidden;
 constexpr int kOffB1 = F * H, kOffW2 = F * H + H, kOffB2 = F * H + 2 * H;
 constexpr int kBwdThreads = 256;
 
-__global__ void mlp_forward(const float *__restrict__ x, uint32_t n, const float *__restrict__ p,
-                            float *__restrict__ hbuf, float *__restrict__ y)
+// One row by one warp: y on lane 0; h0 and h1 = hidden units lane and lane + 32.
+__device__ float mlp_row(const float *xr, const float *p, int lane, float &h0, float &h1)
 {
-    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) / 32;
-    const int lane = threadIdx.x & 31;
-    if (warp >= n) return;
-    const float *xr = x + (uint64_t)warp * F;
     float a0 = p[kOffB1 + lane], a1 = p[kOffB1 + lane + 32];
 #pragma unroll
     for (int i = 0; i < F; i++) {
@@ -45,45 +50,49 @@ __global__ void mlp_forward(const float *__restrict__ x, uint32_t n, const float
         a0 = fmaf(xi, p[i * H + lane], a0);
         a1 = fmaf(xi, p[i * H + lane + 32], a1);
     }
-    const float h0 = fmaxf(a0, 0.f), h1 = fmaxf(a1, 0.f);
+    h0 = fmaxf(a0, 0.f);
+    h1 = fmaxf(a1, 0.f);
+    float s = h0 * p[kOffW2 + lane] + h1 * p[kOffW2 + lane + 32];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xFFFFFFFFu, s, o);
+    return s + p[kOffB2];
+}
+
+__global__ void mlp_forward(const float *__restrict__ x, uint32_t n, const float *__restrict__ p,
+                            float *__restrict__ hbuf, float *__restrict__ y)
+{
+    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) / 32;
+    const int lane = threadIdx.x & 31;
+    if (warp >= n) return;
+    float h0, h1;
+    const float v = mlp_row(x + (uint64_t)warp * F, p, lane, h0, h1);
     if (hbuf) {
         hbuf[(uint64_t)warp * H + lane] = h0;
         hbuf[(uint64_t)warp * H + lane + 32] = h1;
     }
-    float s = h0 * p[kOffW2 + lane] + h1 * p[kOffW2 + lane + 32];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xFFFFFFFFu, s, o);
-    if (lane == 0) y[warp] = s + p[kOffB2];
+    if (lane == 0) y[warp] = v;
 }
 
-__device__ float block_sum(float v, float *sh)
-{
-    sh[threadIdx.x] = v;
-    __syncthreads();
-    for (int s = kBwdThreads / 2; s > 0; s >>= 1) {
-        if ((int)threadIdx.x < s) sh[threadIdx.x] += sh[threadIdx.x + s];
-        __syncthreads();
-    }
-    const float r = sh[0];
-    __syncthreads();
-    return r;
-}
-
+// Gradients to grad, the loss before the step to *loss and, where base is given,
+// the mean square of the targets to *base (CTA 0); with lr > 0 the step of the
+// CTA's own parameters follows (no other CTA reads them).
 __global__ void __launch_bounds__(kBwdThreads) mlp_backward(const float *__restrict__ x, const float *__restrict__ t,
-                                                            uint32_t n, const float *__restrict__ p,
+                                                            uint32_t n, float *p, float *mom,
                                                             const float *__restrict__ hbuf,
                                                             const float *__restrict__ y, float *__restrict__ grad,
-                                                            float *__restrict__ loss)
+                                                            float *loss, float *base, float lr, float mu)
 {
-    __shared__ float sh[kBwdThreads];
-    const int j = blockIdx.x;
+    constexpr int kAll = F + 5;  // W1 column | b1 | W2 | b2 | loss | base
+    __shared__ float sh[kAll][kBwdThreads];
+    const int j = blockIdx.x, k = threadIdx.x;
+    const int vals = j == 0 ? kAll : F + 2;
     const float w2 = p[kOffW2 + j];
     const float inv_n = 1.0f / (float)n;
     float gw1[F];
 #pragma unroll
     for (int i = 0; i < F; i++) gw1[i] = 0.f;
-    float gb1 = 0.f, gw2 = 0.f, gb2 = 0.f, l = 0.f;
-    for (uint32_t r = threadIdx.x; r < n; r += kBwdThreads) {
+    float gb1 = 0.f, gw2 = 0.f, gb2 = 0.f, l = 0.f, b = 0.f;
+    for (uint32_t r = k; r < n; r += kBwdThreads) {
         const float diff = y[r] - t[r];
         const float dy = 2.0f * diff * inv_n;
         const float h = hbuf[(uint64_t)r * H + j];
@@ -91,6 +100,7 @@ __global__ void __launch_bounds__(kBwdThreads) mlp_backward(const float *__restr
         if (j == 0) {
             gb2 += dy;
             l = fmaf(diff, diff, l);
+            b = fmaf(t[r], t[r], b);
         }
         const float da = h > 0.f ? dy * w2 : 0.f;
         gb1 += da;
@@ -98,33 +108,38 @@ __global__ void __launch_bounds__(kBwdThreads) mlp_backward(const float *__restr
         for (int i = 0; i < F; i++) gw1[i] = fmaf(x[(uint64_t)r * F + i], da, gw1[i]);
     }
 #pragma unroll
-    for (int i = 0; i < F; i++) {
-        const float s = block_sum(gw1[i], sh);
-        if (threadIdx.x == 0) grad[i * H + j] = s;
+    for (int i = 0; i < F; i++) sh[i][k] = gw1[i];
+    sh[F][k] = gb1;
+    sh[F + 1][k] = gw2;
+    sh[F + 2][k] = gb2;
+    sh[F + 3][k] = l;
+    sh[F + 4][k] = b;
+    __syncthreads();
+    // the pairs (i, i + s), s = 128 .. 1: down to 32 values in shared memory,
+    // then each warp finishes every eighth sum in registers
+    for (int s = kBwdThreads / 2; s >= 32; s >>= 1) {
+        if (k < s)
+            for (int v = 0; v < vals; v++) sh[v][k] += sh[v][k + s];
+        __syncthreads();
     }
-    const float sb1 = block_sum(gb1, sh);
-    const float sw2 = block_sum(gw2, sh);
-    if (threadIdx.x == 0) {
-        grad[kOffB1 + j] = sb1;
-        grad[kOffW2 + j] = sw2;
-    }
-    if (j == 0) {
-        const float sb2 = block_sum(gb2, sh);
-        const float sl = block_sum(l, sh);
-        if (threadIdx.x == 0) {
-            grad[kOffB2] = sb2;
-            *loss = sl * inv_n;
+    for (int v = k / 32; v < vals; v += kBwdThreads / 32) {
+        float sum = sh[v][k & 31];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) sum += __shfl_down_sync(0xFFFFFFFFu, sum, o);
+        if (k & 31) continue;
+        if (v == F + 3) {
+            *loss = sum * inv_n;
+        } else if (v == F + 4) {
+            if (base) *base = sum / (float)n;
+        } else {
+            const int at = v < F ? v * H + j : v == F ? kOffB1 + j : v == F + 1 ? kOffW2 + j : kOffB2;
+            grad[at] = sum;
+            if (lr > 0.f) {
+                const float m = mu * mom[at] + sum;
+                mom[at] = m;
+                p[at] -= lr * m;
+            }
         }
-    }
-}
-
-__global__ void mlp_sgd(float *p, const float *g, float *m, float lr, float mu)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < kMlpParams) {
-        const float v = mu * m[i] + g[i];
-        m[i] = v;
-        p[i] -= lr * v;
     }
 }
 
@@ -250,37 +265,23 @@ lt_status Mlp::train(const float *h_x, const float *h_y, uint32_t n, float lr, f
     LT_CUDA_TRY(cudaSetDevice(device_));
     LT_TRY(upload(h_x, h_y, n));
     mlp_forward<<<(n * 32 + 255) / 256, 256, 0, st_>>>(d_x_, n, d_params_, d_h_, d_pred_);
-    mlp_backward<<<H, kBwdThreads, 0, st_>>>(d_x_, d_y_, n, d_params_, d_h_, d_pred_, d_grad_, d_loss_);
+    mlp_backward<<<H, kBwdThreads, 0, st_>>>(d_x_, d_y_, n, d_params_, d_mom_, d_h_, d_pred_, d_grad_, d_loss_, nullptr,
+                                             lr, momentum);
     if (h_pred) LT_CUDA_TRY(cudaMemcpyAsync(h_pred, d_pred_, 4ull * n, cudaMemcpyDeviceToHost, st_));
     if (h_grad) LT_CUDA_TRY(cudaMemcpyAsync(h_grad, d_grad_, 4 * kMlpParams, cudaMemcpyDeviceToHost, st_));
-    if (lr > 0.f) mlp_sgd<<<(kMlpParams + 255) / 256, 256, 0, st_>>>(d_params_, d_grad_, d_mom_, lr, momentum);
     LT_CUDA_TRY(cudaGetLastError());
     if (h_loss) LT_CUDA_TRY(cudaMemcpyAsync(h_loss, d_loss_, 4, cudaMemcpyDeviceToHost, st_));
     LT_CUDA_TRY(cudaStreamSynchronize(st_));
     return LT_OK;
 }
 
-lt_status Mlp::train_dev(const float *d_x, const float *d_y, uint32_t n, float lr, float momentum, float *d_loss)
+lt_status Mlp::learn_dev(const float *d_x, const float *d_y, uint32_t n, float lr, float momentum, float *loss,
+                         float *base)
 {
     if (n > cap_) return fail(LT_ERR_CAPACITY, "MLP batch of %u rows exceeds %u", n, cap_);
-    mlp_forward<<<(n * 32 + 255) / 256, 256, 0, st_>>>(d_x, n, d_params_, d_h_, d_pred_);
-    mlp_backward<<<H, kBwdThreads, 0, st_>>>(d_x, d_y, n, d_params_, d_h_, d_pred_, d_grad_, d_loss);
-    mlp_sgd<<<(kMlpParams + 255) / 256, 256, 0, st_>>>(d_params_, d_grad_, d_mom_, lr, momentum);
+    mlp_backward<<<H, kBwdThreads, 0, st_>>>(d_x, d_y, n, d_params_, d_mom_, d_h_, d_pred_, d_grad_, loss, base, lr,
+                                             momentum);
     LT_CUDA_TRY(cudaGetLastError());
-    return LT_OK;
-}
-
-lt_status Mlp::forward_dev(const float *d_x, uint32_t n, float *d_pred)
-{
-    if (n > cap_) return fail(LT_ERR_CAPACITY, "MLP batch of %u rows exceeds %u", n, cap_);
-    mlp_forward<<<(n * 32 + 255) / 256, 256, 0, st_>>>(d_x, n, d_params_, nullptr, d_pred);
-    LT_CUDA_TRY(cudaGetLastError());
-    return LT_OK;
-}
-
-lt_status Mlp::record(cudaEvent_t ev)
-{
-    LT_CUDA_TRY(cudaEventRecord(ev, st_));
     return LT_OK;
 }
 
@@ -297,81 +298,93 @@ constexpr int kRunWarm = 16;      // iterations of a run before its own forecast
 constexpr double kGateKeep = 0.8;  // running average of the validation losses the gate compares
 constexpr int kRing = kHist + kLabelHorizon + 1;    // visit history ring (iterations)
 constexpr int kSnaps = kLabelHorizon / kEvery + 2;  // feature snapshots awaiting labels
-constexpr int kStage = 4;                           // host staging slots (iterations in flight)
+constexpr int kPairs = 2;                           // host staging slots (kEvery iterations each) in flight
+constexpr int kStageWords = kEvery + 3;             // P words each: visits of kEvery iterations | dyn
 
 // ---- device side of the policy: features, labels and forecasts.  The host
-// stages per iteration the visits of every partition (u32) and, every kEvery
-// iterations, its waiting walkers, residency and iterations since last use
-// (f32); everything else lives on the device.
+// stages the visits of every partition in each of kEvery iterations (u32) and,
+// with the last of them, its waiting walkers, residency and iterations since
+// last use (f32); everything else lives on the device.
 
-// ring[slot] = visits; ema = kEmaKeep ema + (1 - kEmaKeep) visits.
-__global__ void pol_iter(uint32_t *ring, float *ema, const uint32_t *visits, uint32_t P, uint32_t slot)
+// One warp per partition p, at iteration t (a multiple of kEvery):
+//  - the staged visits of iterations t - kEvery + 1 .. t: ring[i mod kRing] = v,
+//    ema = kEmaKeep ema + (1 - kEmaKeep) v;
+//  - with X: the feature row of iteration t (layout in mlp.h), one value per
+//    lane; dyn = waiting | resident | gap;
+//  - with Xold: the target of the snapshot taken kLabelHorizon iterations before
+//    t, the visits since then as a correction to the snapshot's moving-average
+//    forecast, and the network on that snapshot (h, pred), for the training step.
+constexpr int kPolThreads = 128;
+__global__ void __launch_bounds__(kPolThreads) pol_step(uint32_t *ring, float *ema, const float *__restrict__ stat,
+                                                        const uint32_t *__restrict__ visits,
+                                                        const float *__restrict__ dyn, float *X, const float *Xold,
+                                                        float *Y, const float *params, float *hbuf, float *pred,
+                                                        uint32_t P, uint64_t t)
 {
-    for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < P; p += gridDim.x * blockDim.x) {
-        const uint32_t v = visits[p];
-        ring[(uint64_t)slot * P + p] = v;
-        ema[p] = kEmaKeep * ema[p] + (1.0f - kEmaKeep) * (float)v;
+    const uint32_t p = (blockIdx.x * kPolThreads + threadIdx.x) / 32;
+    const int lane = threadIdx.x & 31;
+    if (p >= P) return;
+    float e = ema[p];
+#pragma unroll
+    for (int i = 0; i < kEvery; i++) {
+        const uint32_t v = visits[(uint64_t)i * P + p];
+        if (lane == 0) ring[(uint64_t)((t - kEvery + 1 + i) % kRing) * P + p] = v;
+        e = kEmaKeep * e + (1.0f - kEmaKeep) * (float)v;
     }
-}
-
-// Feature rows of iteration t (layout in mlp.h).  dyn = waiting | resident | gap.
-__global__ void pol_features(float *X, const uint32_t *ring, const float *ema, const float *stat, const float *dyn,
-                             uint32_t P, uint64_t t)
-{
-    for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < P; p += gridDim.x * blockDim.x) {
-        float *x = X + (uint64_t)p * kMlpIn;
-        x[0] = log1pf(dyn[p]) / 16.0f;
-        for (int k = 0; k < kHist; k++)
-            x[1 + k] = (uint64_t)k < t ? log1pf((float)ring[(uint64_t)((t - k) % kRing) * P + p]) / 16.0f : 0.0f;
-        x[9] = stat[p];
-        x[10] = stat[P + p];
-        x[11] = dyn[P + p];
-        x[12] = log1pf(dyn[2 * P + p]) / 16.0f;
-        x[13] = log1pf(ema[p]) / 16.0f;
-        x[14] = (float)p / (float)P;
-        x[15] = log1pf(ema[p] * (float)kLabelHorizon) / 16.0f;  // moving-average forecast
+    __syncwarp();
+    if (lane == 0) ema[p] = e;
+    if (X && lane < kMlpIn) {
+        float f;
+        if (lane == 0) {
+            f = log1pf(dyn[p]) / 16.0f;
+        } else if (lane <= kHist) {
+            const int k = lane - 1;
+            f = (uint64_t)k < t ? log1pf((float)ring[(uint64_t)((t - k) % kRing) * P + p]) / 16.0f : 0.0f;
+        } else if (lane < 11) {
+            f = stat[(uint64_t)(lane - 9) * P + p];
+        } else if (lane == 11) {
+            f = dyn[P + p];
+        } else if (lane == 12) {
+            f = log1pf(dyn[2ull * P + p]) / 16.0f;
+        } else if (lane == 13) {
+            f = log1pf(e) / 16.0f;
+        } else if (lane == 14) {
+            f = (float)p / (float)P;
+        } else {
+            f = log1pf(e * (float)kLabelHorizon) / 16.0f;  // moving-average forecast
+        }
+        X[(uint64_t)p * kMlpIn + lane] = f;
     }
-}
-
-// Targets for the snapshot taken kLabelHorizon iterations before t: the
-// visits since then, as a correction to the snapshot's moving-average
-// forecast; base = the mean squared error of that forecast alone (one CTA,
-// fixed reduction order).
-__global__ void __launch_bounds__(256) pol_labels(float *Y, float *base, const float *Xold, const uint32_t *ring,
-                                                  uint32_t P, uint64_t t)
-{
-    __shared__ float sh[256];
-    float acc = 0.f;
-    for (uint32_t p = threadIdx.x; p < P; p += 256) {
+    if (Xold) {
         float sum = 0.f;
         for (int k = 0; k < kLabelHorizon; k++) sum += (float)ring[(uint64_t)((t - k) % kRing) * P + p];
-        const float y = log1pf(sum) / 16.0f - Xold[(uint64_t)p * kMlpIn + 15];
-        Y[p] = y;
-        acc = fmaf(y, y, acc);
+        const float *xr = Xold + (uint64_t)p * kMlpIn;
+        float h0, h1;
+        const float y = mlp_row(xr, params, lane, h0, h1);
+        hbuf[(uint64_t)p * H + lane] = h0;
+        hbuf[(uint64_t)p * H + lane + 32] = h1;
+        if (lane == 0) {
+            Y[p] = log1pf(sum) / 16.0f - xr[15];
+            pred[p] = y;
+        }
     }
-    sh[threadIdx.x] = acc;
-    __syncthreads();
-    for (int s = 128; s > 0; s >>= 1) {
-        if ((int)threadIdx.x < s) sh[threadIdx.x] += sh[threadIdx.x + s];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) *base = sh[0] / (float)P;
 }
 
 // demand = visits over the label horizon as the network predicts them;
 // base_demand = the same from the moving-average forecast alone.
-__global__ void pol_demand(float *demand, float *base_demand, const float *pred, const float *X, uint32_t P)
+__global__ void __launch_bounds__(kPolThreads) pol_forecast(float *demand, float *base_demand, const float *X,
+                                                            const float *params, uint32_t P)
 {
-    for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < P; p += gridDim.x * blockDim.x) {
-        const float f = X[(uint64_t)p * kMlpIn + 15];
-        demand[p] = expm1f(fmaxf(0.f, f + pred[p]) * 16.0f);
+    const uint32_t p = (blockIdx.x * kPolThreads + threadIdx.x) / 32;
+    if (p >= P) return;
+    const float *xr = X + (uint64_t)p * kMlpIn;
+    float h0, h1;
+    const float y = mlp_row(xr, params, threadIdx.x & 31, h0, h1);
+    if ((threadIdx.x & 31) == 0) {
+        const float f = xr[15];
+        demand[p] = expm1f(fmaxf(0.f, f + y) * 16.0f);
         base_demand[p] = expm1f(fmaxf(0.f, f) * 16.0f);
     }
-}
-
-__global__ void pol_copy(float *dst, const float *src, uint32_t n)
-{
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) dst[i] = src[i];
 }
 
 // Eviction scores are predicted visits (walkers entering the partition,
@@ -401,11 +414,9 @@ public:
 
     ~LearnedPolicy() override
     {
-        if (ev_) cudaEventDestroy(ev_);
-        for (cudaEvent_t e : stage_ev_)
+        for (cudaEvent_t e : pair_ev_)
             if (e) cudaEventDestroy(e);
-        for (void *q : {(void *)d_ring_, (void *)d_ema_, (void *)d_stat_, (void *)d_X_, (void *)d_Y_, (void *)d_out_,
-                        (void *)d_pred_})
+        for (void *q : {(void *)d_ring_, (void *)d_ema_, (void *)d_stat_, (void *)d_X_, (void *)d_Y_})
             if (q) cudaFree(q);
         host_free(h_stage_);
         host_free(h_out_);
@@ -426,22 +437,18 @@ public:
         LT_CUDA_TRY(cudaMalloc(&d_stat_, 8ull * P_));
         LT_CUDA_TRY(cudaMalloc(&d_X_, 4ull * kSnaps * P_ * kMlpIn));
         LT_CUDA_TRY(cudaMalloc(&d_Y_, 4ull * P_));
-        LT_CUDA_TRY(cudaMalloc(&d_out_, 4ull * (2 * P_ + 2)));
-        LT_CUDA_TRY(cudaMalloc(&d_pred_, 4ull * P_));
         LT_CUDA_TRY(cudaMemset(d_ring_, 0, 4ull * kRing * P_));
         LT_CUDA_TRY(cudaMemset(d_ema_, 0, 4ull * P_));
-        LT_CUDA_TRY(cudaMemset(d_out_, 0, 4ull * (2 * P_ + 2)));
         LT_CUDA_TRY(cudaMemcpy(d_stat_, stat_.data(), 8ull * P_, cudaMemcpyHostToDevice));
-        LT_TRY(host_alloc(h_stage_, 16ull * P_ * kStage, true));
+        LT_TRY(host_alloc(h_stage_, 4ull * kStageWords * P_ * kPairs, true));
         LT_TRY(host_alloc(h_out_, 4ull * (2 * P_ + 2), true));
         if (!h_stage_.pinned || !h_out_.pinned) return fail(LT_ERR_NOMEM, "pinned staging for the prefetcher");
         void *dv = nullptr;
         LT_CUDA_TRY(cudaHostGetDevicePointer(&dv, h_stage_.ptr, 0));
-        stage_dev_ = (uint8_t *)dv;
+        stage_dev_ = (uint32_t *)dv;
         LT_CUDA_TRY(cudaHostGetDevicePointer(&dv, h_out_.ptr, 0));
         out_dev_ = (float *)dv;
-        LT_CUDA_TRY(cudaEventCreateWithFlags(&ev_, cudaEventDisableTiming));
-        for (cudaEvent_t &e : stage_ev_) LT_CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        for (cudaEvent_t &e : pair_ev_) LT_CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         return LT_OK;
     }
 
@@ -475,25 +482,25 @@ public:
             return;
         }
         if (failed_) return;
-        // stage this iteration's visits (slot reused kStage iterations later)
-        const int slot = (int)(t_ % kStage);
-        if (cudaEventSynchronize(stage_ev_[slot]) != cudaSuccess) return fail_net();
-        uint8_t *stage = (uint8_t *)h_stage_.ptr + 16ull * P_ * slot;
-        const uint8_t *stage_dev = stage_dev_ + 16ull * P_ * slot;
-        std::memcpy(stage, v.visits, 4ull * P_);
+        // stage this iteration's visits; a slot is used again kPairs * kEvery iterations later
+        const int at = (int)((t_ - 1) % kEvery);
+        const int slot = (int)((t_ - 1) / kEvery % kPairs);
+        uint32_t *stage = (uint32_t *)h_stage_.ptr + (uint64_t)kStageWords * P_ * slot;
+        if (at == 0 && cudaEventSynchronize(pair_ev_[slot]) != cudaSuccess) return fail_net();
+        std::memcpy(stage + (uint64_t)at * P_, v.visits, 4ull * P_);
+        if (t_ % kEvery) return;
         cudaStream_t st = net_.stream();
-        const unsigned blocks = (P_ + 255) / 256;
-        pol_iter<<<blocks, 256, 0, st>>>(d_ring_, d_ema_, (const uint32_t *)stage_dev, P_, (uint32_t)(t_ % kRing));
-        if (t_ % kEvery) {
-            if (cudaEventRecord(stage_ev_[slot], st) != cudaSuccess) fail_net();
-            return;
-        }
+        const uint32_t *stage_dev = stage_dev_ + (uint64_t)kStageWords * P_ * slot;
+        const float *dyn_dev = (const float *)(stage_dev + (uint64_t)kEvery * P_);
+        const unsigned blocks = (unsigned)((P_ + kPolThreads / 32 - 1) / (kPolThreads / 32));
         // pick up the previous prediction pass if it has finished; never wait for it
         if (inflight_) {
-            if (cudaEventQuery(ev_) != cudaSuccess) {
+            if (cudaEventQuery(pair_ev_[inflight_slot_]) != cudaSuccess) {
                 cudaGetLastError();
                 skipped_++;
-                if (cudaEventRecord(stage_ev_[slot], st) != cudaSuccess) fail_net();
+                pol_step<<<blocks, kPolThreads, 0, st>>>(d_ring_, d_ema_, d_stat_, stage_dev, dyn_dev, nullptr, nullptr,
+                                                         d_Y_, net_.params(), net_.hidden(), net_.pred(), P_, t_);
+                if (cudaGetLastError() != cudaSuccess || cudaEventRecord(pair_ev_[slot], st) != cudaSuccess) fail_net();
                 return;
             }
             inflight_ = false;
@@ -519,35 +526,34 @@ public:
                 net_used_ += net;
             }
         }
-        float *dyn = (float *)(stage + 4ull * P_);
+        float *dyn = (float *)(stage + (uint64_t)kEvery * P_);
         for (uint32_t p = 0; p < P_; p++) {
             dyn[p] = (float)v.waiting[p];
             dyn[P_ + p] = v.slot_of[p] >= 0 ? 1.0f : 0.0f;
-            dyn[2 * P_ + p] = (float)(v.iteration - std::min<uint64_t>(v.iteration, v.last_used[p]));
+            dyn[2ull * P_ + p] = (float)(v.iteration - std::min<uint64_t>(v.iteration, v.last_used[p]));
         }
         const int s = (int)((t_ / kEvery) % kSnaps);
         float *Xs = d_X_ + (uint64_t)s * P_ * kMlpIn;
-        pol_features<<<blocks, 256, 0, st>>>(Xs, d_ring_, d_ema_, d_stat_, (const float *)(stage_dev + 4ull * P_), P_,
-                                             t_);
         snap_t_[s] = t_;
         // train on the snapshot whose label horizon has passed
         const int old = (int)(((t_ / kEvery) + kSnaps - (kLabelHorizon / kEvery)) % kSnaps);
-        if (t_ >= (uint64_t)kLabelHorizon + kEvery && snap_t_[old] + kLabelHorizon == t_) {
-            const float *Xo = d_X_ + (uint64_t)old * P_ * kMlpIn;
-            pol_labels<<<1, 256, 0, st>>>(d_Y_, d_out_ + P_ + 1, Xo, d_ring_, P_, t_);
-            if (net_.train_dev(Xo, d_Y_, P_, kLearningRate, kMomentum, d_out_ + P_) != LT_OK) return fail_net();
+        const bool train = t_ >= (uint64_t)kLabelHorizon + kEvery && snap_t_[old] + kLabelHorizon == t_;
+        const float *Xo = train ? d_X_ + (uint64_t)old * P_ * kMlpIn : nullptr;
+        pol_step<<<blocks, kPolThreads, 0, st>>>(d_ring_, d_ema_, d_stat_, stage_dev, dyn_dev, Xs, Xo, d_Y_,
+                                                 net_.params(), net_.hidden(), net_.pred(), P_, t_);
+        if (train) {
+            if (net_.learn_dev(Xo, d_Y_, P_, kLearningRate, kMomentum, out_dev_ + P_, out_dev_ + P_ + 1) != LT_OK)
+                return fail_net();
             trained_++;
             train_enqueued_ = true;
         }
         if (trained_ >= 4) {
-            if (net_.forward_dev(Xs, P_, d_pred_) != LT_OK) return fail_net();
-            pol_demand<<<blocks, 256, 0, st>>>(d_out_, d_out_ + P_ + 2, d_pred_, Xs, P_);
+            pol_forecast<<<blocks, kPolThreads, 0, st>>>(out_dev_, out_dev_ + P_ + 2, Xs, net_.params(), P_);
             pred_enqueued_ = true;
         }
-        pol_copy<<<(2 * P_ + 2 + 255) / 256, 256, 0, st>>>(out_dev_, d_out_, 2 * P_ + 2);
-        if (cudaEventRecord(ev_, st) != cudaSuccess || cudaEventRecord(stage_ev_[slot], st) != cudaSuccess)
-            return fail_net();
+        if (cudaGetLastError() != cudaSuccess || cudaEventRecord(pair_ev_[slot], st) != cudaSuccess) return fail_net();
         inflight_ = true;
+        inflight_slot_ = slot;
     }
 
     const char *name() const override { return use_net_ ? "learned" : "frequency"; }
@@ -618,13 +624,13 @@ private:
     double net_avg_ = 1e30, base_avg_ = 0.0;  // validation gate (running losses)
     bool ready_ = false, inflight_ = false, pred_enqueued_ = false, train_enqueued_ = false, failed_ = false;
     std::vector<std::pair<double, double>> losses_;  // (network, moving average) per training batch
-    cudaEvent_t ev_ = nullptr;
-    cudaEvent_t stage_ev_[kStage] = {};
+    cudaEvent_t pair_ev_[kPairs] = {};  // after the work of each staging slot
+    int inflight_slot_ = 0;
     HostBuf h_stage_, h_out_;
-    uint8_t *stage_dev_ = nullptr;
+    uint32_t *stage_dev_ = nullptr;
     float *out_dev_ = nullptr;
     uint32_t *d_ring_ = nullptr;
-    float *d_ema_ = nullptr, *d_stat_ = nullptr, *d_X_ = nullptr, *d_Y_ = nullptr, *d_out_ = nullptr, *d_pred_ = nullptr;
+    float *d_ema_ = nullptr, *d_stat_ = nullptr, *d_X_ = nullptr, *d_Y_ = nullptr;
     std::vector<uint64_t> snap_t_, static_mass_;
     std::vector<float> ema_, stat_;
     std::vector<double> demand_;

@@ -40,12 +40,16 @@ public:
     // parameter layout; applies SGD with momentum when lr > 0.
     lt_status train(const float *h_x, const float *h_y, uint32_t n, float lr, float momentum, float *h_loss,
                     float *h_grad, float *h_pred);
-    // Device-resident rows, enqueued on stream() without waiting: one SGD
-    // step on (d_x, d_y) writing the pre-step loss to d_loss, and a forward.
-    lt_status train_dev(const float *d_x, const float *d_y, uint32_t n, float lr, float momentum, float *d_loss);
-    lt_status forward_dev(const float *d_x, uint32_t n, float *d_pred);
+    // Enqueued on stream() without waiting: one SGD step on device-resident
+    // rows (d_x, d_y) whose hidden units and outputs the caller has written to
+    // hidden() and pred(); the loss before the step to *loss, the mean square of
+    // the targets to *base (device-visible).
+    lt_status learn_dev(const float *d_x, const float *d_y, uint32_t n, float lr, float momentum, float *loss,
+                        float *base);
+    const float *params() const { return d_params_; }
+    float *hidden() const { return d_h_; }
+    float *pred() const { return d_pred_; }
     cudaStream_t stream() const { return st_; }
-    lt_status record(cudaEvent_t ev);
 
 private:
     int device_ = 0;
