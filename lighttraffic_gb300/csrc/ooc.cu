@@ -67,8 +67,6 @@ lt_status dalloc(T **p, uint64_t count)
     return LT_OK;
 }
 
-enum TimerKind { kTGraph = 0, kTCompute = 1, kTZero = 2, kTBucket = 3 };
-
 // Host-link bytes per zero-copy hop: measured with ncu (sectors the
 // system-memory L2 filled from host memory) on the 2^33-edge graph, 0.244 of
 // the 256 bytes two 128-byte lines per hop would take -- hops grouped by
@@ -105,14 +103,17 @@ struct Ooc {
     uint64_t staging_cap = 0;
     uint32_t *d_out = nullptr;      // 5 arrays of staging_cap: cur, step, idx, dest, query
     lt_server *serve = nullptr;  // serving state when queries are being served
-    uint32_t *d_ctl = nullptr;      // hist[P] | visits[P] | pad | out_n | next | next2 (u64) | bucket_err (u32) | pad
+    // hist[P] | visits[P] | pad | out_n | next | next2 (u64) | bucket_err (u32) |
+    // pad | stats (8 u64) | kernel clocks (3 of 3 u64)
+    uint32_t *d_ctl = nullptr;
     uint64_t ctl_words = 0;         // u32 words of d_ctl
     uint32_t *d_planbuf = nullptr;  // cursor[P] | win_off[P] | plan chunks
     uint64_t plan_cap = 0;
     uint32_t *d_work = nullptr;
     uint64_t *d_work_off = nullptr;
     uint64_t work_cap = 0;
-    unsigned long long *d_stats = nullptr;
+    unsigned long long *d_stats = nullptr;   // in d_ctl, the clocks behind it
+    unsigned long long clk_seen[kClocks] = {};  // nanoseconds already in the engine's statistics
 
     HostBuf h_ctl;   // pinned mirror of d_ctl, and its device view
     uint32_t *h_ctl_dev = nullptr;
@@ -191,11 +192,15 @@ struct Ooc {
     int grid[3] = {0, 0, 0};
 
     std::vector<cudaEvent_t> ev_free;
+    // loads started between two passes, back to back on the copy stream: one
+    // span from the first's start to the last's end (load_a, load_b while open)
     struct Timed {
-        cudaEvent_t a, b;
-        int kind;
+        cudaEvent_t a;
+        std::vector<cudaEvent_t> b;
     };
     std::vector<Timed> timed;
+    cudaEvent_t load_a = nullptr;
+    std::vector<cudaEvent_t> load_b;
 
     uint8_t *host_chunk(uint32_t id)
     {
@@ -211,6 +216,8 @@ struct Ooc {
     uint32_t bucket_err_word() const { return hist_words() + 6; }
     uint32_t *ctl_bucket_err() { return d_ctl + bucket_err_word(); }
     uint32_t cleared_words() const { return hist_words() + 6; }
+    uint32_t stats_word() const { return hist_words() + 8; }
+    unsigned long long *clock(int k) { return d_stats + 8 + 3 * k; }
 };
 
 namespace {
@@ -227,37 +234,60 @@ cudaEvent_t ev_get(Ooc &o)
     return ev;
 }
 
-// Resolve the event timers of finished work into the phase timers.
+// Ends the open group of loads.  Groups are timed, not loads: a start event of
+// its own for each of the 220 loads of a burst of served queries made 4.7 ms 5.6.
+void close_loads(Ooc &o)
+{
+    if (!o.load_a) return;
+    if (o.load_b.empty())
+        o.ev_free.push_back(o.load_a);
+    else
+        o.timed.push_back({o.load_a, std::move(o.load_b)});
+    o.load_a = nullptr;
+    o.load_b.clear();
+}
+
+// Resolves the event timers of finished loads into the phase timer.
 void drain_timers(Ooc &o, bool all)
 {
     lt_engine &e = *o.e;
-    // every iteration records a few timers: read them in batches (each read
-    // is a few driver calls), and all of them at the end of a run
-    if (!all && o.timed.size() < 48) return;
+    // read in batches (each read is a few driver calls), and all of them at
+    // the end of a run
+    if (!all && o.timed.size() < 16) return;
+    if (all) close_loads(o);
     size_t keep = 0;
     for (size_t i = 0; i < o.timed.size(); i++) {
         Ooc::Timed &t = o.timed[i];
-        if (!all && cudaEventQuery(t.b) != cudaSuccess) {
+        if (!all && cudaEventQuery(t.b.back()) != cudaSuccess) {
             cudaGetLastError();
-            o.timed[keep++] = t;
+            if (keep != i) o.timed[keep] = std::move(t);
+            keep++;
             continue;
         }
         float ms = 0;
-        cudaEventSynchronize(t.b);
-        cudaEventElapsedTime(&ms, t.a, t.b);
-        if (t.kind == kTGraph)
-            e.stats.graph_loading_ms += ms;
-        else if (t.kind == kTCompute)
-            e.stats.computing_ms += ms;
-        else if (t.kind == kTZero)
-            e.stats.zerocopy_ms += ms;
-        else
-            e.stats.bucket_ms += ms;
-        if (t.kind == kTCompute || t.kind == kTZero) e.stats.step_kernel_ms += ms;
+        cudaEventSynchronize(t.b.back());
+        if (cudaEventElapsedTime(&ms, t.a, t.b.back()) == cudaSuccess) e.stats.graph_loading_ms += ms;
         o.ev_free.push_back(t.a);
-        o.ev_free.push_back(t.b);
+        o.ev_free.insert(o.ev_free.end(), t.b.begin(), t.b.end());
     }
     o.timed.resize(keep);
+}
+
+// Adds what the kernels' clocks (a copy of d_stats and the clocks behind it)
+// show beyond what the statistics already hold.
+void clock_stats(Ooc &o, const unsigned long long *stats)
+{
+    lt_stats &st = o.e->stats;
+    double *to[kClocks] = {&st.computing_ms, &st.zerocopy_ms, &st.bucket_ms};
+    for (int k = 0; k < kClocks; k++) {
+        const unsigned long long *c = stats + 8 + 3 * k;
+        const unsigned long long ns = c[2] + (c[1] > c[0] ? c[1] - c[0] : 0);
+        if (ns <= o.clk_seen[k]) continue;
+        const double ms = 1e-6 * (double)(ns - o.clk_seen[k]);
+        o.clk_seen[k] = ns;
+        *to[k] += ms;
+        if (k != kClockBucket) st.step_kernel_ms += ms;
+    }
 }
 
 // Bytes a load of partition p copies (and its host footprint): the col
@@ -299,10 +329,12 @@ __global__ void upload_kernel(uint32_t *dst, const uint32_t *src, uint64_t n)
 }
 
 // What precedes a pass's step kernels, in one launch: table updates, the work
-// list and its offsets from mapped pinned memory, the control block cleared.
+// list and its offsets from mapped pinned memory, the control block cleared,
+// the last pass's spans added to the kernel clocks' totals.
 __global__ void pass_begin_kernel(unsigned long long *rp, unsigned long long *col, const __grid_constant__ EntryBatch e,
                                   uint32_t *work, const uint32_t *h_work, uint64_t n_work, uint32_t *off,
-                                  const uint32_t *h_off, uint64_t n_off, uint32_t *ctl, uint32_t n_ctl)
+                                  const uint32_t *h_off, uint64_t n_off, uint32_t *ctl, uint32_t n_ctl,
+                                  unsigned long long *clk)
 {
     const uint64_t first = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (uint64_t)gridDim.x * blockDim.x;
     if (first < e.n) {
@@ -312,6 +344,11 @@ __global__ void pass_begin_kernel(unsigned long long *rp, unsigned long long *co
     for (uint64_t i = first; i < n_ctl; i += stride) ctl[i] = 0;
     for (uint64_t i = first; i < n_work; i += stride) work[i] = h_work[i];
     for (uint64_t i = first; i < n_off; i += stride) off[i] = h_off[i];
+    if (n_ctl && first < kClocks) {
+        unsigned long long *c = clk + 3 * first;
+        if (c[1] > c[0]) c[2] += c[1] - c[0];
+        c[0] = c[1] = 0;
+    }
 }
 
 // Launches pass_begin_kernel (several where there are many table updates);
@@ -341,7 +378,7 @@ lt_status pass_begin(Ooc &o, const uint32_t *h_work, uint64_t n_work, const uint
         const uint64_t blocks = std::max<uint64_t>(1, std::min<uint64_t>((words + 255) / 256, 304));
         pass_begin_kernel<<<(unsigned)blocks, 256, 0, e.s_compute>>>(
             o.d_rp, o.d_col, b, o.d_work, n_work ? view(h_work) : nullptr, n_work, (uint32_t *)o.d_work_off,
-            n_off ? view(h_woff) : nullptr, n_off, o.d_ctl, n_ctl);
+            n_off ? view(h_woff) : nullptr, n_off, o.d_ctl, n_ctl, o.d_stats + 8);
         LT_CUDA_TRY(cudaGetLastError());
         e.stats.kernel_launches++;
         n_work = n_off = 0;
@@ -610,27 +647,29 @@ lt_status start_load(Ooc &o, uint32_t p, int32_t slot, std::vector<std::pair<uin
         o.ev_free.push_back(free_ev);
         o.copy_waits = true;
     }
-
+    if (!o.load_a) {
+        o.load_a = ev_get(o);
+        LT_CUDA_TRY(cudaEventRecord(o.load_a, e.s_copy));
+    }
     const uint64_t n0 = g.node_off[p], n1 = g.node_off[p + 1];
     const uint64_t e0 = g.edge_off[p], e1 = g.edge_off[p + 1];
     uint8_t *base = o.d_slots + (uint64_t)slot * o.slot_stride;
     const uint64_t rp_bytes = o.d_index ? 0 : 8 * (n1 - n0 + 1);
     const uint64_t col_off = (rp_bytes + 15) & ~15ull;
-    Ooc::Timed t{ev_get(o), ev_get(o), kTGraph};
-    LT_CUDA_TRY(cudaEventRecord(t.a, e.s_copy));
     if (rp_bytes) LT_CUDA_TRY(cudaMemcpyAsync(base, g.rowptr() + n0, rp_bytes, cudaMemcpyHostToDevice, e.s_copy));
     if (e1 > e0) LT_CUDA_TRY(cudaMemcpyAsync(base + col_off, g.col() + e0, 4 * (e1 - e0), cudaMemcpyHostToDevice, e.s_copy));
-    LT_CUDA_TRY(cudaEventRecord(t.b, e.s_copy));
-    o.timed.push_back(t);
+    const cudaEvent_t copied = ev_get(o);
+    o.load_b.push_back(copied);
+    LT_CUDA_TRY(cudaEventRecord(copied, e.s_copy));
     o.h_rp[p] = (unsigned long long)(uintptr_t)(o.d_index ? (uint8_t *)(o.d_index + n0) : base);
     o.h_col[p] = (unsigned long long)(uintptr_t)(base + col_off);
     o.loaded_at[p] = o.iteration;
     o.slot_of[p] = slot;
     o.part_in_slot[slot] = (int32_t)p;
     if (deferred) {
-        deferred->push_back({p, t.b});
+        deferred->push_back({p, copied});
     } else {
-        LT_CUDA_TRY(cudaStreamWaitEvent(e.s_compute, t.b, 0));
+        LT_CUDA_TRY(cudaStreamWaitEvent(e.s_compute, copied, 0));
         set_entry(o, p);
     }
     e.stats.graph_loading_calls++;
@@ -872,6 +911,7 @@ lt_status step_and_bucket_parts(Ooc &o, const RunParams &rp, const std::vector<u
     lt_graph &g = *o.g;
     const double t_submit = now_ms();
     o.copy_waits = false;
+    close_loads(o);
     Queue *qp = p >= 0 ? &o.q[p] : nullptr;
     uint64_t n_chunk_walkers = 0, nw = 0;
     for (uint32_t x : parts) {
@@ -1045,29 +1085,23 @@ lt_status step_and_bucket_parts(Ooc &o, const RunParams &rp, const std::vector<u
         a.lazy_count = 0;
         LT_CUDA_TRY(cudaEventRecord(o.ev_pre, e.s_compute));
         LT_CUDA_TRY(cudaStreamWaitEvent(o.s_aux, o.ev_pre, 0));
-        Ooc::Timed tc{ev_get(o), ev_get(o), kTCompute};
+        c.clk = o.clock(kClockCached);
         nvtxRangePushA("cached_step");
-        LT_CUDA_TRY(cudaEventRecord(tc.a, o.s_aux));
         const cudaError_t lc = launch_walk_part(c, rp.app, e.sms, o.s_aux);
         nvtxRangePop();
         LT_CUDA_TRY(lc);
-        LT_CUDA_TRY(cudaEventRecord(tc.b, o.s_aux));
         LT_CUDA_TRY(cudaEventRecord(o.ev_aux, o.s_aux));
-        o.timed.push_back(tc);
         e.stats.computing_calls++;
         e.stats.kernel_launches++;
         e.stats.split_launches++;
         grid = std::min(grid - e.sms, kZcSplitCtas * e.sms);
     }
-    Ooc::Timed t{ev_get(o), ev_get(o), zc_launch ? kTZero : kTCompute};
+    a.clk = o.clock(zc_launch ? kClockZero : kClockCached);
     // NVTX ranges name the launch kind for profilers (ncu --nvtx-include)
     nvtxRangePushA(zc_launch ? "zero_copy_step" : "cached_step");
-    LT_CUDA_TRY(cudaEventRecord(t.a, e.s_compute));
     const cudaError_t launched = launch_walk_part(a, rp.app, grid, e.s_compute);
     nvtxRangePop();
     LT_CUDA_TRY(launched);
-    LT_CUDA_TRY(cudaEventRecord(t.b, e.s_compute));
-    o.timed.push_back(t);
     if (split) LT_CUDA_TRY(cudaStreamWaitEvent(e.s_compute, o.ev_aux, 0));
     if (zc_launch)
         e.stats.zerocopy_calls++;
@@ -1100,16 +1134,13 @@ lt_status step_and_bucket_parts(Ooc &o, const RunParams &rp, const std::vector<u
         sa.P = o.P;
         sa.items = e.cfg.bucket_items;
         sa.err = o.ctl_bucket_err();
-        Ooc::Timed tb{ev_get(o), ev_get(o), kTBucket};
-        LT_CUDA_TRY(cudaEventRecord(tb.a, e.s_compute));
+        sa.clk = pa.clk = o.clock(kClockBucket);
         nvtxRangePushA("bucketing");
         cudaError_t bucketed = launch_plan(pa, e.s_compute);
         if (bucketed == cudaSuccess) bucketed = cudaEventRecord(o.ev_ctl, e.s_compute);
         if (bucketed == cudaSuccess) bucketed = launch_scatter(sa, e.device, e.s_compute);
         nvtxRangePop();
         LT_CUDA_TRY(bucketed);
-        LT_CUDA_TRY(cudaEventRecord(tb.b, e.s_compute));
-        o.timed.push_back(tb);
         e.stats.kernel_launches += 2;
         e.stats.device_plans++;
         e.stats.host_submit_ms += now_ms() - t_submit;
@@ -1138,6 +1169,7 @@ lt_status step_and_bucket_parts(Ooc &o, const RunParams &rp, const std::vector<u
     const uint32_t bucket_err = h_hist[o.bucket_err_word()];
     if (bucket_err & 2u) return fail(LT_ERR_CAPACITY, "bucketing: the device plan ran out of free chunks");
     if (bucket_err & 1u) return fail(LT_ERR_TIMEOUT, "bucketing: a bulk copy into shared memory did not complete");
+    clock_stats(o, (const unsigned long long *)(h_hist + o.stats_word()));
     const uint64_t staged = *(const unsigned long long *)(h_hist + o.hist_words());
     if (!dev_plan) {
         // the drained queues' chunks return to the pool
@@ -1206,14 +1238,11 @@ lt_status step_and_bucket_parts(Ooc &o, const RunParams &rp, const std::vector<u
     sa.P = o.P;
     sa.items = e.cfg.bucket_items;
     sa.err = o.ctl_bucket_err();
-    Ooc::Timed tb{ev_get(o), ev_get(o), kTBucket};
-    LT_CUDA_TRY(cudaEventRecord(tb.a, e.s_compute));
+    sa.clk = o.clock(kClockBucket);
     nvtxRangePushA("bucketing");
     const cudaError_t bucketed = launch_scatter(sa, e.device, e.s_compute);
     nvtxRangePop();
     LT_CUDA_TRY(bucketed);
-    LT_CUDA_TRY(cudaEventRecord(tb.b, e.s_compute));
-    o.timed.push_back(tb);
     e.stats.kernel_launches++;
     return LT_OK;
 }
@@ -1829,7 +1858,7 @@ lt_status ooc_create(lt_engine *e, Ooc **out)
     o->P = g.P();
     o->K = std::min<uint32_t>(e->cfg.num_device_partitions, o->P);
     if (o->K < 1) o->K = 1;
-    o->ctl_words = o->hist_words() + 8;
+    o->ctl_words = o->stats_word() + 2 * kStatWords;
     auto bail = [&](lt_status s) {
         ooc_destroy(o);
         return s;
@@ -1893,7 +1922,7 @@ lt_status ooc_create(lt_engine *e, Ooc **out)
     if (s == LT_OK) s = dalloc(&o->d_rp, o->P);
     if (s == LT_OK) s = dalloc(&o->d_col, o->P);
     if (s == LT_OK) s = dalloc(&o->d_ctl, o->ctl_words);
-    if (s == LT_OK) s = dalloc(&o->d_stats, 8);
+    if (s == LT_OK) o->d_stats = (unsigned long long *)(o->d_ctl + o->stats_word());
     if (s == LT_OK) s = host_alloc(o->h_ctl, 4 * o->ctl_words, true);
     if (s == LT_OK) o->h_ctl_dev = (uint32_t *)mapped_host(o->h_ctl.ptr, 4 * o->ctl_words);
     if (s == LT_OK && (cudaStreamCreateWithFlags(&o->s_aux, cudaStreamNonBlocking) != cudaSuccess ||
@@ -1973,7 +2002,7 @@ void ooc_destroy(Ooc *o)
     drain_timers(*o, true);
     for (void *p : {(void *)o->d_index, (void *)o->d_slots, (void *)o->d_node_off, (void *)o->d_edge_off, (void *)o->d_map, (void *)o->d_rp, (void *)o->d_col,
                     (void *)o->d_arena, (void *)o->d_out, (void *)o->d_ctl, (void *)o->d_planbuf, (void *)o->d_work,
-                    (void *)o->d_work_off, (void *)o->d_stats})
+                    (void *)o->d_work_off})
         if (p) cudaFree(p);
     for (HostBuf &b : o->host_slabs) host_free(b);
     host_free(o->h_ctl);
@@ -2530,14 +2559,17 @@ lt_status run_all(lt_engine *e, RunParams &rp, uint32_t runs, uint32_t run_base,
         bool stop = false;
         LT_TRY(run_loop(o, rp, stop));
         if (stop) {
+            unsigned long long hs[kStatWords];
+            LT_CUDA_TRY(cudaMemcpyAsync(hs, o.d_stats, sizeof hs, cudaMemcpyDeviceToHost, st));
             LT_CUDA_TRY(cudaStreamSynchronize(st));
             LT_CUDA_TRY(cudaStreamSynchronize(e->s_copy));
             drain_timers(o, true);
+            clock_stats(o, hs);
             return fail(LT_INTERRUPTED, "run stopped at the checkpoint %s (iteration %llu)", o.ckpt_path.c_str(),
                         (unsigned long long)o.iteration);
         }
     }
-    unsigned long long hs[8];
+    unsigned long long hs[kStatWords];
     LT_CUDA_TRY(cudaMemcpyAsync(hs, o.d_stats, sizeof hs, cudaMemcpyDeviceToHost, st));
     if (counts_out && rp.counts) LT_CUDA_TRY(cudaMemcpyAsync(counts_out, rp.counts, 8ull * g.V, cudaMemcpyDeviceToHost, st));
     if (endpoints_out && rp.endpoints)
@@ -2547,6 +2579,7 @@ lt_status run_all(lt_engine *e, RunParams &rp, uint32_t runs, uint32_t run_base,
     LT_CUDA_TRY(cudaStreamSynchronize(st));
     LT_CUDA_TRY(cudaStreamSynchronize(e->s_copy));
     drain_timers(o, true);
+    clock_stats(o, hs);
     e->stats.updates = hs[0];
     e->stats.moves = hs[1];
     e->stats.teleports = hs[2];
@@ -3180,8 +3213,9 @@ void serve_close(lt_server *s)
     if (!s) return;
     if (s->o && s->o->serve == s) {
         cudaStreamSynchronize(s->e->s_compute);
-        unsigned long long hs[8];
+        unsigned long long hs[kStatWords];
         if (cudaMemcpy(hs, s->o->d_stats, sizeof hs, cudaMemcpyDeviceToHost) == cudaSuccess) {
+            clock_stats(*s->o, hs);
             s->e->stats.updates = hs[0];
             s->e->stats.moves = hs[1];
             s->e->stats.teleports = hs[2];

@@ -163,6 +163,7 @@ __global__ void __launch_bounds__(kPartBlock, part_min_blocks<APP>()) walk_part_
 {
     extern __shared__ __align__(16) uint32_t smem[];
     __shared__ PartWarp<APP == kPPR && !SERVE, SERVE> s_warp[kPartBlock / 32];
+    if (blockIdx.x == 0 && threadIdx.x == 0) a.clk[0] = globaltimer_ns();
     const uint32_t P = a.t.P;
     const bool in_smem = P <= kSmemPartMax;
     const bool col_table = RP32 && P <= kColTableMax;
@@ -565,6 +566,7 @@ __global__ void __launch_bounds__(kPartBlock, part_min_blocks<APP>()) walk_part_
         if (s_stats[2]) atomicAdd(&a.stats[3], s_stats[2]);
         if (s_stats[3]) atomicAdd(&a.stats[4], s_stats[3]);
         if (fin) atomicAdd(&a.stats[5], fin);
+        atomicMax(&a.clk[1], (unsigned long long)globaltimer_ns());
     }
     if (in_smem)
         for (uint32_t i = threadIdx.x; i < P; i += kPartBlock) {
@@ -578,6 +580,7 @@ constexpr int kScatterItems = 4;
 
 __global__ void __launch_bounds__(kPartBlock) scatter_kernel(ScatterArgs a)
 {
+    if (blockIdx.x == 0 && threadIdx.x == 0 && !a.n_dev) a.clk[0] = globaltimer_ns();
     extern __shared__ uint32_t smem[];
     const uint32_t P = a.P;
     const bool in_smem = P <= kSmemPartMax;
@@ -622,6 +625,7 @@ __global__ void __launch_bounds__(kPartBlock) scatter_kernel(ScatterArgs a)
         }
         if (in_smem) __syncthreads();
     }
+    if (threadIdx.x == 0) atomicMax(&a.clk[1], (unsigned long long)globaltimer_ns());
 }
 
 // Bucketing by a block-local counting sort (P <= kSmemPartMax).  A tile of
@@ -674,6 +678,7 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) bucket_sort_kernel(Scatte
     uint32_t *s_ch0 = s_base + P;                              // P: chunk holding s_base
     uint32_t *s_ch1 = s_ch0 + P;                               // P: the next chunk, where the run crosses into it
     uint16_t *s_inv = reinterpret_cast<uint16_t *>(s_ch1 + P); // T: tile position at sorted position j
+    if (blockIdx.x == 0 && threadIdx.x == 0 && !a.n_dev) a.clk[0] = globaltimer_ns();
     const uint32_t *src[kBucketFields] = {a.in_cur, a.in_step, a.in_idx, a.in_q, a.in_dest};
     if (a.err && (*(volatile unsigned int *)a.err & 2u)) return;
     const uint64_t n = a.n_dev ? *a.n_dev : a.n;
@@ -803,6 +808,7 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) bucket_sort_kernel(Scatte
     // (bounded) before this CTA's shared memory is released
     while (waited0 < issued0 && mbar_wait_bounded(&mbar[0], waited0 & 1, kBulkWaitNs)) waited0++;
     while (waited1 < issued1 && mbar_wait_bounded(&mbar[1], waited1 & 1, kBulkWaitNs)) waited1++;
+    if (threadIdx.x == 0) atomicMax(&a.clk[1], (unsigned long long)globaltimer_ns());
 }
 
 // One CTA plans every destination: per destination the chunks its arrivals
@@ -815,6 +821,7 @@ __global__ void __launch_bounds__(kPlanBlock) plan_kernel(PlanArgs a)
     constexpr uint32_t kPerMax = kSmemPartMax / kPlanBlock;
     __shared__ uint32_t warp_tot[kPlanBlock / 32];
     __shared__ uint32_t tot_new, tot_slots;
+    if (threadIdx.x == 0) a.clk[0] = globaltimer_ns();
     const uint32_t P = a.P;
     const uint32_t per = (P + kPlanBlock - 1) / kPlanBlock;
     for (uint32_t i = threadIdx.x; i < a.ctl_words; i += kPlanBlock) a.ctl_host[i] = a.ctl[i];
