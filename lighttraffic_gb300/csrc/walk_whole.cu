@@ -389,12 +389,28 @@ __global__ void __launch_bounds__(kWholeBlock, 8) walk_whole_kernel(const __grid
     if (tel) atomicAdd((unsigned long long *)&a.stats[2], tel);
 }
 
+// CTAs of a launch with W walkers, at most: no more than have walkers, but one
+// per SM.  PPR walks differ in length, so that a lane's second and third walker
+// fill the time its warp would wait for its longest one: six walkers per lane
+// (whole CTAs per SM, two at least, for the latencies of a graph in DRAM).  One
+// walker per lane -> this, device arrays, p = 0.15: 150 000 walks on RMAT 2^16 /
+// 7e5 59 -> 53 us, 300 000 86 -> 65, on 2^20 / 2^24 96 -> 84, on 2^22 / 2^26
+// 106 -> 106; 600 000 105 -> 88, 114 -> 96, 128 -> 121; 1.2 million 126 -> 128,
+// 140 -> 133, 171 -> 170.  Three walkers per lane 600 000 95, 103, 125; eight 88,
+// 112, 128; one CTA per SM 150 000 on 2^22 / 2^26 101, two 95.
+template <int APP>
+uint64_t most_ctas(uint64_t W, int sms)
+{
+    const uint64_t full = std::max<uint64_t>(sms, (W + kWholeBlock - 1) / kWholeBlock);
+    if (APP != kPPR) return full;
+    const uint64_t six = sms * ((W - 1) / (6ull * sms * kWholeBlock) + 1);
+    return std::min(full, std::max<uint64_t>(2ull * sms, six));
+}
+
 template <int APP, int START, int C>
 cudaError_t launch_t(const WholeArgs &a, int grid, cudaStream_t st)
 {
-    // no more CTAs than have walkers, but one per SM
-    const uint64_t need = std::max<uint64_t>(a.sms, (a.W + kWholeBlock - 1) / kWholeBlock);
-    if ((uint64_t)grid > need) grid = (int)need;
+    grid = (int)std::min<uint64_t>((uint64_t)grid, most_ctas<APP>(a.W, a.sms));
     WholeArgs b = a;
     b.pool = pool_walkers(a.W, (uint64_t)grid * (kWholeBlock / 32));
     if constexpr (APP == kWalk) {

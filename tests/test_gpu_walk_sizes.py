@@ -96,3 +96,14 @@ def test_pagerank_shared_counters(lt, require_gpu, degree, layout):
         lt.check(lt.lib.lt_walk_device(1, 1, d_rp.data_ptr(), d_col.data_ptr(), *args, counts.data_ptr(), None, None, *tail))
     assert (counts.cpu().numpy().astype(np.uint64) == want).all()
     assert stats.tolist() == [int(x) for x in st]
+
+
+@pytest.mark.parametrize("walkers", [77824, 77825, 466944, 466945, 700417])  # edges of 2 and 3 CTAs per SM
+@pytest.mark.parametrize("prob", [0.5, 0.15])
+def test_ppr_ctas(lt, require_gpu, graph, walkers, prob):
+    rp, col = graph
+    e = lt.Engine(lt.Graph.from_csr(rp, col, 1 << 30), seed=55)
+    want, _, st = oracle.ppr(rp, col, 3, walkers, prob=prob, seed=55)
+    assert (e.ppr(3, walkers, prob) == want).all()
+    s = e.stats()
+    assert (s["updates"], s["moves"], s["teleports"]) == tuple(int(x) for x in st)
