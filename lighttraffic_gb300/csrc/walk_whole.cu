@@ -94,14 +94,18 @@ __device__ __forceinline__ void count1(const WholeArgs &a, uint32_t v, const Hin
 // Hub counters of PageRank.  Counter updates crowd the few lines that hold the
 // hubs' counters (RMAT 2^23 / 2^27: 1 % of 92 M updates go to one line), and
 // the L2 slice of such a line, at 105 % of its tag rate against 64 % on
-// average, set the kernel's time.  A CTA therefore counts up to 512 vertices
-// of at least E / 2^13 out-edges in shared memory and adds them up once at its
+// average, set the kernel's time.  A CTA therefore counts up to 4096 vertices
+// of at least E / 2^15 out-edges in shared memory and adds them up once at its
 // end; a vertex takes its slot at its first visit whose row is read (the first
-// to come keeps it: a hub is likely to be that).  PageRank on RMAT 2^23 / 2^27:
-// 1759 -> 1557 us, u64 on RMAT 2^21 / 4e7: 228 -> 201; 1024 slots from E / 2^14
-// 1561, 128 slots from E / 2^12 1559; serving the hubs' rows from shared
-// memory as well gave nothing.
-constexpr int kHotBits = 9;
+// to come keeps it: a hub is likely to be that).  The CTAs are as large as they
+// can be: each adds up its own table, which for a short launch on a small graph
+// is as much traffic as the updates it spares.  No tables -> 512 slots (from
+// E / 2^13) and 256 threads -> this: 10 steps from 3 million vertices drawn on
+// RMAT 2^16 / 7e5 - -> 515 -> 274 us, on 2^18 / 2^22 - -> 369 -> 289, on 2^20 /
+// 2^24 - -> 376 -> 306; RMAT 2^23 / 2^27 1759 -> 1557 -> 1561, u64 on RMAT 2^21 /
+// 4e7 228 -> 201 -> 190.  512 slots and 1024 threads on 2^16 495, 1024 slots 348,
+// 2048 293; serving the hubs' rows from shared memory as well gave nothing.
+constexpr int kHotBits = 12;
 constexpr uint32_t kHotSlots = 1u << kHotBits;
 constexpr uint32_t kHotMinDegree = 64;
 constexpr uint32_t kNoVertex = 0xFFFFFFFFu;
@@ -110,7 +114,7 @@ template <int L>
 __device__ __forceinline__ uint32_t hot_degree(const WholeArgs &a)
 {
     const uint64_t E = L == kLayoutPacked ? a.rows[2ull * a.V] : L == kLayoutCompact ? a.rowptr32[a.V] : a.rowptr[a.V];
-    return (uint32_t)min(0xFFFFFFFFull, max((unsigned long long)kHotMinDegree, (unsigned long long)E >> 13));
+    return (uint32_t)min(0xFFFFFFFFull, max((unsigned long long)kHotMinDegree, (unsigned long long)E >> 15));
 }
 
 template <int START>
@@ -182,9 +186,13 @@ __device__ __forceinline__ void path_flush(PathSegment &p, bool due)
     }
 }
 
+// Threads of a CTA (2048 per SM either way): PageRank's share the hub counters.
+template <int APP>
+constexpr int block_of = APP == kPageRank ? 1024 : kWholeBlock;
+
 // GATHER: paths go through shared memory (kWalk only).
 template <int APP, int START, int C, bool GATHER>
-__global__ void __launch_bounds__(kWholeBlock, 8) walk_whole_kernel(const __grid_constant__ WholeArgs a)
+__global__ void __launch_bounds__(block_of<APP>, 2048 / block_of<APP>) walk_whole_kernel(const __grid_constant__ WholeArgs a)
 {
     const int lane = threadIdx.x & 31;
     const Hints h{l2_policy_evict_last(), l2_policy_evict_first()};
@@ -197,7 +205,7 @@ __global__ void __launch_bounds__(kWholeBlock, 8) walk_whole_kernel(const __grid
     // the first walkers are dealt out without the counter, 32 (PPR: a pool) to
     // each warp, the warps of the same number in their CTAs before the next
     // ones, so that few walkers spread over all SMs
-    const uint64_t dealt = (uint64_t)gridDim.x * (APP == kPPR ? kWholeBlock / 32 * a.pool : kWholeBlock);
+    const uint64_t dealt = (uint64_t)gridDim.x * (APP == kPPR ? kWholeBlock / 32 * a.pool : block_of<APP>);
     bool first_deal = true;
     // PPR: the warp's pool of walkers with their lengths drawn
     __shared__ PprPool pools[APP == kPPR ? kWholeBlock / 32 : 1];
@@ -210,8 +218,8 @@ __global__ void __launch_bounds__(kWholeBlock, 8) walk_whole_kernel(const __grid
     __shared__ uint32_t hot_v[kHot ? kHotSlots : 1], hot_n[kHot ? kHotSlots : 1];
     uint32_t hot_min = 0;
     if (kHot) {
-        for (uint32_t i = threadIdx.x; i < kHotSlots; i += kWholeBlock) {
-            hot_v[i] = kNoVertex;
+        for (uint32_t i = threadIdx.x; i < kHotSlots; i += block_of<APP>) {
+            hot_v[i] = a.hot ? kNoVertex : kNoVertex - 1u;  // free, or taken
             hot_n[i] = 0;
         }
         hot_min = hot_degree<C>(a);
@@ -356,7 +364,7 @@ __global__ void __launch_bounds__(kWholeBlock, 8) walk_whole_kernel(const __grid
     // walk one per hop and one where it ends early.
     if (kHot) {
         __syncthreads();
-        for (uint32_t i = threadIdx.x; i < kHotSlots; i += kWholeBlock)
+        for (uint32_t i = threadIdx.x; i < kHotSlots; i += block_of<APP>)
             if (hot_n[i]) count_n<C>(a, hot_v[i], hot_n[i], h);
     }
     if (!a.stats) return;
@@ -401,7 +409,7 @@ __global__ void __launch_bounds__(kWholeBlock, 8) walk_whole_kernel(const __grid
 template <int APP>
 uint64_t most_ctas(uint64_t W, int sms)
 {
-    const uint64_t full = std::max<uint64_t>(sms, (W + kWholeBlock - 1) / kWholeBlock);
+    const uint64_t full = std::max<uint64_t>(sms, (W + block_of<APP> - 1) / block_of<APP>);
     if (APP != kPPR) return full;
     const uint64_t six = sms * ((W - 1) / (6ull * sms * kWholeBlock) + 1);
     return std::min(full, std::max<uint64_t>(2ull * sms, six));
@@ -412,6 +420,8 @@ cudaError_t launch_t(const WholeArgs &a, int grid, cudaStream_t st)
 {
     grid = (int)std::min<uint64_t>((uint64_t)grid, most_ctas<APP>(a.W, a.sms));
     WholeArgs b = a;
+    // a CTA's counters have 32 bits: 19 times its share of these updates
+    b.hot = a.length == 0 || a.W < (1ull << 36) / a.length;
     b.pool = pool_walkers(a.W, (uint64_t)grid * (kWholeBlock / 32));
     if constexpr (APP == kWalk) {
         if (a.paths && a.length >= kPathGatherMin && a.W > 2ull * a.sms * kWholeBlock * 8) {
@@ -419,7 +429,7 @@ cudaError_t launch_t(const WholeArgs &a, int grid, cudaStream_t st)
             return cudaGetLastError();
         }
     }
-    walk_whole_kernel<APP, START, C, false><<<grid, kWholeBlock, 0, st>>>(b);
+    walk_whole_kernel<APP, START, C, false><<<grid, block_of<APP>, 0, st>>>(b);
     return cudaGetLastError();
 }
 
@@ -437,7 +447,7 @@ template <int APP, int START, int C>
 int occupancy_t()
 {
     int n = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, walk_whole_kernel<APP, START, C, false>, kWholeBlock, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, walk_whole_kernel<APP, START, C, false>, block_of<APP>, 0);
     return n;
 }
 

@@ -38,6 +38,7 @@ struct WholeArgs {
     Limit53 lim;             // of floor(p 2^53): PPR stop prob or PageRank alpha
     ModN by_v;               // remainders by V
     uint32_t pool;           // PPR: walkers a warp draws lengths for at a time (set by the launcher)
+    int hot;                       // PageRank: CTAs count hubs in shared memory; set by the launcher
     uint32_t long_len;       // PPR: walks longer than this begin first in their pool
 };
 
