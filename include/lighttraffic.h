@@ -116,7 +116,7 @@ typedef struct lt_engine_cfg {
     uint32_t load_factor;            /* wave runs: a partition is loaded once its waiting walkers reach
                                         load_factor x zerocopy_threshold (0 = 256 / host bytes per
                                         zero-copy hop: 8 with the device index, 4 without) */
-    int bucket_items;                /* bucketing tile: 16 (0) = 4096 walkers, 8 = 2048 */
+    int bucket_items;                /* bucketing tile: 16 (0) = up to 8192 walkers, 8 = 2048 */
     int no_prefill;                  /* wave runs: 1 = leave a cold cache to fill as walkers arrive
                                         instead of loading the policy's forecast set at a run's start */
     int hot_tier;                    /* wave runs with the device index: percent (0 = off, at most 90) of

@@ -629,7 +629,7 @@ __global__ void __launch_bounds__(kPartBlock) scatter_kernel(ScatterArgs a)
 }
 
 // Bucketing by a block-local counting sort (P <= kSmemPartMax).  A tile of
-// T = BLOCK x ITEMS staged walkers is ranked per destination in shared
+// T = BLOCK x items staged walkers is ranked per destination in shared
 // memory (shared atomics), the per-destination counts are scanned across the
 // block and reserved in the destination windows with one global atomic per
 // (tile, destination) -- the two-level scheme of insertToQueueKernel
@@ -637,42 +637,45 @@ __global__ void __launch_bounds__(kPartBlock) scatter_kernel(ScatterArgs a)
 // sort permutation as per-destination runs: consecutive threads write
 // consecutive queue slots.
 //
-// The CTAs are persistent and double-buffered: while a tile is sorted, the
-// bulk-copy unit (cp.async.bulk, one copy per field, completion counted on an
-// mbarrier) brings the CTA's next tile from the staging area into shared
-// memory, so the kernel issues no global loads of walker fields.  A tile's
-// chunk ids are looked up once per destination, not per walker.  The staged
-// field arrays start 16-byte aligned and hold n rounded up to 4 words (the
-// copies round up to 16 bytes).  If a copy does not complete within a second,
-// the CTA records it in *err and reads the remaining tiles from global memory
-// directly, so no walker is lost.
-// Two shapes, chosen by the autotuner: 1024 threads x 4 walkers (T = 4096,
-// the default; one CTA per SM) and 512 threads x 4 walkers (T = 2048; two
-// CTAs per SM, so that one CTA's barrier waits overlap the other's work; on
-// c2 its bucketing took 145 ms per run against 97).  Every phase of a tile
-// ends at a block barrier; 256-thread CTAs of a 4096-walker tile left 8
-// warps per SM to hide the latencies (c2s launch: 46 against 38 us).
+// The CTAs are persistent.  The bulk-copy unit (cp.async.bulk, one copy per
+// field, completion counted on an mbarrier) brings a tile from the staging area
+// into shared memory, so the kernel issues no global loads of walker fields.  A
+// tile's chunk ids are looked up once per destination, not per walker.  The
+// staged field arrays start 16-byte aligned and hold n rounded up to 4 words
+// (the copies round up to 16 bytes).  If a copy does not complete within a
+// second, the CTA records it in *err and reads the remaining tiles from global
+// memory directly, so no walker is lost.
+// What bounds it is the runs, one per tile and destination, each its own add,
+// lookups and partly written sectors: with 1 090 partitions and 5.8 M walkers a
+// pass took 162 us in tiles of 2048, 105 of 4096 and 81 of 8192, whether one or
+// two CTAs shared an SM and whether a second buffer held the next tile (4096
+// walkers: 104, 113, 105 us).  So a tile is as large as shared memory holds: 1024
+// threads x 8 walkers, fewer where that would leave SMs without a tile.  PPR on
+// RMAT 2^30 / 2^33, 1 112 partitions: bucketing 80 -> 54 ms of an 834 -> 803 ms
+// run.  512 threads x 4 walkers, two CTAs per SM, are the autotuner's other
+// choice.  256-thread CTAs of a 4096-walker tile left 8 warps per SM to hide the
+// latencies (46 against 38 us).
 constexpr int kBucketFields = 5;                    // cur, step, idx, query, dest
 constexpr uint64_t kBulkWaitNs = 1000000000ull;     // bounded wait on one tile's copies
 
-template <int BLOCK, int ITEMS>
-size_t bucket_smem(uint32_t P)
-{
-    const uint64_t T = (uint64_t)BLOCK * ITEMS;
-    // two tiles of kBucketFields u32 fields | 2 mbarriers | 4 u32 per destination | u16 permutation
-    return 4 * 2 * kBucketFields * T + 16 + 16ull * P + 2 * T;
-}
+// a tile of kBucketFields u32 fields | mbarrier | 4 u32 per destination | u16 permutation
+size_t bucket_smem(uint32_t P, uint64_t T) { return 4 * kBucketFields * T + 16 + 16ull * P + 2 * T; }
 
 template <int BLOCK, int ITEMS>
-__global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) bucket_sort_kernel(ScatterArgs a)
+__global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) bucket_sort_kernel(ScatterArgs a, uint32_t most)
 {
-    constexpr uint32_t T = BLOCK * ITEMS;
+    static_assert(BLOCK * ITEMS <= (int)kChunk);
     constexpr uint32_t kPerMax = kSmemPartMax / BLOCK;
     extern __shared__ __align__(16) uint32_t smem[];
     __shared__ uint32_t warp_tot[BLOCK / 32];
     __shared__ uint32_t tile_total;
     const uint32_t P = a.P;
-    uint64_t *mbar = reinterpret_cast<uint64_t *>(smem + 2 * kBucketFields * T);
+    const uint64_t n = a.n_dev ? *a.n_dev : a.n;
+    // items per thread: as few as one tile per CTA needs
+    uint32_t items = 1;
+    while (items < most && n > (uint64_t)gridDim.x * BLOCK * items) items *= 2;
+    const uint32_t T = BLOCK * items;
+    uint64_t *mbar = reinterpret_cast<uint64_t *>(smem + kBucketFields * T);
     uint32_t *s_off = reinterpret_cast<uint32_t *>(mbar + 2);  // P: tile count, then offset in the sorted tile
     uint32_t *s_base = s_off + P;                              // P: first reserved slot of the window
     uint32_t *s_ch0 = s_base + P;                              // P: chunk holding s_base
@@ -681,51 +684,38 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) bucket_sort_kernel(Scatte
     if (blockIdx.x == 0 && threadIdx.x == 0 && !a.n_dev) a.clk[0] = globaltimer_ns();
     const uint32_t *src[kBucketFields] = {a.in_cur, a.in_step, a.in_idx, a.in_q, a.in_dest};
     if (a.err && (*(volatile unsigned int *)a.err & 2u)) return;
-    const uint64_t n = a.n_dev ? *a.n_dev : a.n;
     const uint64_t tiles = (n + T - 1) / T;
     bool bulk = true;
 #pragma unroll
     for (int f = 0; f < kBucketFields; f++) bulk = bulk && ((uintptr_t)src[f] & 15) == 0;
     if (threadIdx.x == 0) {
-        mbar_init(&mbar[0], 1);
-        mbar_init(&mbar[1], 1);
+        mbar_init(mbar, 1);
         mbar_init_fence();
     }
     __syncthreads();
-    // thread 0: copies of tile `tile` into buffer b
-    auto issue = [&](uint64_t tile, int b) {
+    // thread 0: copies of tile `tile`
+    auto issue = [&](uint64_t tile) {
         const uint64_t t0 = tile * T;
         const uint32_t m = (uint32_t)(n - t0 < T ? n - t0 : T);
         const uint32_t bytes = (4 * m + 15) & ~15u;
-        mbar_arrive_expect_tx(&mbar[b], kBucketFields * bytes);
+        mbar_arrive_expect_tx(mbar, kBucketFields * bytes);
 #pragma unroll
-        for (int f = 0; f < kBucketFields; f++) bulk_load_smem(smem + (b * kBucketFields + f) * T, src[f] + t0, bytes, &mbar[b]);
+        for (int f = 0; f < kBucketFields; f++) bulk_load_smem(smem + f * T, src[f] + t0, bytes, mbar);
     };
-    // copies issued into / completions waited for on buffer 0 and buffer 1
-    uint32_t issued0 = 0, issued1 = 0, waited0 = 0, waited1 = 0;
+    uint32_t issued = 0, waited = 0;  // copies issued / completions waited for
     uint64_t tile = blockIdx.x;
     if (bulk && tile < tiles) {
-        if (threadIdx.x == 0) issue(tile, 0);
-        issued0++;
+        if (threadIdx.x == 0) issue(tile);
+        issued++;
     }
     const uint32_t per = (P + BLOCK - 1) / BLOCK;  // destinations a thread reserves and scans
-    for (uint32_t it = 0; tile < tiles; tile += gridDim.x, it++) {
-        const int b = it & 1;
+    for (; tile < tiles; tile += gridDim.x) {
         const uint64_t t0 = tile * T;
         const uint32_t m = (uint32_t)(n - t0 < T ? n - t0 : T);
-        if (bulk && tile + gridDim.x < tiles) {
-            // buffer b^1 was last read by the previous tile, which ended at a barrier
-            if (threadIdx.x == 0) issue(tile + gridDim.x, b ^ 1);
-            if (b) issued0++;
-            else issued1++;
-        }
         for (uint32_t i = threadIdx.x; i < P; i += BLOCK) s_off[i] = 0;
         if (bulk) {
-            const bool ok = mbar_wait_bounded(&mbar[b], (b ? waited1 : waited0) & 1, kBulkWaitNs);
-            if (ok) {
-                if (b) waited1++;
-                else waited0++;
-            }
+            const bool ok = mbar_wait_bounded(mbar, waited & 1, kBulkWaitNs);
+            waited += ok;
             if (__syncthreads_or(!ok)) {
                 if (threadIdx.x == 0 && a.err) atomicOr(a.err, 1u);
                 bulk = false;
@@ -735,7 +725,7 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) bucket_sort_kernel(Scatte
         }
         const uint32_t *f_cur, *f_step, *f_idx, *f_q, *f_dest;
         if (bulk) {
-            const uint32_t *buf = smem + b * kBucketFields * T;
+            const uint32_t *buf = smem;
             f_cur = buf, f_step = buf + T, f_idx = buf + 2 * T, f_q = buf + 3 * T, f_dest = buf + 4 * T;
         } else {
             f_cur = a.in_cur + t0, f_step = a.in_step + t0, f_idx = a.in_idx + t0, f_q = a.in_q + t0,
@@ -743,9 +733,9 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) bucket_sort_kernel(Scatte
         }
         uint32_t dest[ITEMS], rank[ITEMS];
 #pragma unroll
-        for (int k = 0; k < ITEMS; k++) {
+        for (uint32_t k = 0; k < ITEMS; k++) {
             const uint32_t i = k * BLOCK + threadIdx.x;
-            dest[k] = i < m ? f_dest[i] : 0xFFFFFFFFu;
+            dest[k] = k < items && i < m ? f_dest[i] : 0xFFFFFFFFu;
             rank[k] = dest[k] != 0xFFFFFFFFu ? atomicAdd(&s_off[dest[k]], 1u) : 0u;
         }
         __syncthreads();
@@ -772,7 +762,7 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) bucket_sort_kernel(Scatte
             const uint32_t w = win[j] + base[j] / kChunk;
             s_base[d] = base[j];
             s_ch0[d] = a.plan_chunks[w];
-            // a run (at most T < kChunk walkers) spans one chunk or two
+            // a run (at most T <= kChunk walkers) spans one chunk or two
             s_ch1[d] = (base[j] + cnt[j] - 1) / kChunk != base[j] / kChunk ? a.plan_chunks[w + 1] : 0u;
         }
         uint32_t off = scan_detail::block_exclusive<uint32_t, BLOCK>(mine, warp_tot, &tile_total);
@@ -803,11 +793,15 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) bucket_sort_kernel(Scatte
             c[3 * kChunk + jj] = f_q[i];
         }
         __syncthreads();
+        // the tile's fields have been read: the next one's come in
+        if (bulk && tile + gridDim.x < tiles) {
+            if (threadIdx.x == 0) issue(tile + gridDim.x);
+            issued++;
+        }
     }
     // copies still in flight exist only after a wait gave up: wait for them
     // (bounded) before this CTA's shared memory is released
-    while (waited0 < issued0 && mbar_wait_bounded(&mbar[0], waited0 & 1, kBulkWaitNs)) waited0++;
-    while (waited1 < issued1 && mbar_wait_bounded(&mbar[1], waited1 & 1, kBulkWaitNs)) waited1++;
+    while (waited < issued && mbar_wait_bounded(mbar, waited & 1, kBulkWaitNs)) waited++;
     if (threadIdx.x == 0) atomicMax(&a.clk[1], (unsigned long long)globaltimer_ns());
 }
 
@@ -963,48 +957,31 @@ cudaError_t launch_plan(const PlanArgs &a, cudaStream_t st)
 cudaError_t launch_scatter(const ScatterArgs &a, int device, cudaStream_t st)
 {
     if (a.n == 0) return cudaSuccess;
-    // per device and partition count: SMs, and the CTAs per SM of both shapes
-    // (one launch per wave iteration: no attribute queries on that path)
+    // per device: SMs and the shared memory of a CTA (one launch per wave
+    // iteration: no attribute queries on that path)
     static thread_local int cached_device = -1;
-    static thread_local uint32_t cached_P = 0;
-    static thread_local int sms = 0, smem_optin = 0, per_sm_big = 0, per_sm_small = 0;
-    if (cached_device != device || (a.P <= kSmemPartMax && cached_P != a.P)) {
+    static thread_local int sms = 0, smem_most = 0;
+    if (cached_device != device) {
         cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
-        // room for the kernels' static shared memory
-        const int dyn = smem_optin - 1024;
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&smem_most, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+        smem_most -= 1024;  // room for the kernels' static shared memory
         if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(bucket_sort_kernel<1024, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn);
+            e = cudaFuncSetAttribute(bucket_sort_kernel<1024, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_most);
         if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(bucket_sort_kernel<512, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn);
-        per_sm_big = per_sm_small = 0;
-        if (e == cudaSuccess && a.P <= kSmemPartMax && bucket_smem<1024, 4>(a.P) + 1024 <= (size_t)smem_optin)
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_big, bucket_sort_kernel<1024, 4>, 1024,
-                                                              bucket_smem<1024, 4>(a.P));
-        if (e == cudaSuccess && a.P <= kSmemPartMax)
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_small, bucket_sort_kernel<512, 4>, 512,
-                                                              bucket_smem<512, 4>(a.P));
-        if (e != cudaSuccess) {
-            cached_device = -1;
-            return e;
-        }
+            e = cudaFuncSetAttribute(bucket_sort_kernel<512, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_most);
+        if (e != cudaSuccess) return e;
         cached_device = device;
-        cached_P = a.P;
     }
     if (a.P <= kSmemPartMax) {
-        // 4096-walker tiles unless 2048 are asked for (items 8), or where
-        // 4096 do not fit (P above about 3 700)
-        const bool small = a.items == 8 || per_sm_big == 0;
-        const int block = small ? 512 : 1024;
-        const size_t smem = small ? bucket_smem<512, 4>(a.P) : bucket_smem<1024, 4>(a.P);
-        const uint64_t tile = (uint64_t)block * 4;
-        const uint64_t tiles = (a.n + tile - 1) / tile;
-        const int per_sm = std::max(1, small ? per_sm_small : per_sm_big);
-        const uint64_t blocks = std::min<uint64_t>(tiles, (uint64_t)sms * per_sm);
-        if (small)
-            bucket_sort_kernel<512, 4><<<(unsigned)blocks, block, smem, st>>>(a);
-        else
-            bucket_sort_kernel<1024, 4><<<(unsigned)blocks, block, smem, st>>>(a);
+        if (a.items == 8) {
+            const uint64_t blocks = std::min<uint64_t>((a.n + 511) / 512, 2ull * sms);
+            bucket_sort_kernel<512, 4><<<(unsigned)blocks, 512, bucket_smem(a.P, 2048), st>>>(a, 4);
+        } else {
+            // where 8192 walkers do not fit beside the tables (P above 3 000) 4096 do
+            const uint32_t most = bucket_smem(a.P, 8192) <= (size_t)smem_most ? 8 : 4;
+            const uint64_t blocks = std::min<uint64_t>((a.n + 1023) / 1024, (uint64_t)sms);
+            bucket_sort_kernel<1024, 8><<<(unsigned)blocks, 1024, bucket_smem(a.P, 1024ull * most), st>>>(a, most);
+        }
         return cudaGetLastError();
     }
     const uint64_t tile = (uint64_t)kPartBlock * kScatterItems;

@@ -129,7 +129,7 @@ struct ScatterArgs {
     const uint32_t *win_off;       // P: start of the destination's window in plan_chunks
     const uint32_t *plan_chunks;   // chunk ids of every window
     uint32_t P;
-    int items;                     // bucketing tile: 16 (0) = 4096 walkers, 8 = 2048
+    int items;                     // bucketing tile: 16 (0) = up to 8192 walkers, 8 = 2048
     unsigned int *err;             // bit 0 set when a tile's bulk copy did not complete in time;
                                    // the pass does nothing while bit 1 (a failed device plan) is set
     // non-null: the staged count lives here (device memory) and n only bounds it

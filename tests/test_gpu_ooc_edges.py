@@ -72,3 +72,17 @@ def test_ppr_lengths(lt, require_gpu, skewed, walkers, prob):
     want, _, st = oracle.ppr(rp, col, 0, walkers, prob=prob, seed=12345678901)
     assert (e.ppr(0, walkers, prob) == want).all()
     assert e.stats()["moves"] == int(st[1])
+
+
+@pytest.mark.parametrize("part_bytes", [300, 1000, 64 << 10])  # about 3 700 partitions (tiles of 4096), 970 and 14
+@pytest.mark.parametrize("walkers", [1023, 1025, 160003, 2600003])  # one tile to several of the largest per CTA
+@pytest.mark.parametrize("items", [0, 8])
+def test_bucket_tiles(lt, require_gpu, regular, part_bytes, walkers, items):
+    rp, col = regular
+    g = lt.Graph.from_csr(rp, col, part_bytes)
+    share = -(-8 * len(rp) // part_bytes)
+    e = lt.Engine(g, partitions=min(g.num_partitions - 1, share + 2), seed=9, sched=3, bucket_items=items)
+    want, st = oracle.pagerank(rp, col, walkers, length=4, seed=9, start_mode=2)
+    assert (e.pagerank(walkers, length=4, start=2) == want).all()
+    s = e.stats()
+    assert (s["updates"], s["moves"], s["teleports"]) == tuple(int(x) for x in st)
