@@ -977,7 +977,7 @@ cudaError_t launch_scatter(const ScatterArgs &a, int device, cudaStream_t st)
             const uint64_t blocks = std::min<uint64_t>((a.n + 511) / 512, 2ull * sms);
             bucket_sort_kernel<512, 4><<<(unsigned)blocks, 512, bucket_smem(a.P, 2048), st>>>(a, 4);
         } else {
-            // where 8192 walkers do not fit beside the tables (P above 3 000) 4096 do
+            // where 8192 walkers do not fit beside the tables (P above 3 199) 4096 do
             const uint32_t most = bucket_smem(a.P, 8192) <= (size_t)smem_most ? 8 : 4;
             const uint64_t blocks = std::min<uint64_t>((a.n + 1023) / 1024, (uint64_t)sms);
             bucket_sort_kernel<1024, 8><<<(unsigned)blocks, 1024, bucket_smem(a.P, 1024ull * most), st>>>(a, most);

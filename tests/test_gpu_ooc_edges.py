@@ -24,7 +24,7 @@ def skewed():
     return oracle.rmat(14, 1 << 18, seed=6)
 
 
-@pytest.mark.parametrize("part_bytes", [200, 400, 1000, 64 << 10])  # 5 800, 2 700, 970 and 14 partitions
+@pytest.mark.parametrize("part_bytes", [200, 400, 1000, 64 << 10])  # 4 514, 2 008, 757 and 12 partitions
 @pytest.mark.parametrize("sched", [0, 4])
 @pytest.mark.parametrize("index", [True, False])
 def test_partition_counts(lt, require_gpu, regular, part_bytes, sched, index):
@@ -74,7 +74,7 @@ def test_ppr_lengths(lt, require_gpu, skewed, walkers, prob):
     assert e.stats()["moves"] == int(st[1])
 
 
-@pytest.mark.parametrize("part_bytes", [300, 1000, 64 << 10])  # about 3 700 partitions (tiles of 4096), 970 and 14
+@pytest.mark.parametrize("part_bytes", [240, 1000, 64 << 10])  # 3 611 partitions (tiles of 4096), 757 and 12
 @pytest.mark.parametrize("walkers", [1023, 1025, 160003, 2600003])  # one tile to several of the largest per CTA
 @pytest.mark.parametrize("items", [0, 8])
 def test_bucket_tiles(lt, require_gpu, regular, part_bytes, walkers, items):
