@@ -199,6 +199,9 @@ struct Ooc {
         std::vector<cudaEvent_t> b;
     };
     std::vector<Timed> timed;
+    // claimed by a wave iteration, issued together before its kernels
+    std::vector<uint32_t> claimed;
+    std::vector<std::pair<uint32_t, cudaEvent_t>> *claimed_to = nullptr;
     cudaEvent_t load_a = nullptr;
     std::vector<cudaEvent_t> load_b;
 
@@ -635,10 +638,11 @@ int32_t free_slot(Ooc &o)
 // may still be read by them).  The table entry is published on the compute
 // stream once the copy is done: right away (the next kernel waits for the
 // copy), or, for the loads of a wave, before the next wave's kernel.
-lt_status start_load(Ooc &o, uint32_t p, int32_t slot, std::vector<std::pair<uint32_t, cudaEvent_t>> *deferred)
+//
+// claim_load takes the slot and makes the copy stream wait; issue_load copies.
+lt_status claim_load(Ooc &o, uint32_t p, int32_t slot)
 {
     lt_engine &e = *o.e;
-    lt_graph &g = *o.g;
     if (!o.copy_waits) {
         // once for all loads between two passes
         cudaEvent_t free_ev = ev_get(o);
@@ -647,13 +651,40 @@ lt_status start_load(Ooc &o, uint32_t p, int32_t slot, std::vector<std::pair<uin
         o.ev_free.push_back(free_ev);
         o.copy_waits = true;
     }
-    if (!o.load_a) {
-        o.load_a = ev_get(o);
-        LT_CUDA_TRY(cudaEventRecord(o.load_a, e.s_copy));
-    }
+    o.loaded_at[p] = o.iteration;
+    o.slot_of[p] = slot;
+    o.part_in_slot[slot] = (int32_t)p;
+    return LT_OK;
+}
+
+// The first load of a group records its start (see close_loads).
+lt_status open_loads(Ooc &o)
+{
+    if (o.load_a) return LT_OK;
+    o.load_a = ev_get(o);
+    LT_CUDA_TRY(cudaEventRecord(o.load_a, o.e->s_copy));
+    return LT_OK;
+}
+
+// The addresses of p's slices in its slot, and the load's statistics.
+void loaded(Ooc &o, uint32_t p, uint8_t *base, uint64_t rp_bytes, uint64_t col_off)
+{
+    lt_graph &g = *o.g;
+    o.h_rp[p] = (unsigned long long)(uintptr_t)(o.d_index ? (uint8_t *)(o.d_index + g.node_off[p]) : base);
+    o.h_col[p] = (unsigned long long)(uintptr_t)(base + col_off);
+    o.e->stats.graph_loading_calls++;
+    o.e->stats.h2d_graph_bytes += rp_bytes + 4 * (g.edge_off[p + 1] - g.edge_off[p]);
+    o.e->stats.partition_loads++;
+}
+
+lt_status issue_load(Ooc &o, uint32_t p, std::vector<std::pair<uint32_t, cudaEvent_t>> *deferred)
+{
+    lt_engine &e = *o.e;
+    lt_graph &g = *o.g;
+    LT_TRY(open_loads(o));
     const uint64_t n0 = g.node_off[p], n1 = g.node_off[p + 1];
     const uint64_t e0 = g.edge_off[p], e1 = g.edge_off[p + 1];
-    uint8_t *base = o.d_slots + (uint64_t)slot * o.slot_stride;
+    uint8_t *base = o.d_slots + (uint64_t)o.slot_of[p] * o.slot_stride;
     const uint64_t rp_bytes = o.d_index ? 0 : 8 * (n1 - n0 + 1);
     const uint64_t col_off = (rp_bytes + 15) & ~15ull;
     if (rp_bytes) LT_CUDA_TRY(cudaMemcpyAsync(base, g.rowptr() + n0, rp_bytes, cudaMemcpyHostToDevice, e.s_copy));
@@ -661,21 +692,101 @@ lt_status start_load(Ooc &o, uint32_t p, int32_t slot, std::vector<std::pair<uin
     const cudaEvent_t copied = ev_get(o);
     o.load_b.push_back(copied);
     LT_CUDA_TRY(cudaEventRecord(copied, e.s_copy));
-    o.h_rp[p] = (unsigned long long)(uintptr_t)(o.d_index ? (uint8_t *)(o.d_index + n0) : base);
-    o.h_col[p] = (unsigned long long)(uintptr_t)(base + col_off);
-    o.loaded_at[p] = o.iteration;
-    o.slot_of[p] = slot;
-    o.part_in_slot[slot] = (int32_t)p;
+    loaded(o, p, base, rp_bytes, col_off);
     if (deferred) {
         deferred->push_back({p, copied});
     } else {
         LT_CUDA_TRY(cudaStreamWaitEvent(e.s_compute, copied, 0));
         set_entry(o, p);
     }
-    e.stats.graph_loading_calls++;
-    e.stats.h2d_graph_bytes += rp_bytes + 4 * (e1 - e0);
-    e.stats.partition_loads++;
     return LT_OK;
+}
+
+lt_status start_load(Ooc &o, uint32_t p, int32_t slot, std::vector<std::pair<uint32_t, cudaEvent_t>> *deferred)
+{
+    LT_TRY(claim_load(o, p, slot));
+    return issue_load(o, p, deferred);
+}
+
+// Loads of small partitions by one kernel: column slices of up to kCopyBatch
+// partitions, from host memory by coalesced 4-byte loads (a slice may start at
+// any word).  A copy and its event cost the host some 4 us and the copy engine
+// as much beside the transfer, which is 5 us for 1 MB.  Few CTAs, with 229 KB in
+// flight: the pass's own reads of host memory queue behind theirs.  A burst of
+// queries on RMAT 2^20 / 2^24 (70 partitions of 1 MB, 7 loads a pass): copies 5.0
+// ms, 10 CTAs 4.16, 14 4.08, 20 4.57, 28 4.7, 56 5.0, 112 5.4; 48 queries of some
+// 8000 walks, copies -> 14 CTAs: partitions of 256 KB 6.15 -> 5.5, 512 KB 5.3 ->
+// 4.7, 1 MB 3.75 -> 3.1, 2 MB 2.6 -> 2.3, 4 and 8 MB the same.
+constexpr uint64_t kCopyPartBytes = 3 << 20;
+constexpr uint32_t kCopyBatch = 32;
+constexpr int kCopyCtas = 14, kCopyThreads = 256, kCopyUnroll = 16;
+struct CopyBatch {
+    const uint32_t *src[kCopyBatch];
+    uint32_t *dst[kCopyBatch];
+    uint64_t words[kCopyBatch];
+    uint32_t n;
+};
+
+__global__ void __launch_bounds__(kCopyThreads) load_kernel(const __grid_constant__ CopyBatch b)
+{
+    constexpr uint64_t kTile = (uint64_t)kCopyThreads * kCopyUnroll;
+    uint64_t tile = blockIdx.x;  // among those of the slices from p on
+    for (uint32_t p = 0; p < b.n; p++) {
+        const uint32_t *src = b.src[p];
+        uint32_t *dst = b.dst[p];
+        const uint64_t n = b.words[p], tiles = (n + kTile - 1) / kTile;
+        for (; tile < tiles; tile += gridDim.x) {
+            const uint64_t i = tile * kTile + threadIdx.x;
+            uint32_t v[kCopyUnroll];
+#pragma unroll
+            for (int k = 0; k < kCopyUnroll; k++)
+                if (i + k * kCopyThreads < n) v[k] = src[i + k * kCopyThreads];
+#pragma unroll
+            for (int k = 0; k < kCopyUnroll; k++)
+                if (i + k * kCopyThreads < n) dst[i + k * kCopyThreads] = v[k];
+        }
+        tile -= tiles;
+    }
+}
+
+// Issues the loads a wave iteration has claimed (see wave_step).
+lt_status issue_claimed(Ooc &o)
+{
+    lt_engine &e = *o.e;
+    lt_graph &g = *o.g;
+    lt_status s = LT_OK;
+    const bool small = o.d_index && o.zc_col_base && o.slot_stride <= kCopyPartBytes && o.claimed.size() > 1;
+    for (size_t at = 0; at < o.claimed.size();) {
+        if (!small) {
+            const lt_status l = issue_load(o, o.claimed[at++], o.claimed_to);
+            if (s == LT_OK) s = l;
+            continue;
+        }
+        CopyBatch b{};
+        const uint32_t n = (uint32_t)std::min<size_t>(kCopyBatch, o.claimed.size() - at);
+        lt_status l = open_loads(o);
+        const cudaEvent_t copied = ev_get(o);
+        o.load_b.push_back(copied);
+        for (uint32_t k = 0; k < n; k++) {
+            const uint32_t p = o.claimed[at + k];
+            uint8_t *base = o.d_slots + (uint64_t)o.slot_of[p] * o.slot_stride;
+            b.src[k] = (const uint32_t *)(o.zc_col_base + 4 * g.edge_off[p]);
+            b.dst[k] = (uint32_t *)base;
+            b.words[k] = g.edge_off[p + 1] - g.edge_off[p];
+            b.n++;
+            loaded(o, p, base, 0, 0);
+            o.claimed_to->push_back({p, copied});
+        }
+        load_kernel<<<kCopyCtas, kCopyThreads, 0, e.s_copy>>>(b);
+        cudaError_t c = cudaGetLastError();
+        if (c == cudaSuccess) c = cudaEventRecord(copied, e.s_copy);
+        if (l == LT_OK && c != cudaSuccess) l = fail(LT_ERR_CUDA, "partition loads: %s", cudaGetErrorString(c));
+        if (s == LT_OK) s = l;
+        e.stats.kernel_launches++;
+        at += n;
+    }
+    o.claimed.clear();
+    return s;
 }
 
 lt_status load_partition(Ooc &o, uint32_t p, std::vector<std::pair<uint32_t, cudaEvent_t>> *deferred)
@@ -1478,6 +1589,17 @@ lt_status wave_step(Ooc &o, const RunParams &rp, WaveState &w, bool &done)
     auto &idle = w.idle;
     auto &draining = w.draining;
     auto &loading = w.loading;
+    // the loads this iteration chooses are issued together, or on the way out
+    struct Claims {
+        Ooc &o;
+        ~Claims() { issue_claimed(o); }
+    } claims{o};
+    o.claimed_to = &inflight;
+    auto claim = [&](uint32_t p, int32_t slot) {
+        LT_TRY(claim_load(o, p, slot));
+        o.claimed.push_back(p);
+        return LT_OK;
+    };
     done = false;
     {
         // publish the loads whose copies have finished; the others stay in
@@ -1571,7 +1693,7 @@ lt_status wave_step(Ooc &o, const RunParams &rp, WaveState &w, bool &done)
                 slot = o.slot_of[w];
                 LT_TRY(evict_partition(o, w));
             }
-            LT_TRY(start_load(o, c, slot, &inflight));
+            LT_TRY(claim(c, slot));
             loading[c] = 1;
             o.last_used[c] = o.iteration;
             started++;
@@ -1587,7 +1709,7 @@ lt_status wave_step(Ooc &o, const RunParams &rp, WaveState &w, bool &done)
                     const int32_t slot = free_slot(o);
                     if (slot < 0) break;
                     if (o.slot_of[p] >= 0 || loading[p]) continue;
-                    LT_TRY(start_load(o, p, slot, &inflight));
+                    LT_TRY(claim(p, slot));
                     loading[p] = 1;
                     o.last_used[p] = o.iteration;
                     e.stats.prefill_loads++;
@@ -1613,7 +1735,7 @@ lt_status wave_step(Ooc &o, const RunParams &rp, WaveState &w, bool &done)
                 if (started >= m) break;
                 const int32_t slot = free_slot(o);
                 if (slot < 0) break;
-                LT_TRY(start_load(o, f.second, slot, &inflight));
+                LT_TRY(claim(f.second, slot));
                 loading[f.second] = 1;
                 o.last_used[f.second] = o.iteration;
                 started++;
@@ -1674,7 +1796,7 @@ lt_status wave_step(Ooc &o, const RunParams &rp, WaveState &w, bool &done)
                     swaps++;
                     const int32_t slot = o.slot_of[pout];
                     LT_TRY(evict_partition(o, pout));
-                    LT_TRY(start_load(o, pin, slot, &inflight));
+                    LT_TRY(claim(pin, slot));
                     loading[pin] = 1;
                     o.last_used[pin] = o.iteration;
                     started++;
@@ -1682,6 +1804,7 @@ lt_status wave_step(Ooc &o, const RunParams &rp, WaveState &w, bool &done)
                 }
             }
         }
+        LT_TRY(issue_claimed(o));
         if (started) e.stats.explicit_iterations++;
         if (!e.cfg.pipeline) {
             // no pipelining (--no-pipeline): the loads finish before this

@@ -86,3 +86,23 @@ def test_bucket_tiles(lt, require_gpu, regular, part_bytes, walkers, items):
     assert (e.pagerank(walkers, length=4, start=2) == want).all()
     s = e.stats()
     assert (s["updates"], s["moves"], s["teleports"]) == tuple(int(x) for x in st)
+
+
+@pytest.mark.parametrize("part_bytes", [2000, 16 << 10, 120 << 10])  # 487, 59 and 8 slices of odd lengths at any word
+@pytest.mark.parametrize("pipeline", [True, False])
+@pytest.mark.parametrize("sched", [3, 4])
+def test_small_loads(lt, require_gpu, part_bytes, pipeline, sched):
+    rng = np.random.default_rng(12)
+    V = 30011
+    deg = rng.integers(0, 13, V)
+    rp = np.concatenate([[0], np.cumsum(deg)]).astype(np.uint64)
+    col = rng.integers(0, V, int(rp[-1])).astype(np.uint32)
+    g = lt.Graph.from_csr(rp, col, part_bytes)
+    share = -(-8 * len(rp) // part_bytes)
+    e = lt.Engine(g, partitions=min(g.num_partitions - 1, share + max(1, g.num_partitions // 2)), seed=3, sched=sched,
+                  pipeline=pipeline, load_factor=1)
+    for run in range(2):
+        want, _, st = oracle.ppr(rp, col, 7, 120011, prob=0.1, seed=3)
+        assert (e.ppr(7, 120011, 0.1) == want).all()
+        s = e.stats()
+        assert (s["updates"], s["moves"]) == (int(st[0]), int(st[1]))
