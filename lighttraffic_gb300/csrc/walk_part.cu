@@ -5,9 +5,10 @@
 // insertToQueue kernels (src/WalkManager.h:60-282) together with the 1-thread
 // page kernels of src/buffer/Pool.h:484-528.
 //
-// Step kernel (persistent, one walker per lane, warp-aggregated refill):
-//   input  = the chunks queued for one partition, plus walkers created lazily
-//            from their ordinal (PPR source walkers, per-vertex starts);
+// Step kernel (persistent, one walker per lane; a warp takes blocks of input
+// ordinals from one counter):
+//   input  = the chunks queued for the partitions drained, plus walkers created
+//            lazily from their ordinal (PPR source walkers, per-vertex starts);
 //   a walker keeps stepping while the partition holding its vertex is readable
 //   -- cached in a device slot, or mapped from pinned host memory for a
 //   zero-copy pass -- which generalises the reference's "walk while inside the
@@ -15,12 +16,14 @@
 //   updates that read no graph data (the final PPR / PageRank count, PageRank
 //   teleports) run wherever the walker is;
 //   a walker whose next update needs an unreadable partition is written to a
-//   staging area (warp-aggregated slot reservation) and counted in a
-//   per-destination histogram (shared memory, flushed once per CTA).
-// Scatter kernel: appends staged walkers to their destination queues; a CTA
-// counts its tile per destination in shared memory and reserves one range per
+//   staging area (gathered in the warp's shared memory, one reservation for 32)
+//   and counted in a per-destination histogram (shared memory, flushed once per
+//   CTA).
+// Bucketing: appends staged walkers to their destination queues; a CTA sorts
+// its tile by destination in shared memory and reserves one range per
 // destination with one global atomic (the two-level scheme of
-// src/WalkManager.h:122-190), into chunks the host allocated beforehand.
+// src/WalkManager.h:122-190), into chunks that the plan kernel or the host has
+// taken from the free ones.
 #include <algorithm>
 
 #include "lt_core.cuh"
@@ -147,19 +150,20 @@ __device__ __forceinline__ void serve_count(const StepArgs &a, bool have, uint2 
     __syncwarp();
 }
 
-// Resident CTAs per SM the register budget is sized for: PPR fits 48
-// registers with no spills (5 x 256 threads), PageRank and generic walks 40
-// (6 x 256); unbounded, PPR took 55 (4 CTAs) and hops in flight were the limit
-// on zero-copy reads.
-template <int APP>
-constexpr int part_min_blocks() { return APP == kPPR ? 5 : 6; }
+// Resident CTAs per SM the register budget is sized for: 64 registers a thread,
+// no spills.  With 5 (PPR) and 6 (the others) 20 to 88 bytes spilled: cached
+// partitions alone 25 -> 14 ms per run (PPR of 100 M walks on RMAT 2^26 / 2^30),
+// PageRank of 7e5 walkers on RMAT 2^20 / 2^24, 21 of 70 partitions cached, 1.42 ->
+// 1.36 ms, walks of 20 hops on RMAT 2^22 / 2^26 by the plain scheduler 30.8 ->
+// 29.7; kernels that wait for host reads are the same.
+constexpr int kPartMinBlocks = 4;
 
 // HOT: the hot-vertex tier is on (a.hot_on); SERVE: query mode (a.q_seed);
 // RP32: row offsets are u32 offsets from the partition's first edge, all
 // partitions' back to back at a.zc_rp_base.  Separate instances keep the
 // registers of the others.
 template <int APP, bool HOT, bool SERVE, bool RP32>
-__global__ void __launch_bounds__(kPartBlock, part_min_blocks<APP>()) walk_part_kernel(const __grid_constant__ StepArgs a)
+__global__ void __launch_bounds__(kPartBlock, kPartMinBlocks) walk_part_kernel(const __grid_constant__ StepArgs a)
 {
     extern __shared__ __align__(16) uint32_t smem[];
     __shared__ PartWarp<APP == kPPR && !SERVE, SERVE> s_warp[kPartBlock / 32];
