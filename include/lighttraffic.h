@@ -157,7 +157,7 @@ typedef struct lt_stats {
     uint64_t zerocopy_calls;
     uint64_t walker_loading_calls;
     uint64_t walker_evicting_calls;
-    double step_kernel_ms;    /* CUDA-event time of the step kernels of the last run */
+    double step_kernel_ms;    /* time of the step kernels of the last run */
     uint64_t handoffs;        /* walkers staged and bucketed into another partition's queue */
     uint64_t overlap_computes; /* plain / FIFO loop: cached partitions computed while a load was in
                                   flight (getComputedPartition, src/Scheduler.h:194-208) */
@@ -171,7 +171,7 @@ typedef struct lt_stats {
                                   policy forecasts more entries for */
     uint64_t prefill_loads;    /* wave runs: loads into a cold cache at a run's start, in the order of
                                   the policy's forecast (entries of its previous runs) */
-    double bucket_ms;          /* CUDA-event time of the bucketing (scatter) kernels */
+    double bucket_ms;          /* time of the planning and bucketing kernels */
     double host_wait_ms;       /* host time blocked waiting for each iteration's step kernel */
     uint64_t device_plans;     /* bucketing passes planned on the device (the others by the host) */
     /* host time of the out-of-core loop outside waits, by phase (wave runs): */

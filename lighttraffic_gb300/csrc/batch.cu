@@ -13,9 +13,11 @@
 //             semantics of app/ppr.cu:22-42 to its endpoint; endpoints are
 //             gathered and added to their queries' tables (linear probing, u32
 //             counts) 32 at a time;
-//   count   : one CTA per query counts its occupied slots;
-//   offsets : exclusive scan of the counts;
-//   compact : one CTA per query writes (vertex, count) pairs in slot order.
+//   count   : occupied slots of every 4096-slot chunk of the tables;
+//   offsets : exclusive scan of the chunks' counts, and each query's first pair;
+//   compact : (vertex, count) pairs in slot order, chunk by chunk, gathered in
+//             shared memory and written where the results go: the caller's
+//             device arrays or page-locked host arrays.
 #include "batch.h"
 
 #include <algorithm>

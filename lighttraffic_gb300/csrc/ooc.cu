@@ -16,10 +16,11 @@
 // Wave runs (learned, frequency, batched; wave_step) drain every cached queue
 // per launch while the next loads stream in -- see the comment at wave_step.
 // Queue bookkeeping lives on the host (exact counts, no per-decision D2H of
-// queue metadata as in src/buffer/Pool.h:604-606); per iteration one small
-// D2H (the destination histogram) crosses the link, and the work list and
-// chunk plan go up by a kernel reading mapped pinned memory.  Checkpoints and
-// resume of runs, and the serving loop, are at the end of the file.
+// queue metadata as in src/buffer/Pool.h:604-606); per iteration the plan kernel
+// writes one small control block (the destination histogram, kernel times) to
+// mapped pinned memory, and the pass's first kernel reads table updates, the
+// work list and the plan's inputs from there.  Checkpoints and resume of runs,
+// and the serving loop, are at the end of the file.
 #include "ooc.h"
 
 #include <algorithm>

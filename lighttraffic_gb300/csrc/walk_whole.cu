@@ -9,10 +9,10 @@
 //  * Persistent grid: SMs x resident CTAs; each lane owns one walker at a time.
 //  * Lazy walker creation: walker i is created from its index alone (start
 //    vertex and, for PPR, its geometric length are pure functions of
-//    (seed, run, i)), so no walker array is ever materialised.  A lane whose
-//    walker ends takes the next index from a warp-aggregated atomic counter
-//    (one atomic per warp refill), keeping every lane busy despite the
-//    geometric length spread of PPR walks.
+//    (seed, run, i)), so no walker array is ever materialised.  The first
+//    walkers are dealt out; a warp takes further ones from an atomic counter
+//    (one atomic per refill; PPR: per pool of walkers with their lengths
+//    drawn), keeping its lanes busy despite the spread of PPR's lengths.
 //  * Graph reads: rowptr[cur], rowptr[cur+1] (16 B) and col[e] (4 B) through
 //    the read-only path; counters are u64 reductions resolved in L2.  Column
 //    loads are evict-first, row offsets and counters evict-last (mem.cuh).
