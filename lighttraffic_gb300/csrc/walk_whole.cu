@@ -228,61 +228,8 @@ __global__ void __launch_bounds__(block_of<APP>, 2048 / block_of<APP>) walk_whol
     uint32_t n_mov = 0, n_end = 0;  // hops taken; walks that ended at a vertex without out-edges
     Rand4 r{};                      // PageRank: the draw of the walker's next step
 
-    while (true) {
-        const unsigned busy = __ballot_sync(kFull, active);
-        const int idle = 32 - __popc(busy);
-        // ended walks keep their segments until a lane's is full or their lanes
-        // are refilled (or nothing is left to do)
-        if (GATHER && (__any_sync(kFull, path.n == kPathWords) || (exhausted ? idle == 32 : idle >= kRefillMin)))
-            path_flush(path, path.n == kPathWords || !active);
-        const uint32_t rank = __popc(~busy & ((1u << lane) - 1u));  // of an idle lane among them
-        if (APP == kPPR) {
-            if (pool_at == pool_n && idle >= kRefillMin && !exhausted) {
-                pool_base = first_deal ? a.pool * ((uint64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x)
-                                       : dealt + take(a.next, a.pool);
-                first_deal = false;
-                exhausted = pool_base + a.pool >= a.W;
-                pool_at = 0;
-                pool_n = pool_base >= a.W ? 0u : (uint32_t)min((uint64_t)a.pool, a.W - pool_base);
-                ppr_pool_fill(pool, pool_n, a.long_len, a.lim, [&](uint32_t t, uint32_t at) {
-                    return walk_draw(a.keys, t, kTagInit, a.run, pool_base + at);
-                });
-            }
-            if (pool_at < pool_n && idle >= kTakeMin) {
-                if (!active && pool_at + rank < pool_n) {
-                    idx = pool_base + pool.at[pool_at + rank];
-                    step = pool.len[pool_at + rank];
-                    cur = first_vertex<START>(a, idx);
-                    active = true;
-                }
-                pool_at = min(pool_n, pool_at + (uint32_t)idle);
-            } else if (idle == 32 && exhausted) {
-                break;
-            }
-        } else if (idle >= kRefillMin && !exhausted) {
-            const uint64_t base = first_deal ? 32ull * ((uint64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x)
-                                             : dealt + take(a.next, (uint32_t)idle);
-            exhausted = first_deal ? dealt >= a.W : base + idle >= a.W;
-            first_deal = false;
-            if (!active && base + rank < a.W) {
-                idx = base + rank;
-                cur = first_vertex<START>(a, idx);
-                step = a.length;
-                active = true;
-                if (GATHER) {
-                    path.out = a.paths + idx * (uint64_t)(a.length + 1);
-                    path.buf[0] = cur;
-                    path.n = 1;
-                } else if (APP == kWalk && a.paths) {
-                    a.paths[idx * (uint64_t)(a.length + 1)] = cur;
-                }
-                if (APP == kPageRank) r = walk_draw(a.keys, step, kTagStep, a.run, idx);
-            }
-        } else if (idle == 32) {
-            break;
-        }
-        if (!active) continue;
-
+    // one hop or update of the lane's walker
+    auto hop = [&]() {
         // The draws do not depend on the graph: they are made between the
         // row's loads and their first use.
         if (APP == kPPR) {
@@ -355,6 +302,72 @@ __global__ void __launch_bounds__(block_of<APP>, 2048 / block_of<APP>) walk_whol
             active = step != 0;
         }
         if (!active && a.endpoints) a.endpoints[idx] = cur;
+    };
+
+    while (true) {
+        const unsigned busy = __ballot_sync(kFull, active);
+        const int idle = 32 - __popc(busy);
+        // ended walks keep their segments until a lane's is full or their lanes
+        // are refilled (or nothing is left to do)
+        if (GATHER && (__any_sync(kFull, path.n == kPathWords) || (exhausted ? idle == 32 : idle >= kRefillMin)))
+            path_flush(path, path.n == kPathWords || !active);
+        const uint32_t rank = __popc(~busy & ((1u << lane) - 1u));  // of an idle lane among them
+        if (APP == kPPR) {
+            if (pool_at == pool_n && idle >= kRefillMin && !exhausted) {
+                pool_base = first_deal ? a.pool * ((uint64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x)
+                                       : dealt + take(a.next, a.pool);
+                first_deal = false;
+                exhausted = pool_base + a.pool >= a.W;
+                pool_at = 0;
+                pool_n = pool_base >= a.W ? 0u : (uint32_t)min((uint64_t)a.pool, a.W - pool_base);
+                ppr_pool_fill(pool, pool_n, a.long_len, a.lim, [&](uint32_t t, uint32_t at) {
+                    return walk_draw(a.keys, t, kTagInit, a.run, pool_base + at);
+                });
+            }
+            if (pool_at < pool_n && idle >= kTakeMin) {
+                if (!active && pool_at + rank < pool_n) {
+                    idx = pool_base + pool.at[pool_at + rank];
+                    step = pool.len[pool_at + rank];
+                    cur = first_vertex<START>(a, idx);
+                    active = true;
+                }
+                pool_at = min(pool_n, pool_at + (uint32_t)idle);
+            } else if (idle == 32 && exhausted) {
+                break;
+            }
+        } else if (idle >= kRefillMin && !exhausted) {
+            const uint64_t base = first_deal ? 32ull * ((uint64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x)
+                                             : dealt + take(a.next, (uint32_t)idle);
+            exhausted = first_deal ? dealt >= a.W : base + idle >= a.W;
+            first_deal = false;
+            if (!active && base + rank < a.W) {
+                idx = base + rank;
+                cur = first_vertex<START>(a, idx);
+                step = a.length;
+                active = true;
+                if (GATHER) {
+                    path.out = a.paths + idx * (uint64_t)(a.length + 1);
+                    path.buf[0] = cur;
+                    path.n = 1;
+                } else if (APP == kWalk && a.paths) {
+                    a.paths[idx * (uint64_t)(a.length + 1)] = cur;
+                }
+                if (APP == kPageRank) r = walk_draw(a.keys, step, kTagStep, a.run, idx);
+            }
+        } else if (idle == 32) {
+            break;
+        }
+        // No walkers to come: the lanes finish theirs without asking.  In a launch
+        // that does not fill the chip a warp's instructions wait for one another,
+        // and the votes and branches of a refill were a quarter of a hop's time
+        // (device arrays, RMAT 2^16 / 2^20, p = 0.15: 5 000 PPR walks 41 -> 32 us,
+        // 20 000 65 -> 49, 300 000 72 -> 61; 300 000 walks of 20 hops 44 -> 39;
+        // 20 000 PageRank walks of 10 33 -> 30; large launches the same).
+        if (!GATHER && exhausted && (APP != kPPR || pool_at == pool_n)) {
+            while (active) hop();
+            break;
+        }
+        if (active) hop();
     }
 
     // Statistics: one atomic per CTA and counter (one per warp would queue
