@@ -709,15 +709,19 @@ lt_status start_load(Ooc &o, uint32_t p, int32_t slot, std::vector<std::pair<uin
     return issue_load(o, p, deferred);
 }
 
-// Loads of small partitions by one kernel: column slices of up to kCopyBatch
-// partitions, from host memory by coalesced 4-byte loads (a slice may start at
-// any word).  A copy and its event cost the host some 4 us and the copy engine
+// Loads of small partitions while serving, by one kernel: column slices of up to
+// kCopyBatch partitions, from host memory by coalesced 4-byte loads (a slice may
+// start at any word).  A copy and its event cost the host some 4 us and the copy engine
 // as much beside the transfer, which is 5 us for 1 MB.  Few CTAs, with 229 KB in
 // flight: the pass's own reads of host memory queue behind theirs.  A burst of
 // queries on RMAT 2^20 / 2^24 (70 partitions of 1 MB, 7 loads a pass): copies 5.0
 // ms, 10 CTAs 4.16, 14 4.08, 20 4.57, 28 4.7, 56 5.0, 112 5.4; 48 queries of some
 // 8000 walks, copies -> 14 CTAs: partitions of 256 KB 6.15 -> 5.5, 512 KB 5.3 ->
-// 4.7, 1 MB 3.75 -> 3.1, 2 MB 2.6 -> 2.3, 4 and 8 MB the same.
+// 4.7, 1 MB 3.75 -> 3.1, 2 MB 2.6 -> 2.3, 4 and 8 MB the same.  Runs keep the
+// copies: a kernel's slices land together, and the passes that find none of them
+// are many and nearly empty (16 walks per vertex on RMAT 2^20 / 2^24 with 12 of 70
+// partitions: 97 passes, with the kernel 104 to 180), which gains a run 5 % but
+// leaves the prefetcher little to learn from.
 constexpr uint64_t kCopyPartBytes = 3 << 20;
 constexpr uint32_t kCopyBatch = 32;
 constexpr int kCopyCtas = 14, kCopyThreads = 256, kCopyUnroll = 16;
@@ -756,7 +760,7 @@ lt_status issue_claimed(Ooc &o)
     lt_engine &e = *o.e;
     lt_graph &g = *o.g;
     lt_status s = LT_OK;
-    const bool small = o.d_index && o.zc_col_base && o.slot_stride <= kCopyPartBytes && o.claimed.size() > 1;
+    const bool small = o.serve && o.d_index && o.zc_col_base && o.slot_stride <= kCopyPartBytes && o.claimed.size() > 1;
     for (size_t at = 0; at < o.claimed.size();) {
         if (!small) {
             const lt_status l = issue_load(o, o.claimed[at++], o.claimed_to);
