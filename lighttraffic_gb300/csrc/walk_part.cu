@@ -869,12 +869,15 @@ cudaError_t launch_part(const StepArgs &a, int grid, size_t smem, cudaStream_t s
     return cudaGetLastError();
 }
 
+// The limit on a kernel's dynamic shared memory belongs to the kernel, not to
+// the engine whose partition count asks for it, and part_smem is not monotonic
+// (35 016 bytes at 1 536 partitions, 22 744 at 1 537): it is set to the most any
+// engine takes, so that engines of different partition counts run side by side.
 template <int APP, bool HOT, bool SERVE, bool RP32>
 int occ_part(size_t smem)
 {
-    if (smem > 16 * 1024)
-        cudaFuncSetAttribute(walk_part_kernel<APP, HOT, SERVE, RP32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem);
+    static const int most = (int)std::max(part_smem(kColTableMax), part_smem(kSmemPartMax));
+    cudaFuncSetAttribute(walk_part_kernel<APP, HOT, SERVE, RP32>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
     int n = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, walk_part_kernel<APP, HOT, SERVE, RP32>, kPartBlock, smem);
     return n;
