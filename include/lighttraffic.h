@@ -401,7 +401,9 @@ lt_status lt_walk_device_noalloc(int app, int start_mode, const uint64_t *d_rowp
 lt_status lt_ppr_batch(lt_engine *e, uint32_t n, const uint32_t *sources, const uint64_t *walkers,
                        const uint64_t *seeds, float prob, uint64_t *out_offsets, uint32_t *out_vertices,
                        uint32_t *out_counts, uint64_t out_capacity);
-/* The same on device buffers, on `stream`; returns without waiting. */
+/* The same on device buffers, on `stream`; returns without waiting.  Batches
+ * of one engine share its buffers: each waits on the device for the one
+ * before, whatever their streams. */
 lt_status lt_ppr_batch_device(lt_engine *e, uint32_t n, const uint32_t *d_sources, const uint64_t *d_walkers,
                               const uint64_t *d_seeds, float prob, uint64_t *d_out_offsets,
                               uint32_t *d_out_vertices, uint32_t *d_out_counts, uint64_t out_capacity,

@@ -449,6 +449,9 @@ struct BatchState {
     BatchTune graph_tune;
     Header h_hdr{};
     BatchIn h_in{};
+    // behind the last batch enqueued: a batch's queries, tables and outputs lie
+    // in the buffers above, so the next one waits for it, on whatever stream
+    cudaEvent_t ev_last = nullptr;
 };
 
 namespace {
@@ -496,6 +499,7 @@ lt_status ensure(BatchState &b, uint32_t n, uint64_t W, uint64_t T)
     const uint32_t qcap = std::max<uint32_t>(n, std::max<uint32_t>(b.qcap, 64));
     const uint64_t wcap = std::max<uint64_t>(W, b.wcap);
     const uint64_t tcap = std::max<uint64_t>(T, b.tcap);
+    LT_CUDA_TRY(cudaEventSynchronize(b.ev_last));
     free_buffers(b);
     b.qcap = qcap;
     b.wcap = wcap;
@@ -612,6 +616,7 @@ lt_status run_graph(lt_engine *e, BatchState &b, const BatchIn &in, uint64_t thr
         b.graph_tune = b.tune;
     }
     LT_CUDA_TRY(cudaGraphLaunch(b.exec, st));
+    LT_CUDA_TRY(cudaEventRecord(b.ev_last, st));
     return LT_OK;
 }
 
@@ -629,8 +634,11 @@ lt_status check_inputs(lt_engine *e, uint32_t n, float prob)
 
 lt_status batch_create(lt_engine *e, BatchState **out)
 {
+    cudaEvent_t ev;
+    LT_CUDA_TRY(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
     BatchState *b = new BatchState();
     b->e = e;
+    b->ev_last = ev;
     *out = b;
     return LT_OK;
 }
@@ -638,7 +646,9 @@ lt_status batch_create(lt_engine *e, BatchState **out)
 void batch_destroy(BatchState *b)
 {
     if (!b) return;
+    cudaEventSynchronize(b->ev_last);
     free_buffers(*b);
+    cudaEventDestroy(b->ev_last);
     delete b;
 }
 
@@ -661,6 +671,7 @@ lt_status batch_run_device(lt_engine *e, uint32_t n, const uint32_t *d_sources, 
     if (W > out_capacity) return fail(LT_ERR_CAPACITY, "output capacity %llu is below the %llu walkers of the batch",
                                       (unsigned long long)out_capacity, (unsigned long long)W);
     LT_TRY(ensure(b, n, W, table_slots(w.data(), n, b.tune.load_shift)));
+    LT_CUDA_TRY(cudaStreamWaitEvent(st, b.ev_last, 0));
     LT_CUDA_TRY(cudaMemcpyAsync(b.d_src, d_sources, 4ull * n, cudaMemcpyDeviceToDevice, st));
     LT_CUDA_TRY(cudaMemcpyAsync(b.d_walkers, d_walkers, 8ull * n, cudaMemcpyDeviceToDevice, st));
     LT_CUDA_TRY(cudaMemcpyAsync(b.d_seeds, d_seeds, 8ull * n, cudaMemcpyDeviceToDevice, st));
@@ -683,14 +694,15 @@ lt_status batch_run(lt_engine *e, uint32_t n, const uint32_t *sources, const uin
                                       (unsigned long long)out_capacity, (unsigned long long)W);
     LT_TRY(ensure(b, n, W, table_slots(walkers, n, b.tune.load_shift)));
     cudaStream_t st = e->s_compute;
+    LT_CUDA_TRY(cudaStreamWaitEvent(st, b.ev_last, 0));
     const double t0 = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now().time_since_epoch()).count();
     LT_CUDA_TRY(cudaMemcpyAsync(b.d_src, sources, 4ull * n, cudaMemcpyHostToDevice, st));
     LT_CUDA_TRY(cudaMemcpyAsync(b.d_walkers, walkers, 8ull * n, cudaMemcpyHostToDevice, st));
     if (seeds) {
         LT_CUDA_TRY(cudaMemcpyAsync(b.d_seeds, seeds, 8ull * n, cudaMemcpyHostToDevice, st));
     } else {
-        std::vector<uint64_t> s(n, e->cfg.seed);
-        LT_CUDA_TRY(cudaMemcpy(b.d_seeds, s.data(), 8ull * n, cudaMemcpyHostToDevice));
+        const std::vector<uint64_t> s(n, e->cfg.seed);
+        LT_CUDA_TRY(cudaMemcpyAsync(b.d_seeds, s.data(), 8ull * n, cudaMemcpyHostToDevice, st));
     }
     // outputs in page-locked memory are written by the kernels themselves: no
     // copies, and no wait for the pairs' number before them
