@@ -470,6 +470,8 @@ void free_buffers(BatchState &b)
     if (b.graph) cudaGraphDestroy(b.graph);
     b.exec = nullptr;
     b.graph = nullptr;
+    b.qcap = 0;
+    b.wcap = b.tcap = 0;
 }
 
 template <typename T>
@@ -493,17 +495,8 @@ uint64_t table_slots(const uint64_t *walkers, uint32_t n, int shift)
     return t;
 }
 
-lt_status ensure(BatchState &b, uint32_t n, uint64_t W, uint64_t T)
+lt_status alloc_buffers(BatchState &b, uint32_t qcap, uint64_t wcap, uint64_t tcap)
 {
-    if (b.d_hdr && n <= b.qcap && W <= b.wcap && T <= b.tcap) return LT_OK;
-    const uint32_t qcap = std::max<uint32_t>(n, std::max<uint32_t>(b.qcap, 64));
-    const uint64_t wcap = std::max<uint64_t>(W, b.wcap);
-    const uint64_t tcap = std::max<uint64_t>(T, b.tcap);
-    LT_CUDA_TRY(cudaEventSynchronize(b.ev_last));
-    free_buffers(b);
-    b.qcap = qcap;
-    b.wcap = wcap;
-    b.tcap = tcap;
     LT_TRY(dalloc(&b.d_hdr, 1));
     LT_TRY(dalloc(&b.d_in, 1));
     LT_TRY(dalloc(&b.d_src, qcap));
@@ -521,7 +514,24 @@ lt_status ensure(BatchState &b, uint32_t n, uint64_t W, uint64_t T)
     LT_TRY(dalloc(&b.d_cnt, tcap));
     LT_TRY(dalloc(&b.d_out_v, wcap));
     LT_TRY(dalloc(&b.d_out_c, wcap));
+    b.qcap = qcap;
+    b.wcap = wcap;
+    b.tcap = tcap;
     return LT_OK;
+}
+
+lt_status ensure(BatchState &b, uint32_t n, uint64_t W, uint64_t T)
+{
+    if (n <= b.qcap && W <= b.wcap && T <= b.tcap) return LT_OK;
+    const uint32_t qcap = std::max<uint32_t>(n, std::max<uint32_t>(b.qcap, 64));
+    const uint64_t wcap = std::max<uint64_t>(W, b.wcap);
+    const uint64_t tcap = std::max<uint64_t>(T, b.tcap);
+    LT_CUDA_TRY(cudaEventSynchronize(b.ev_last));
+    free_buffers(b);
+    // all of them or none: a batch that does not fit leaves nothing behind
+    const lt_status s = alloc_buffers(b, qcap, wcap, tcap);
+    if (s != LT_OK) free_buffers(b);
+    return s;
 }
 
 BatchArgs args_of(lt_engine *e, BatchState &b, uint64_t thr)

@@ -1378,36 +1378,32 @@ uint64_t lazy_budget(Ooc &o, int32_t p, uint64_t left)
     return std::min(g, left);
 }
 
-lt_status ensure_pool(Ooc &o, uint64_t W)
+void free_pool(Ooc &o)
 {
-    lt_engine &e = *o.e;
-    uint64_t B = e.cfg.num_device_walkers ? e.cfg.num_device_walkers : W;
-    if (B > W) B = W;
-    if (B < kChunk) B = kChunk;
-    const uint64_t want = (B + kChunk - 1) / kChunk + 2ull * o.P + 2;
-    if (want > 0xFFFFFFF0ull) return fail(LT_ERR_CAPACITY, "walker pool too large");
-    if (o.d_arena && o.n_chunks == want) return LT_OK;
     for (void *p : {(void *)o.d_arena, (void *)o.d_out, (void *)o.d_planbuf, (void *)o.d_work, (void *)o.d_work_off})
         if (p) cudaFree(p);
-    host_free(o.h_plan);
-    host_free(o.h_work);
+    for (HostBuf *b : {&o.h_plan, &o.h_work, &o.h_planin}) host_free(*b);
     o.d_arena = nullptr;
     o.d_out = o.d_planbuf = o.d_work = nullptr;
     o.d_work_off = nullptr;
-    o.n_chunks = (uint32_t)want;
-    o.staging_cap = (uint64_t)o.n_chunks * kChunk;
-    o.plan_cap = o.n_chunks + (uint64_t)o.P;
-    o.work_cap = o.n_chunks;
-    LT_TRY(dalloc(&o.d_arena, (uint64_t)o.n_chunks * kChunkBytes));
+    o.n_chunks = 0;
+}
+
+lt_status alloc_pool(Ooc &o, uint32_t chunks)
+{
+    o.staging_cap = (uint64_t)chunks * kChunk;
+    o.plan_cap = chunks + (uint64_t)o.P;
+    o.work_cap = chunks;
+    LT_TRY(dalloc(&o.d_arena, (uint64_t)chunks * kChunkBytes));
     LT_TRY(dalloc(&o.d_out, 5 * o.staging_cap));
     LT_TRY(dalloc(&o.d_planbuf, 2ull * o.P + o.plan_cap));
     LT_TRY(dalloc(&o.d_work, o.work_cap));
     LT_TRY(dalloc(&o.d_work_off, o.work_cap));
     LT_TRY(host_alloc(o.h_plan, 4 * (2ull * o.P + o.plan_cap), true));
     LT_TRY(host_alloc(o.h_work, 12 * o.work_cap + 8, true));
-    host_free(o.h_planin);
-    o.planin_words = 2ull * o.P + o.n_chunks;
+    o.planin_words = 2ull * o.P + chunks;
     LT_TRY(host_alloc(o.h_planin, 2 * 4 * o.planin_words, true));
+    o.n_chunks = chunks;
     o.h_plan_dev = o.h_work_dev = o.h_planin_dev = nullptr;
     void *dv = nullptr;
     if (o.h_planin.pinned && cudaHostGetDevicePointer(&dv, o.h_planin.ptr, 0) == cudaSuccess)
@@ -1416,6 +1412,22 @@ lt_status ensure_pool(Ooc &o, uint64_t W)
     if (o.h_work.pinned && cudaHostGetDevicePointer(&dv, o.h_work.ptr, 0) == cudaSuccess) o.h_work_dev = (uint8_t *)dv;
     cudaGetLastError();
     return LT_OK;
+}
+
+lt_status ensure_pool(Ooc &o, uint64_t W)
+{
+    lt_engine &e = *o.e;
+    uint64_t B = e.cfg.num_device_walkers ? e.cfg.num_device_walkers : W;
+    if (B > W) B = W;
+    if (B < kChunk) B = kChunk;
+    const uint64_t want = (B + kChunk - 1) / kChunk + 2ull * o.P + 2;
+    if (want > 0xFFFFFFF0ull) return fail(LT_ERR_CAPACITY, "walker pool too large");
+    if (o.n_chunks == want) return LT_OK;
+    free_pool(o);
+    // all of it or none: a pool that does not fit leaves nothing behind
+    const lt_status s = alloc_pool(o, (uint32_t)want);
+    if (s != LT_OK) free_pool(o);
+    return s;
 }
 
 void reset_queues(Ooc &o)
