@@ -256,7 +256,8 @@ void lt_engine_destroy(lt_engine *e);
 lt_status lt_engine_drop_cache(lt_engine *e);
 
 /* PPR from one source (app/ppr.cu main + AppManager, :45-113): num_walkers
- * walks with stop probability prob; counts_out (host, u64[V], may be NULL)
+ * walks with stop probability prob (in [2^-26, 1] wherever one is given: the
+ * lengths of walks have 32 bits); counts_out (host, u64[V], may be NULL)
  * receives per-vertex endpoint counts (AppManager::reduce, :65-67). */
 lt_status lt_run_ppr(lt_engine *e, uint32_t source, uint64_t num_walkers, float prob,
                      uint64_t *counts_out);

@@ -634,7 +634,7 @@ lt_status check_inputs(lt_engine *e, uint32_t n, float prob)
 {
     if (!e->resident || !e->d_rowptr)
         return fail(LT_ERR_UNSUPPORTED, "batched PPR needs every partition cached on the device");
-    if (!(prob > 0.0f && prob <= 1.0f)) return fail(LT_ERR_INVALID, "PPR stop probability must be in (0, 1]");
+    LT_TRY(check_stop_prob(prob));
     if (n == 0) return fail(LT_ERR_INVALID, "empty batch");
     LT_CUDA_TRY(cudaSetDevice(e->device));
     return engine_ensure_loaded(e);

@@ -352,7 +352,7 @@ lt_status lt_engine_drop_cache(lt_engine *e)
 lt_status lt_run_ppr(lt_engine *e, uint32_t source, uint64_t num_walkers, float prob, uint64_t *counts_out)
 {
     if (!e) return fail(LT_ERR_INVALID, "null engine");
-    if (!(prob > 0.0f && prob <= 1.0f)) return fail(LT_ERR_INVALID, "PPR stop probability must be in (0, 1]");
+    LT_TRY(check_stop_prob(prob));
     return engine_run(e, LT_APP_PPR, LT_START_SOURCE, source, num_walkers, 0, 1, 0, prob, counts_out, nullptr, nullptr);
 }
 

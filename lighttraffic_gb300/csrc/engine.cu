@@ -69,6 +69,18 @@ uint64_t count_updates(int app, uint64_t W, uint32_t length)
     return 0;
 }
 
+}  // namespace
+
+lt_status check_stop_prob(float prob)
+{
+    if (!(prob > 0.0f && prob <= 1.0f)) return fail(LT_ERR_INVALID, "PPR stop probability must be in (0, 1]");
+    if (prob < kMinStopProb)
+        return fail(LT_ERR_INVALID, "PPR stop probability below 2^-26: walk lengths would not fit 32 bits");
+    return LT_OK;
+}
+
+namespace {
+
 // One launch of the resident step kernel, standard (u64 row offsets and
 // counters) or compact (u32, when d_rowptr32 is given).
 lt_status walk_launch(int app, int start, const uint64_t *d_rowptr, const uint32_t *d_rowptr32, const uint32_t *d_col,
@@ -86,7 +98,7 @@ lt_status walk_launch(int app, int start, const uint64_t *d_rowptr, const uint32
         return fail(LT_ERR_INVALID, "counts buffer is required for PPR and PageRank");
     if (app != kWalk && layout == kLayoutCompact && !d_counts32)
         return fail(LT_ERR_INVALID, "counts buffer is required for PPR and PageRank");
-    if (app == kPPR && !(prob > 0.0f && prob <= 1.0f)) return fail(LT_ERR_INVALID, "PPR stop probability must be in (0, 1]");
+    if (app == kPPR) LT_TRY(check_stop_prob(prob));
     if (app != kPPR && length == 0) return fail(LT_ERR_INVALID, "walk length must be positive");
     if (start == kStartSource && source >= V) return fail(LT_ERR_INVALID, "source %u out of range (V=%u)", source, V);
     if (run > 0xFFFFFFu) return fail(LT_ERR_INVALID, "run index %u exceeds 2^24 - 1", run);

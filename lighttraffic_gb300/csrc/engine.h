@@ -65,6 +65,8 @@ lt_status walk_device(int app, int start, const uint64_t *d_rowptr, const uint32
                       uint64_t *d_counts, uint32_t *d_endpoints, uint32_t *d_paths, void *d_scratch,
                       uint64_t *d_stats, cudaStream_t st, int block_ctas);
 size_t walk_scratch_bytes();
+// a PPR stop probability that every entry point takes: [kMinStopProb, 1]
+lt_status check_stop_prob(float prob);
 lt_status walk_device_compact(int app, int start, const uint32_t *d_rowptr32, const uint32_t *d_col, uint32_t V,
                               uint32_t source, uint64_t W, uint32_t length, float prob, uint32_t run, uint64_t seed,
                               uint32_t *d_counts32, uint32_t *d_endpoints, uint32_t *d_paths, void *d_scratch,

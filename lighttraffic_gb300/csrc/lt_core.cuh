@@ -140,6 +140,12 @@ inline uint64_t threshold53(float p)
     return (uint64_t)(d * 9007199254740992.0);
 }
 
+// The smallest PPR stop probability taken.  A walk's length has 32 bits and is
+// drawn until a draw stops it: at 2^-26 one of 2^32 walks is longer than 2^32
+// with probability 2^32 e^-64 < 1e-18; far below, lengths would wrap, and under
+// 2^-53, where floor(p 2^53) = 0, no draw would ever stop a walk.
+constexpr float kMinStopProb = 1.0f / (1 << 26);
+
 LT_HD float rcp_f32(float d)
 {
 #ifdef __CUDA_ARCH__

@@ -2392,8 +2392,8 @@ lt_status get_header(Reader &r, const char *path, CkptHeader &h)
     // the checks run_setup and the engine entry points make on a fresh run
     if (h.start == kStartSource && h.source >= h.V)
         return fail(LT_ERR_FORMAT, "%s: source %u outside the graph's %u vertices", path, h.source, h.V);
-    if (h.app == kPPR && !(h.prob > 0.0f && h.prob <= 1.0f))
-        return fail(LT_ERR_FORMAT, "%s: PPR stop probability outside (0, 1]", path);
+    if (h.app == kPPR && !(h.prob >= kMinStopProb && h.prob <= 1.0f))
+        return fail(LT_ERR_FORMAT, "%s: PPR stop probability outside [2^-26, 1]", path);
     if (h.app == kPageRank && !(h.prob >= 0.0f && h.prob <= 1.0f))
         return fail(LT_ERR_FORMAT, "%s: PageRank probability outside [0, 1]", path);
     if (h.app != kPPR && h.length == 0) return fail(LT_ERR_FORMAT, "%s: walk length 0", path);
@@ -3219,7 +3219,7 @@ lt_status serve_open(lt_engine *e, uint32_t max_active, uint64_t table_slots, fl
 {
     if (!e->ooc) return fail(LT_ERR_UNSUPPORTED, "serving runs on the out-of-core engine (-p below the partition count)");
     if (e->ooc->serve) return fail(LT_ERR_INVALID, "the engine already serves");
-    if (!(prob > 0.0f && prob <= 1.0f)) return fail(LT_ERR_INVALID, "PPR stop probability must be in (0, 1]");
+    LT_TRY(check_stop_prob(prob));
     if (max_active == 0 || table_slots < 64) return fail(LT_ERR_INVALID, "no room for queries");
     LT_CUDA_TRY(cudaSetDevice(e->device));
     Ooc &o = *e->ooc;
