@@ -40,8 +40,8 @@ struct HostBuf {
 };
 lt_status host_alloc(HostBuf &b, size_t bytes, bool want_pinned);
 void host_free(HostBuf &b);
-// The device's address of page-locked host memory [p, p + bytes), null where
-// either end is not page-locked memory of one allocation.
+// The device's address of page-locked host memory [p, p + bytes); null where
+// that is not part of one page-locked allocation or registered region.
 void *mapped_host(const void *p, size_t bytes);
 
 }  // namespace lt

@@ -6,6 +6,8 @@
 #include <cstring>
 #include <string>
 
+#include <cuda.h>
+
 namespace lt {
 
 namespace {
@@ -28,16 +30,29 @@ const char *last_error() { return g_last_error.c_str(); }
 
 void *mapped_host(const void *p, size_t bytes)
 {
-    cudaPointerAttributes first{}, last{};
-    const uint8_t *end = (const uint8_t *)p + (bytes ? bytes - 1 : 0);
-    if (!p || cudaPointerGetAttributes(&first, p) != cudaSuccess || cudaPointerGetAttributes(&last, end) != cudaSuccess) {
-        cudaGetLastError();
+    // The runtime's pointer attributes tell nothing of an allocation's extent,
+    // and under unified addressing the device addresses of any two page-locked
+    // bytes differ as their host addresses do: the driver's range attributes
+    // (of the allocation, or of the registered region) decide.
+    using Query = CUresult (*)(unsigned, CUpointer_attribute *, void **, CUdeviceptr);
+    static const Query query = [] {
+        void *f = nullptr;
+        cudaDriverEntryPointQueryResult found = cudaDriverEntryPointSymbolNotFound;
+        const cudaError_t e = cudaGetDriverEntryPointByVersion("cuPointerGetAttributes", &f, 12000, cudaEnableDefault, &found);
+        if (e != cudaSuccess) cudaGetLastError();
+        return e == cudaSuccess && found == cudaDriverEntryPointSuccess ? (Query)f : (Query) nullptr;
+    }();
+    if (!p || !query) return nullptr;
+    unsigned type = 0;
+    CUdeviceptr dev = 0, start = 0;
+    size_t size = 0;
+    CUpointer_attribute what[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_DEVICE_POINTER,
+                                  CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+    void *out[] = {&type, &dev, &start, &size};
+    if (query(4, what, out, (CUdeviceptr)p) != CUDA_SUCCESS || type != CU_MEMORYTYPE_HOST || !dev || dev < start)
         return nullptr;
-    }
-    if (first.type != cudaMemoryTypeHost || last.type != cudaMemoryTypeHost || !first.devicePointer ||
-        (uint8_t *)last.devicePointer - (uint8_t *)first.devicePointer != end - (const uint8_t *)p)
-        return nullptr;
-    return first.devicePointer;
+    const uint64_t at = dev - start;
+    return at < size && bytes <= size - at ? (void *)dev : nullptr;
 }
 
 lt_status host_alloc(HostBuf &b, size_t bytes, bool want_pinned)
