@@ -685,7 +685,16 @@ lt_status batch_run_device(lt_engine *e, uint32_t n, const uint32_t *d_sources, 
     LT_CUDA_TRY(cudaMemcpyAsync(b.d_src, d_sources, 4ull * n, cudaMemcpyDeviceToDevice, st));
     LT_CUDA_TRY(cudaMemcpyAsync(b.d_walkers, d_walkers, 8ull * n, cudaMemcpyDeviceToDevice, st));
     LT_CUDA_TRY(cudaMemcpyAsync(b.d_seeds, d_seeds, 8ull * n, cudaMemcpyDeviceToDevice, st));
-    return run_graph(e, b, BatchIn{n, d_offsets, d_vertices, d_counts}, threshold53(prob), st);
+    // the kernels store whole elements: results for addresses that are not a
+    // multiple of their size go through the engine's own arrays
+    if (((uintptr_t)d_offsets & 7) == 0 && (((uintptr_t)d_vertices | (uintptr_t)d_counts) & 3) == 0)
+        return run_graph(e, b, BatchIn{n, d_offsets, d_vertices, d_counts}, threshold53(prob), st);
+    LT_TRY(run_graph(e, b, BatchIn{n, b.d_qout, b.d_out_v, b.d_out_c}, threshold53(prob), st));
+    LT_CUDA_TRY(cudaMemcpyAsync(d_offsets, b.d_qout, 8ull * (n + 1), cudaMemcpyDeviceToDevice, st));
+    LT_CUDA_TRY(cudaMemcpyAsync(d_vertices, b.d_out_v, 4ull * W, cudaMemcpyDeviceToDevice, st));
+    LT_CUDA_TRY(cudaMemcpyAsync(d_counts, b.d_out_c, 4ull * W, cudaMemcpyDeviceToDevice, st));
+    LT_CUDA_TRY(cudaEventRecord(b.ev_last, st));
+    return LT_OK;
 }
 
 lt_status batch_run(lt_engine *e, uint32_t n, const uint32_t *sources, const uint64_t *walkers, const uint64_t *seeds,
@@ -716,8 +725,8 @@ lt_status batch_run(lt_engine *e, uint32_t n, const uint32_t *sources, const uin
     }
     // outputs in page-locked memory are written by the kernels themselves: no
     // copies, and no wait for the pairs' number before them
-    const BatchIn direct{n, (uint64_t *)mapped_host(out_offsets, 8ull * (n + 1)), (uint32_t *)mapped_host(out_vertices, 4 * W),
-                         (uint32_t *)mapped_host(out_counts, 4 * W)};
+    const BatchIn direct{n, mapped_results(out_offsets, n + 1ull), mapped_results(out_vertices, W),
+                         mapped_results(out_counts, W)};
     const bool pinned = direct.qout && direct.out_v && direct.out_c;
     LT_CUDA_TRY(cudaEventRecord(e->ev_k0, st));
     LT_TRY(run_graph(e, b, pinned ? direct : BatchIn{n, b.d_qout, b.d_out_v, b.d_out_c}, threshold53(prob), st));

@@ -43,5 +43,12 @@ void host_free(HostBuf &b);
 // The device's address of page-locked host memory [p, p + bytes); null where
 // that is not part of one page-locked allocation or registered region.
 void *mapped_host(const void *p, size_t bytes);
+// The same for results: n elements that kernels store whole, so their address
+// has to be a multiple of their size (a copy takes any).
+template <typename T>
+T *mapped_results(T *p, uint64_t n)
+{
+    return (uintptr_t)p % sizeof(T) == 0 ? (T *)mapped_host(p, n * sizeof(T)) : nullptr;
+}
 
 }  // namespace lt

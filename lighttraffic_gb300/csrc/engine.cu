@@ -385,11 +385,11 @@ lt_status engine_run(lt_engine *e, int app, int start, uint32_t source, uint64_t
     bool counts_done = false;
     if (compact && cnt) {
         // straight into the caller's page-locked memory where that is what it
-        // is (both of its ends): a copy after the kernel costs 9 us more at
-        // V = 47 000 and 13 us at V = 4.6 M
+        // is: a copy after the kernel costs 9 us more at V = 47 000 and 13 us
+        // at V = 4.6 M
         uint64_t *dst = e->d_counts, *host_stats = e->h_stats_dev;
         if (counts_out) {
-            uint64_t *out = (uint64_t *)mapped_host(counts_out, 8ull * g.V);
+            uint64_t *out = mapped_results(counts_out, g.V);
             counts_done = out != nullptr;
             if (out) dst = out;
         }
