@@ -157,7 +157,8 @@ typedef struct lt_stats {
     uint64_t zerocopy_calls;
     uint64_t walker_loading_calls;
     uint64_t walker_evicting_calls;
-    double step_kernel_ms;    /* time of the step kernels of the last run */
+    double step_kernel_ms;    /* time of the step kernels of the last run (batches: to where the
+                                  results begin to be written) */
     uint64_t handoffs;        /* walkers staged and bucketed into another partition's queue */
     uint64_t overlap_computes; /* plain / FIFO loop: cached partitions computed while a load was in
                                   flight (getComputedPartition, src/Scheduler.h:194-208) */

@@ -381,6 +381,8 @@ lt_status engine_run(lt_engine *e, int app, int start, uint32_t source, uint64_t
         e->stats.kernel_launches++;
         e->stats.computing_calls++;
     }
+    // the end of the step kernels: what follows may write host memory
+    LT_CUDA_TRY(cudaEventRecord(e->ev_k1, st));
     uint64_t *hs = (uint64_t *)e->h_stats.ptr;
     bool counts_done = false;
     if (compact && cnt) {
@@ -400,7 +402,6 @@ lt_status engine_run(lt_engine *e, int app, int start, uint32_t source, uint64_t
     } else {
         LT_CUDA_TRY(cudaMemcpyAsync(hs, e->d_stats, 24, cudaMemcpyDeviceToHost, st));
     }
-    LT_CUDA_TRY(cudaEventRecord(e->ev_k1, st));
     if (counts_out && !counts_done)
         LT_CUDA_TRY(cudaMemcpyAsync(counts_out, e->d_counts, 8ull * g.V, cudaMemcpyDeviceToHost, st));
     if (endpoints_out) LT_CUDA_TRY(cudaMemcpyAsync(endpoints_out, e->d_endpoints, 4 * W, cudaMemcpyDeviceToHost, st));
