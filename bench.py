@@ -973,7 +973,7 @@ def gb300_batch(args, cfg):
         "e2e": {"value": moves * ws / statistics.mean(e2e), "unit": "steps/s",
                 "h2d_bytes_per_step": 20 * n, "d2h_bytes_per_step": 8 * (n + 1) + 8 * pairs,
                 "ms_per_step": statistics.mean(e2e) * 1e3},
-        "gpu_launches": 6 * args.steps,
+        "gpu_launches": st["kernel_launches"] * args.steps,
         "clocks": clk,
     }
     if not args.no_cpu_baseline and ws == 1:

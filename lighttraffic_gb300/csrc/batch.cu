@@ -757,7 +757,7 @@ lt_status batch_run(lt_engine *e, uint32_t n, const uint32_t *sources, const uin
     e->stats.computing_ms = ms;
     e->stats.computing_calls = 1;
     e->stats.iterations = 1;
-    e->stats.kernel_launches = 6;
+    e->stats.kernel_launches = 6 + scan_launches(b.nch);  // see enqueue_pipeline
     e->stats.running_ms =
         std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now().time_since_epoch()).count() - t0;
     return LT_OK;

@@ -148,6 +148,9 @@ __device__ __forceinline__ uint64_t warp_find_last(const uint64_t *off, uint64_t
     return lo;
 }
 
+// kernels that exclusive_scan launches
+inline uint32_t scan_launches(uint64_t n) { return n == 0 ? 0 : n <= kScanOneCta ? 1 : 3; }
+
 // out[i] = sum(in[0..i)) for i in [0, n]; out has n+1 entries (out[n] = total).
 // tmp must hold ceil(n / kScanTile) + 1 Out values.  In and out may not alias.
 template <typename In, typename Out>
