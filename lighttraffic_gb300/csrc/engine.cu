@@ -378,7 +378,7 @@ lt_status engine_run(lt_engine *e, int app, int start, uint32_t source, uint64_t
                            cnt && !compact ? e->d_counts : nullptr, cnt && compact ? e->d_counts32 : nullptr,
                            endpoints_out ? e->d_endpoints : nullptr, paths_out ? e->d_paths : nullptr, e->d_scratch,
                            e->d_stats, st, e->cfg.ctas_per_sm, nullptr, r == 0));
-        e->stats.kernel_launches++;
+        e->stats.kernel_launches += whole_launches(app, W, length, e->sms);
         e->stats.computing_calls++;
     }
     // the end of the step kernels: what follows may write host memory

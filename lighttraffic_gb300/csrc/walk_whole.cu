@@ -341,7 +341,7 @@ __global__ void __launch_bounds__(block_of<APP>, 2048 / block_of<APP>) walk_whol
             exhausted = first_deal ? dealt >= a.W : base + idle >= a.W;
             first_deal = false;
             if (!active && base + rank < a.W) {
-                idx = base + rank;
+                idx = (kHot ? a.first : 0u) + base + rank;
                 cur = first_vertex<START>(a, idx);
                 step = a.length;
                 active = true;
@@ -428,13 +428,47 @@ uint64_t most_ctas(uint64_t W, int sms)
     return std::min(full, std::max<uint64_t>(2ull * sms, six));
 }
 
+// A hub counter of a CTA has 32 bits, and nothing bounds the share of a launch's
+// walkers that one CTA takes while others wait for SMs that another stream's
+// kernels hold.  So PageRank calls of 2^32 updates and more become launches of
+// fewer, one after the other, where each still fills the chip several times
+// over (a launch's start and end are then 1e-4 of its time), and one launch
+// without tables where the walks are too long for that.  4.8e9 updates in two
+// launches, and in one without tables: RMAT 2^21 / 4e7 49.8 ms, 61.5; 2^23 / 2^27 93.0,
+// 113.5; 2^16 / 2^20 34.0, 153.6.
+constexpr uint64_t kHotUpdates = (1ull << 32) - 1;
+
+uint64_t hot_walkers(uint32_t length) { return length ? kHotUpdates / length : 0; }
+
+bool pagerank_hot(uint64_t W, uint32_t length, int sms)
+{
+    return W <= hot_walkers(length) || hot_walkers(length) >= 4 * 2048ull * sms;
+}
+
 template <int APP, int START, int C>
 cudaError_t launch_t(const WholeArgs &a, int grid, cudaStream_t st)
 {
-    grid = (int)std::min<uint64_t>((uint64_t)grid, most_ctas<APP>(a.W, a.sms));
     WholeArgs b = a;
-    // a CTA's counters have 32 bits: 19 times its share of these updates
-    b.hot = a.length == 0 || a.W < (1ull << 36) / a.length;
+    if constexpr (APP == kPageRank) {
+        b.hot = pagerank_hot(a.W, a.length, a.sms);
+        const uint64_t n = whole_launches(APP, a.W, a.length, a.sms);
+        if (n > 1) {
+            b.W = (a.W + n - 1) / n;
+            for (b.first = 0; b.first < a.W; b.first += b.W) {
+                b.W = std::min(b.W, a.W - b.first);
+                if (b.first) {
+                    const cudaError_t cleared = cudaMemsetAsync(b.next, 0, sizeof *b.next, st);
+                    if (cleared != cudaSuccess) return cleared;
+                }
+                const int ctas = (int)std::min<uint64_t>((uint64_t)grid, most_ctas<APP>(b.W, a.sms));
+                walk_whole_kernel<APP, START, C, false><<<ctas, block_of<APP>, 0, st>>>(b);
+                const cudaError_t launched = cudaGetLastError();
+                if (launched != cudaSuccess) return launched;
+            }
+            return cudaSuccess;
+        }
+    }
+    grid = (int)std::min<uint64_t>((uint64_t)grid, most_ctas<APP>(a.W, a.sms));
     b.pool = pool_walkers(a.W, (uint64_t)grid * (kWholeBlock / 32));
     if constexpr (APP == kWalk) {
         if (a.paths && a.length >= kPathGatherMin && a.W > 2ull * a.sms * kWholeBlock * 8) {
@@ -481,6 +515,12 @@ int occupancy_c(int app, int start)
 }
 
 }  // namespace
+
+uint64_t whole_launches(int app, uint64_t W, uint32_t length, int sms)
+{
+    if (app != kPageRank || !pagerank_hot(W, length, sms)) return 1;
+    return (W + hot_walkers(length) - 1) / hot_walkers(length);
+}
 
 // SMs of the device and resident CTAs per SM of a kernel instance: properties
 // of the device and the code, asked for once (the occupancy query costs a

@@ -38,7 +38,8 @@ struct WholeArgs {
     Limit53 lim;             // of floor(p 2^53): PPR stop prob or PageRank alpha
     ModN by_v;               // remainders by V
     uint32_t pool;           // PPR: walkers a warp draws lengths for at a time (set by the launcher)
-    int hot;                       // PageRank: CTAs count hubs in shared memory; set by the launcher
+    int hot;                 // PageRank: CTAs count hubs in shared memory; set by the launcher
+    uint64_t first;          // PageRank: index of the launch's first walker; set by the launcher
     uint32_t long_len;       // PPR: walks longer than this begin first in their pool
 };
 
@@ -47,6 +48,9 @@ enum Layout : int { kLayoutWide = 0, kLayoutCompact = 1, kLayoutPacked = 2 };
 int whole_sms(int device);
 // Persistent grid size: SMs x resident CTAs (capped by ctas_per_sm when > 0).
 int whole_grid(int app, int start, int device, int ctas_per_sm, int layout = kLayoutWide);
+// Launches a call of W walkers becomes (one after the other, a.next cleared
+// between them).
+uint64_t whole_launches(int app, uint64_t W, uint32_t length, int sms);
 cudaError_t launch_walk_whole(const WholeArgs &a, int app, int start, int grid, cudaStream_t st,
                               int layout = kLayoutWide);
 
