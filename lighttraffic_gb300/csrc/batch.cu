@@ -194,14 +194,15 @@ __device__ __forceinline__ void table_add(const BatchArgs &a, uint32_t q, uint32
     atomicAdd(&a.hdr->error, 1ull);
 }
 
-// Endpoints wait here until a warp has 32 of them: added one by one as the
-// walks end, a few lanes' table probes (a load and two atomics in a row) would
-// hold up the hops of the others in nearly every iteration.
 // Threads per SM the registers are sized for: 48 registers without spills.
 // 256 queries of 7.3 M walks on RMAT 2^22 / 2^26: 2048 (32 registers, spilled) 2.6 ms per batch, 1536 1.52, 1280 1.47,
 // 1024 1.53.
 constexpr int kThreadsPerSm = 1280;
 
+// What a warp keeps in shared memory.  Endpoints wait here until there are 32 of
+// them: added one by one as the walks end, a few lanes' table probes (a load and
+// two atomics in a row) would hold up the hops of the others in nearly every
+// iteration.
 struct BatchWarp {
     PprPool pool;
     uint2 ends[64];  // (query, vertex)

@@ -169,9 +169,9 @@ LT_HD float rcp_approx_f32(float d)
 
 // x mod d for 0 < d <= 2^20 by folding: with m close below 2^32 / d, e = 2^32 -
 // m d is congruent to 2^32 and below 2 d, so hi 2^32 + lo = hi e + lo (mod d).
-// Three folds bring x below 2^32 + e, one more below 2^32 (d <= 2^20: the
-// folds' high words are below 2^32, 2^21, 2^10 + 1 and 2), and one
-// multiplication by m leaves less than 3 d.
+// With d <= 2^20, e < 2^21: a fold leaves a high word of at most e, the next
+// one of at most 2^10, the third x below 2^32 + 2^31 (a high word of at most
+// 1), the fourth below 2^32; one multiplication by m then leaves less than 3 d.
 //
 // m: a single-precision reciprocal scaled down by 2^-22 (so that it never
 // exceeds 2^32 / d; its relative error stays below 2^-21) and one Newton step
@@ -273,14 +273,6 @@ LT_HD uint32_t ppr_length(uint64_t seed, uint32_t run, uint64_t idx, uint64_t th
         if (m53_of(r) < thr) return step;
         step++;
     }
-}
-
-LT_HD uint32_t start_vertex(int start, uint32_t source, uint32_t V, uint64_t seed, uint32_t run, uint64_t idx)
-{
-    if (start == kStartSource) return source;
-    if (start == kStartPerVertex) return (uint32_t)(idx % V);
-    const Rand4 r = walk_draw(seed, 0, kTagInit, run, idx);
-    return (uint32_t)mod_u64(r64_of(r), V);
 }
 
 // 16-bit lane l (0..7) of a Philox output, used by the RMAT generator.

@@ -80,7 +80,6 @@ __device__ __forceinline__ void red_add_u64(unsigned long long *a, uint64_t n, u
 }
 
 __device__ __forceinline__ void red_add1_u64(unsigned long long *a, uint64_t pol) { red_add_u64(a, 1, pol); }
-__device__ __forceinline__ void red_add1_u32(unsigned int *a, uint64_t pol) { red_add_u32(a, 1, pol); }
 
 // ---- bulk copies global -> shared (the TMA unit's untiled mode) and the
 // mbarriers that count their bytes.  Both addresses and the size must be

@@ -1046,7 +1046,9 @@ lt_status step_and_bucket_parts(Ooc &o, const RunParams &rp, const std::vector<u
     // 0.952 -> 0.934 s per run; two CTAs per SM for the cached kernel: 0.973).
     // 512 lanes per SM keep the host link full; more only take issue slots
     // and cache from the cached kernel (PPR of 8.4 M walks on RMAT 2^24 / 2^28
-    // with 14 of 35 partitions: 4 CTAs per SM 10.1 ms, 3 9.17, 2 9.14, 1 9.14).
+    // with 14 of 35 partitions: 4 CTAs per SM 10.1 ms, 3 9.17, 2 9.14, 1 9.14; of
+    // 730 M on RMAT 2^30 / 2^33 with 212 of 1112: 3 863 and 953 ms in two
+    // processes, 2 859 and 934).
     auto in_group = [&](uint32_t x) { return o.zc_mask_any && ((o.zc_mask[x >> 5] >> (x & 31)) & 1u); };
     std::vector<uint32_t> order;
     uint64_t nw_a = 0, walkers_a = 0;  // the cached part of a split launch

@@ -579,55 +579,38 @@ __global__ void __launch_bounds__(kPartBlock, kPartMinBlocks) walk_part_kernel(c
         }
 }
 
-// Tile of kScatterItems walkers per thread.
+// Bucketing above kSmemPartMax partitions, whose counts do not fit shared
+// memory: one global atomic per walker, kScatterItems of a thread in flight.
 constexpr int kScatterItems = 4;
 
 __global__ void __launch_bounds__(kPartBlock) scatter_kernel(ScatterArgs a)
 {
-    if (blockIdx.x == 0 && threadIdx.x == 0 && !a.n_dev) a.clk[0] = globaltimer_ns();
-    extern __shared__ uint32_t smem[];
-    const uint32_t P = a.P;
-    const bool in_smem = P <= kSmemPartMax;
-    uint32_t *s_cnt = smem;       // P: walkers of this tile per destination
-    uint32_t *s_base = smem + P;  // P: reserved base slot per destination
+    if (blockIdx.x == 0 && threadIdx.x == 0) a.clk[0] = globaltimer_ns();
     const uint64_t tile = (uint64_t)kPartBlock * kScatterItems;
     for (uint64_t t0 = (uint64_t)blockIdx.x * tile; t0 < a.n; t0 += (uint64_t)gridDim.x * tile) {
-        uint32_t rank[kScatterItems], dest[kScatterItems];
-        if (in_smem) {
-            for (uint32_t i = threadIdx.x; i < P; i += blockDim.x) s_cnt[i] = 0;
-            __syncthreads();
-        }
+        uint32_t pos[kScatterItems], dest[kScatterItems];
 #pragma unroll
         for (int k = 0; k < kScatterItems; k++) {
             const uint64_t i = t0 + (uint64_t)k * kPartBlock + threadIdx.x;
             dest[k] = 0xFFFFFFFFu;
             if (i < a.n) {
                 dest[k] = a.in_dest[i];
-                rank[k] = in_smem ? atomicAdd(&s_cnt[dest[k]], 1u) : atomicAdd(&a.cursor[dest[k]], 1u);
+                pos[k] = atomicAdd(&a.cursor[dest[k]], 1u);
             }
-        }
-        if (in_smem) {
-            __syncthreads();
-            for (uint32_t i = threadIdx.x; i < P; i += blockDim.x)
-                if (s_cnt[i]) s_base[i] = atomicAdd(&a.cursor[i], s_cnt[i]);
-            __syncthreads();
         }
 #pragma unroll
         for (int k = 0; k < kScatterItems; k++) {
             const uint64_t i = t0 + (uint64_t)k * kPartBlock + threadIdx.x;
             if (i < a.n) {
-                const uint32_t d = dest[k];
-                const uint32_t pos = in_smem ? s_base[d] + rank[k] : rank[k];
-                const uint32_t chunk = a.plan_chunks[a.win_off[d] + pos / kChunk];
+                const uint32_t chunk = a.plan_chunks[a.win_off[dest[k]] + pos[k] / kChunk];
                 uint32_t *c = reinterpret_cast<uint32_t *>(a.arena + (uint64_t)chunk * kChunkBytes);
-                const uint32_t j = pos % kChunk;
+                const uint32_t j = pos[k] % kChunk;
                 c[j] = a.in_cur[i];
                 c[kChunk + j] = a.in_step[i];
                 c[2 * kChunk + j] = a.in_idx[i];
                 c[3 * kChunk + j] = a.in_q[i];
             }
         }
-        if (in_smem) __syncthreads();
     }
     if (threadIdx.x == 0) atomicMax(&a.clk[1], (unsigned long long)globaltimer_ns());
 }
@@ -992,11 +975,8 @@ cudaError_t launch_scatter(const ScatterArgs &a, int device, cudaStream_t st)
         return cudaGetLastError();
     }
     const uint64_t tile = (uint64_t)kPartBlock * kScatterItems;
-    uint64_t blocks = (a.n + tile - 1) / tile;
-    const uint64_t cap = (uint64_t)sms * 8;
-    if (blocks > cap) blocks = cap;
-    const size_t smem = a.P <= kSmemPartMax ? sizeof(uint32_t) * 2ull * a.P : 0;
-    scatter_kernel<<<(unsigned)blocks, kPartBlock, smem, st>>>(a);
+    const uint64_t blocks = std::min<uint64_t>((a.n + tile - 1) / tile, (uint64_t)sms * 8);
+    scatter_kernel<<<(unsigned)blocks, kPartBlock, 0, st>>>(a);
     return cudaGetLastError();
 }
 

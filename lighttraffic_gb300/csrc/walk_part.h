@@ -24,12 +24,12 @@ constexpr uint32_t kPartMapN = 2048;                       // blocks of vertices
 constexpr uint32_t kZcMaskWords = kSmemPartMax / 32;       // zero-copy set of one launch, one bit per partition
 
 // Device view of the partition table: node / edge ranges of every partition
-// and, for readable partitions, the addresses of their rowptr slice (n+1
-// global edge offsets) and col slice -- a device cache slot, or pinned host
-// memory read zero-copy, marked by bit 0 of the rowptr address.  An entry may
-// change while a step kernel runs only from unreadable or zero-copy to a
-// cache slot whose copy has completed; a slot is never overwritten while a
-// kernel that may read it runs.
+// and, for the cached ones, the addresses of their rowptr slice (n+1 global edge
+// offsets, or u32 ones of the device index) and col slice in a device cache
+// slot.  Partitions read zero-copy are not in it: each launch names its own
+// (zc_part, zc_mask).  The entries change only between step kernels
+// (pass_begin_kernel), and a slot is never overwritten while a kernel that may
+// read it runs.
 struct PartTable {
     const uint32_t *node_off;             // P+1
     const uint64_t *edge_off;             // P+1
@@ -175,12 +175,5 @@ cudaError_t launch_walk_part(const StepArgs &a, int app, int grid, cudaStream_t 
 cudaError_t launch_scatter(const ScatterArgs &a, int device, cudaStream_t st);
 // P <= kSmemPartMax
 cudaError_t launch_plan(const PlanArgs &a, cudaStream_t st);
-
-// Ordinal t of the lazily created walkers of partition [nb, ne) under the
-// per-vertex start: walkers j*V + v (v in [nb, ne)), ordered j-major.
-__host__ __device__ inline uint64_t per_vertex_id(uint64_t t, uint32_t nb, uint32_t n, uint32_t V)
-{
-    return (t / n) * (uint64_t)V + nb + (t % n);
-}
 
 }  // namespace lt
